@@ -108,32 +108,32 @@ def listed():
         # The smallest run the engine takes: one vector of 8 lanes, little
         # more than the 1000 frames a run must have.  Start-up, launches and
         # result reads are all of it.
-        one(name="fp64 one vector, 1200 steps", trajectories=8, steps=1200, freq=1, dt=1e-4, tau=1e-5, frames=True),
+        one(name="fp64 one vector 1200 steps", trajectories=8, steps=1200, freq=1, dt=1e-4, tau=1e-5, frames=True),
         # The reference's own sample input (4 ranks x 8 lanes, dt 1e-4, a flip
         # at about every second step, every statistic, every series and
         # event list), shortened: few long trajectories.
-        one(name="fp64 sample input, 32 long", trajectories=32, steps=160000, freq=80, dt=1e-4, tau=1e-5, full=True,
+        one(name="fp64 sample input 32 long", trajectories=32, steps=160000, freq=80, dt=1e-4, tau=1e-5, full=True,
             frames=True),
         # A study of a double-barrier model on one GPU: some hundred
         # trajectories, the sample inputs' time step.
-        one(name="fp64 double, 900", double=True, trajectories=900, steps=60000, freq=50, dt=1e-4, tau=1e-2),
+        one(name="fp64 double 900", double=True, trajectories=900, steps=60000, freq=50, dt=1e-4, tau=1e-2),
         # A few thousand underdamped trajectories, an odd number of them.
-        one(name="fp64 underdamped, 5003", over=False, trajectories=5003, steps=36000, freq=30),
+        one(name="fp64 underdamped 5003", over=False, trajectories=5003, steps=36000, freq=30),
         # A plain FP64 job of the benchmark's width.
-        one(name="fp64 large, 65536", trajectories=65536, steps=60000, freq=50, tau=0.2),
+        one(name="fp64 large 65536", trajectories=65536, steps=60000, freq=50, tau=0.2),
         # The smallest and an ordinary request of the serving ranges, alone.
-        one(name="fp32 small, 1024", fp32=True, trajectories=1024, steps=24000, freq=20, over=False),
-        one(name="fp32 double, 20011", fp32=True, double=True, trajectories=20011, steps=48000, freq=40, tau=0.1),
+        one(name="fp32 small 1024", fp32=True, trajectories=1024, steps=24000, freq=20, over=False),
+        one(name="fp32 double 20011", fp32=True, double=True, trajectories=20011, steps=48000, freq=40, tau=0.1),
         # The benchmark's batch: jobs of 65536 trajectories with heights and
         # flip rates of the precision workload.
-        many(name="fp32 batch, 4 x 65536", jobs=4, fixed=65536, steps=120000, freq=100, mix="precision"),
+        many(name="fp32 batch 4 x 65536", jobs=4, fixed=65536, steps=120000, freq=100, mix="precision"),
         # The parameter scan: unequal jobs over both dampings in one graph.
-        many(name="fp32 scan graph, 16 sets", kind="graph", jobs=16, lo=10.0, hi=15.0, steps=24000, freq=20, mix="scan"),
+        many(name="fp32 scan graph 16 sets", kind="graph", jobs=16, lo=10.0, hi=15.0, steps=24000, freq=20, mix="scan"),
         # Requests of all four model types served together.
-        many(name="fp32 serving burst, 20 jobs", kind="serve", jobs=20, lo=10.0, hi=15.0, steps=24000, freq=20,
+        many(name="fp32 serving burst 20 jobs", kind="serve", jobs=20, lo=10.0, hi=15.0, steps=24000, freq=20,
              mix="serving"),
         # First passages of the double-barrier model: uneven lengths, capped.
-        many(name="fp32 first passage, 2 x 30000", kind="passage", jobs=2, fixed=30000, cap=100000, mix="passage",
+        many(name="fp32 first passage 2 x 30000", kind="passage", jobs=2, fixed=30000, cap=100000, mix="passage",
              steps=24000, freq=20),
     ]
 
