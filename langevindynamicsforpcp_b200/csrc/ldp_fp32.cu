@@ -17,13 +17,24 @@
 // for the double model, the flank meeting point) neither the force, the
 // cell, the well nor the local barrier changes.  Each thread keeps the open
 // band (lo, hi) around its position, the force of its current barrier state
-// and the high word of its flip threshold in registers, so a step is the
-// Philox/Box-Muller draw, the position update and three compares.  Every
-// step that leaves the band, draws a flip (or a threshold tie), or reaches a
-// frame or the last step takes the general step below, which follows the
-// FP64 step exactly (wrap, indices, flip, cell-table entry with lazy
-// catch-up, force, renewal statistics, frame, end).
+// and a countdown to its next frame, flip or last step in registers.  A block
+// of four steps is one Philox block, two Box-Muller pairs, the four moves and
+// one test for the warp: whether every lane stayed in its band and no
+// countdown ended.  If not (about one block in five), the lanes concerned take
+// the block again step by step.  Their special steps are quick steps, inline
+// (a frame, a flank entered or left, the edge between the two cells of a pair
+// crossed), or take the slow path out of line: a light step, or the general
+// step, which follows the FP64 step exactly (wrap, indices, flip, cell-table
+// entry with lazy catch-up, force, renewal statistics, frame, end).
 //
+// What bounds it: instruction issue.  4 jobs x 65536 trajectories x 120000
+// steps, frames every 100: 76.8 ms with a test and a branch at each step and
+// light steps (an out-of-line call's worth of state around them), 63.0 ms
+// with this loop; 161 instead of 194 warp instructions a block of four steps.
+// Nothing lives in a register across an out-of-line call (the lane state is in
+// shared memory there): with calls inside the loop it spilled at each block
+// (71.4 ms).
+
 // Rare state lives in shared memory (statistics clocks and flags, the cached
 // state of the cell left last, the state-1 step count), counts and duration
 // sums go out as fire-and-forget atomics, and the cell-table ring is written
@@ -53,6 +64,16 @@ enum : uint32_t { B_HAS_FPT = 1u << 24, B_HAS_FPT2 = 1u << 25, B_HAS_TPT = 1u <<
 // the cell left last (valid, its state).
 enum : int32_t { W_LB = 1, W_EVICT = 2, W_CVALID = 4, W_CSTATE = 8 };
 
+// The word of a lane's quick steps (see quick_step), kept in a register by
+// the hot loop: quick steps allowed (the barrier flanks do not reach the cell
+// edges); the lane's cell and a neighbour form a pair whose shared edge it may
+// cross quickly; it is in the pair's other cell now; the other cell is the
+// right neighbour; the two barriers' states; the countdown ends at a frame
+// and nothing else; the pair's edge was crossed at least once.
+enum : uint32_t {
+    P_FAST = 1, P_PAIR = 2, P_SWAP = 4, P_RIGHT = 8, P_S0 = 16, P_S1 = 32, P_FRAME = 64, P_CROSSED = 128
+};
+
 // Per-thread rare state, structure of arrays (conflict-free by thread).
 struct RareSm {
     uint32_t bits[kMaxBlock];
@@ -69,14 +90,18 @@ struct RareSm {
     long long since[kMaxBlock];   // first step of the current state-1 run
     // Lane state the hot loop hands to the general step and takes back, and
     // the lane state only the general step uses.
-    float xp[kMaxBlock], rv[kMaxBlock], F[kMaxBlock], lo[kMaxBlock], hi[kMaxBlock], c1[kMaxBlock];
+    float xp[kMaxBlock], rv[kMaxBlock], F[kMaxBlock], lo[kMaxBlock], hi[kMaxBlock];
+    uint4 fix[kMaxBlock];         // Philox constants of the lane's step blocks (philox_fix) ...
+    uint2 fixk[kMaxBlock];        // ... the first key word of its third round, and the noise scale (float bits)
     uint32_t traj[kMaxBlock];
-    uint32_t gtraj[kMaxBlock];    // the trajectory's random-stream index (traj + the job's g0)
-    uint32_t key0[kMaxBlock], key1[kMaxBlock];
-    float kn[kMaxBlock];
     long long nflip[kMaxBlock];   // step of the current barrier's next flip
     int32_t left[kMaxBlock], job[kMaxBlock], cell[kMaxBlock], state[kMaxBlock], sw[kMaxBlock];
+    uint32_t pw[kMaxBlock];       // P_* word (quick steps)
+    long long nev[kMaxBlock];     // first step that is special for another reason than a frame
+    long long xs[kMaxBlock];      // step of the last quick crossing
+    uint32_t j[kMaxBlock], jh[kMaxBlock];   // next block of four steps, 4j+1 .. 4j+4: j's low and high word
 };
+static_assert(sizeof(RareSm) <= 56 * 1024, "four blocks to an SM");
 
 __device__ __forceinline__ void red_add(int64_t* p, int64_t v) {
     atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)v);
@@ -91,6 +116,37 @@ __device__ __forceinline__ int fkey(bool dbl, int cell, int lb) { return dbl ? c
 __device__ __forceinline__ long long next_flip(const JobF& J, uint32_t traj, uint64_t s, int st) {
     const Words w = philox_at(s, traj, TAG_FLIP, J.key0, J.key1);
     return flip_schedule(s, w.w0, w.w1, J.ln1m[st]);
+}
+
+// The Philox blocks of a lane's steps (counter: block index j, stream g,
+// TAG_STEP = 0) differ only in j, and its high word changes every 2^34 steps.
+// The products of g, hence the first round's second half and the second
+// round's first multiply, are the same for all of them: philox_fix holds what
+// follows from them, philox_step takes it from there (17 wide multiplies and
+// 19 xors instead of 20 and 20, 15 key additions instead of 18); the words
+// are philox's.
+__device__ __forceinline__ uint4 philox_fix(uint32_t g, uint32_t jh, uint32_t k0, uint32_t k1) {
+    const uint64_t p1 = (uint64_t)g * 0xCD9E8D57u;
+    const uint32_t c0 = (uint32_t)(p1 >> 32) ^ jh ^ k0;   // after round 1 (its c1 is (uint32_t)p1)
+    const uint64_t p0 = (uint64_t)c0 * 0xD2511F53u;       // of round 2
+    return make_uint4(k1, (uint32_t)p1 ^ (k0 + 0x9E3779B9u), (uint32_t)(p0 >> 32) ^ (k1 + 0xBB67AE85u), (uint32_t)p0);
+}
+__device__ __forceinline__ Words philox_step(uint32_t jl, uint4 fix, uint32_t k0) {
+    const uint64_t q0 = (uint64_t)jl * 0xD2511F53u;       // round 1
+    const uint64_t q1 = (uint64_t)((uint32_t)(q0 >> 32) ^ fix.x) * 0xCD9E8D57u;   // round 2
+    uint32_t c0 = (uint32_t)(q1 >> 32) ^ fix.y, c1 = (uint32_t)q1, c2 = (uint32_t)q0 ^ fix.z, c3 = fix.w;
+    uint32_t k1 = fix.x + 2u * 0xBB67AE85u;
+#pragma unroll
+    for (int r = 2; r < 10; ++r) {
+        if (r > 2) { k0 += 0x9E3779B9u; k1 += 0xBB67AE85u; }
+        const uint64_t p0 = (uint64_t)c0 * 0xD2511F53u;
+        const uint64_t p1 = (uint64_t)c2 * 0xCD9E8D57u;
+        c0 = (uint32_t)(p1 >> 32) ^ c1 ^ k0;
+        c2 = (uint32_t)(p0 >> 32) ^ c3 ^ k1;
+        c1 = (uint32_t)p1;
+        c3 = (uint32_t)p0;
+    }
+    return Words{c0, c1, c2, c3};
 }
 
 // Uniform in (0, 1): the high 23 bits of w as a mantissa, offset by 2^-24.
@@ -231,10 +287,12 @@ __device__ __forceinline__ bool cg_hit32(int well, int size) { return (well % si
 // state is rounded to FP32.  Writes the thread's rare state.
 template <bool DBL, bool OVER>
 __device__ __noinline__ void f_start(const JobF* Jp, longlong2* ring, int64_t nslots, int ring_slots, int64_t slot,
-                                     uint32_t traj, RareSm* sm, int t, float* xp, float* rv, int* cell, int* state,
-                                     int* sw) {
+                                     uint32_t traj, RareSm* sm, int t) {
     const JobF& J = *Jp;
     const uint32_t g = traj + J.g0;   // the trajectory's random streams
+    float* xp = &sm->xp[t];
+    float* rv = &sm->rv[t];
+    int32_t *cell = &sm->cell[t], *state = &sm->state[t], *sw = &sm->sw[t];
     if (J.resume) {
         // Continue from the state kept at step S = step0 - 1: the ring, the
         // hot state, the statistics clocks; the state-1 steps counted so far
@@ -409,6 +467,19 @@ __device__ __noinline__ void f_keep_state(const JobF* Jp, const SlotsDev* Sp, co
     J.tpt2_last[traj] = sm.tpt2[t];
 }
 
+// A lane without a trajectory: at rest in an unbounded band.
+__device__ __forceinline__ void idle_lane(RareSm& sm, int t) {
+    const float kInf = __int_as_float(0x7f800000);
+    sm.job[t] = -1;
+    sm.xp[t] = sm.rv[t] = sm.F[t] = 0.f;
+    sm.lo[t] = -kInf;
+    sm.hi[t] = kInf;
+    sm.fixk[t] = make_uint2(0u, 0u);   // no noise
+    sm.left[t] = kLeftMax;
+    sm.pw[t] = 0;
+    sm.j[t] = sm.jh[t] = 0;
+}
+
 // Ends a lane's trajectory after step `done` (general step): keeps its
 // continuation state when the job asks for it and the trajectory completed,
 // then retires it.  The lane's cell, state and slot word in sm are current.
@@ -423,11 +494,10 @@ __device__ __noinline__ void f_end_lane(const JobF* Jp, const SlotsDev* Sp, Rare
 }
 
 // The general step s of one lane (position already advanced):
-// the FP64 step order of ldp_fp64.cu from the index update on.  Out of line,
-// on the lane state in shared memory, so that the hot loop's registers do
-// not carry its working set.
+// the FP64 step order of ldp_fp64.cu from the index update on, on the lane
+// state in shared memory.
 template <bool DBL, bool OVER>
-__device__ __noinline__ void general_step(const JobF* jobs, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
+__device__ __forceinline__ void general_step(const JobF* jobs, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
                                           uint64_t s) {
     RareSm& sm = *smp;
     const SlotsDev& S = *Sp;
@@ -448,11 +518,7 @@ __device__ __noinline__ void general_step(const JobF* jobs, const SlotsDev* Sp, 
         sm.state[t] = state;
         sm.sw[t] = sw;
         f_end_lane<OVER>(&J, &S, &sm, t, slot, done, xp, v, rv, flags);
-        sm.job[t] = -1;
-        sm.lo[t] = -kInf;
-        sm.hi[t] = kInf;
-        sm.F[t] = 0.f;
-        sm.left[t] = kLeftMax;
+        idle_lane(sm, t);
     };
 
     // Cell (double model: local barrier) entry (UpdateBarrierStateEta,
@@ -631,7 +697,7 @@ __device__ __noinline__ void general_step(const JobF* jobs, const SlotsDev* Sp, 
     if (xp > lo && xp < hi && (long long)s != sm.nflip[t]) {
         // Only the countdown ran out: a frame and/or the last step.
         const float F = sm.F[t];
-        const float vk = OVER ? 0.0f : fmaf(F, sm.c1[t], rv);
+        const float vk = OVER ? 0.0f : fmaf(F, J.hdt_invM, rv);
         if ((long long)s == sm.nxf[t]) {
             f_record<DBL>(J, traj, sm.fidx[t], cell, xp, vk, F, state);
             sm.fidx[t] += 1;
@@ -691,7 +757,7 @@ __device__ __noinline__ void general_step(const JobF* jobs, const SlotsDev* Sp, 
     const float F = force_of<DBL>(J, xp, state);
     bool finish = false;
     if (dCell || dWell) finish = events((int64_t)s, dWell, dCell, well);
-    const float vk = OVER ? 0.0f : fmaf(F, sm.c1[t], rv);
+    const float vk = OVER ? 0.0f : fmaf(F, J.hdt_invM, rv);
     if (left == 0) {
         if ((long long)s == sm.nxf[t]) {
             f_record<DBL>(J, traj, sm.fidx[t], cell, xp, vk, F, state);
@@ -712,11 +778,9 @@ __device__ __noinline__ void general_step(const JobF* jobs, const SlotsDev* Sp, 
     if (finish) retire(s, vk, 0);
 }
 
-// The light step: the commonest special steps, handled in the hot loop
-// with the same result the general step gives them, so that the warp does
-// not pay for the out-of-line call.  Returns 0 when the step needs the
-// general step; 1 when it was handled and the countdown is unchanged; 2 when
-// it was handled and *lrel holds the steps from s to the next special step.
+// The light step: special steps with few consequences, with the same result
+// the general step gives them.  Returns false when the step needs the general
+// step.
 //  * A frame step (the countdown ends at a frame, not at a flip or the last
 //    step), the position inside its band, no WRITEX series: the frame is
 //    written (FP64 cell * L + xp) and the countdown restarts.
@@ -729,24 +793,21 @@ __device__ __noinline__ void general_step(const JobF* jobs, const SlotsDev* Sp, 
 //    pending flip and state-1 run change as in the general step's cell
 //    entry, the ring is written through, the transition-path clocks restart.
 template <bool DBL>
-__device__ __forceinline__ int light_step(const JobF* jobs, const SlotsDev& S, RareSm& sm, int t, int64_t slot,
-                                          int job, uint32_t traj, uint64_t s, bool countdown, float& xp, float& lo,
-                                          float& hi, float& F, int& lrel) {
-    const JobF& J = jobs[job];
+__device__ __forceinline__ bool light_step(const JobF& J, const SlotsDev& S, RareSm& sm, int t, int64_t slot,
+                                           uint32_t traj, uint64_t s, bool countdown, float& xp, float& lo, float& hi,
+                                           float& F) {
     const long long nflip = sm.nflip[t];
     if (countdown) {
         const long long nxf = sm.nxf[t];
         if (!(xp > lo && xp < hi) || (long long)s != nxf || (long long)s == nflip || s == J.nsteps || J.write_x)
-            return 0;
+            return false;
         const int fidx = sm.fidx[t];
         if (fidx < J.nframe && J.fx) J.fx[(int64_t)fidx * J.ntraj + traj] = (double)sm.cell[t] * J.Ld + (double)xp;
         sm.fidx[t] = fidx + 1;
-        const long long nx2 = nxf + (long long)J.freq_save;
-        sm.nxf[t] = nx2;
-        lrel = steps_to_special(J, s, nx2, nflip);
-        return 2;
+        sm.nxf[t] = nxf + (long long)J.freq_save;
+        return true;
     }
-    if ((long long)s == nflip) return 0;
+    if ((long long)s == nflip) return false;
     const float hL = J.halfL;
     int sw = sm.sw[t];
     if (xp >= -hL && xp < hL) {
@@ -754,42 +815,42 @@ __device__ __forceinline__ int light_step(const JobF* jobs, const SlotsDev& S, R
         // barrier changes, or xp sits on a breakpoint
         float l2, h2;
         band_of<DBL>(J, xp, &l2, &h2);
-        if (!(xp > l2 && xp < h2)) return 0;
-        if ((xp < 0.0f) != (lo < 0.0f)) return 0;
-        if (DBL && ((xp < J.xc ? 0 : W_LB) != (sw & W_LB))) return 0;
+        if (!(xp > l2 && xp < h2)) return false;
+        if ((xp < 0.0f) != (lo < 0.0f)) return false;
+        if (DBL && ((xp < J.xc ? 0 : W_LB) != (sw & W_LB))) return false;
         lo = l2;
         hi = h2;
         F = force_of<DBL>(J, xp, sm.state[t]);
-        return 1;
+        return true;
     }
-    if (!J.edge_flat || !J.eta) return 0;
+    if (!J.edge_flat || !J.eta) return false;
     float xn;
     int dc;
     if (xp >= hL) {
         xn = xp - J.L;
         dc = 1;
-        if (!(xn > -hL && xn < J.edge_lo)) return 0;
+        if (!(xn > -hL && xn < J.edge_lo)) return false;
     } else if (xp < -hL) {
         xn = xp + J.L;
         dc = -1;
-        if (!(xn > J.edge_hi && xn < hL)) return 0;
+        if (!(xn > J.edge_hi && xn < hL)) return false;
     } else {
-        return 0;   // not finite
+        return false;   // not finite
     }
     const int cell_prev = sm.cell[t], cell = cell_prev + dc;
     const int well = cell - (xn < 0.0f ? 1 : 0);
-    if (well != cell_prev - (lo < 0.0f ? 1 : 0)) return 0;
+    if (well != cell_prev - (lo < 0.0f ? 1 : 0)) return false;
     const int lb = DBL ? (xn < J.xc ? 0 : 1) : 0;
-    if (DBL && lb == (sw & W_LB)) return 0;   // the general step enters a key only when lb changes
+    if (DBL && lb == (sw & W_LB)) return false;   // the general step enters a key only when lb changes
     const int key_prev = fkey(DBL, cell_prev, sw & W_LB), key = fkey(DBL, cell, lb);
-    if (!(sw & W_CVALID) || sm.ckey[t] != key || sm.cflip[t] <= (long long)s) return 0;
+    if (!(sw & W_CVALID) || sm.ckey[t] != key || sm.cflip[t] <= (long long)s) return false;
     const uint32_t bits = sm.bits[t];
     const int evm = J.evm;
-    if ((evm & EV_FPT) && (bits & B_FPT_UP)) return 0;
-    if ((evm & EV_FPT2) && ((bits & B_FPT2_UP) || sm.idx2[t] != well)) return 0;
-    if ((evm & EV_TPT) && !(bits & B_TPT2_UP) && sm.tpt2w[t] != well) return 0;
-    if ((evm & EV_CG) && sm.cgw[t] != well) return 0;
-    if ((evm & EV_WT) && (bits & B_WT_PASSED)) return 0;
+    if ((evm & EV_FPT) && (bits & B_FPT_UP)) return false;
+    if ((evm & EV_FPT2) && ((bits & B_FPT2_UP) || sm.idx2[t] != well)) return false;
+    if ((evm & EV_TPT) && !(bits & B_TPT2_UP) && sm.tpt2w[t] != well) return false;
+    if ((evm & EV_CG) && sm.cgw[t] != well) return false;
+    if ((evm & EV_WT) && (bits & B_WT_PASSED)) return false;
     // leave key_prev (its eviction, if its entry displaced another cell's,
     // is counted now), enter the cached key
     const int st_prev = sm.state[t];
@@ -819,8 +880,251 @@ __device__ __forceinline__ int light_step(const JobF* jobs, const SlotsDev& S, R
     if (dc > 0) { lo = -hL; hi = J.edge_lo; }
     else { lo = J.edge_hi; hi = hL; }
     F = 0.0f;
-    lrel = steps_to_special(J, s, sm.nxf[t], nb);
-    return 2;
+    return true;
+}
+
+// The last step after s whose block index has the same high word as the
+// next step's: a special step, since the lane's Philox constants hold it.
+__device__ __forceinline__ long long block_wrap(uint64_t s) { return (long long)(((s >> 34) + 1) << 34); }
+
+// The high word of the lane's block index and its Philox constants for next
+// step s + 1.
+__device__ __forceinline__ void bind_block(const JobF& J, RareSm& sm, int t, uint64_t s) {
+    sm.jh[t] = (uint32_t)(s >> 34);
+    sm.fix[t] = philox_fix(sm.traj[t] + J.g0, (uint32_t)(s >> 34), J.key0, J.key1);
+    sm.fixk[t] = make_uint2(J.key0 + 2u * 0x9E3779B9u, __float_as_uint(J.bm_k));
+}
+
+// After a special step s (or before the first step, s one less): the word of
+// the lane's quick steps and its countdown.  A pair is formed when a crossing
+// of the nearer cell edge would be a light crossing (light_step) and stays
+// one, whatever the number of crossings, until the next special step: the
+// neighbour is the cached cell, no statistic fires, no eviction is pending.
+// The countdown also ends at the neighbour's pending flip, past which its
+// cached state is no longer known.
+template <bool DBL>
+__device__ __forceinline__ void settle(const JobF& J, RareSm& sm, int t, uint64_t s, float xp) {
+    const int state = sm.state[t], sw = sm.sw[t], cell = sm.cell[t];
+    uint32_t pw = (state ? P_S0 : 0u) | (J.edge_flat ? P_FAST : 0u);
+    long long nev = sm.nflip[t] < (long long)J.nsteps ? sm.nflip[t] : (long long)J.nsteps;
+    const long long wrap = block_wrap(s);
+    nev = wrap < nev ? wrap : nev;
+    if ((s & ((1ull << 34) - 1)) == 0) bind_block(J, sm, t, s);   // a new high word from the next step on
+    if (J.edge_flat && J.eta && (sw & W_CVALID) && !(sw & W_EVICT) && sm.cflip[t] > (long long)s) {
+        const bool right = !(xp < 0.0f);
+        const int lb = sw & W_LB;
+        const int well = cell - (right ? 0 : 1);
+        const int key = fkey(DBL, right ? cell + 1 : cell - 1, lb ^ 1);
+        const uint32_t bits = sm.bits[t];
+        const int evm = J.evm;
+        bool ok = sm.ckey[t] == key && (!DBL || (lb != 0) == right);
+        ok = ok && !((evm & EV_FPT) && (bits & B_FPT_UP));
+        ok = ok && !((evm & EV_FPT2) && ((bits & B_FPT2_UP) || sm.idx2[t] != well));
+        ok = ok && !((evm & EV_TPT) && !(bits & B_TPT2_UP) && sm.tpt2w[t] != well);
+        ok = ok && !((evm & EV_CG) && sm.cgw[t] != well);
+        ok = ok && !((evm & EV_WT) && (bits & B_WT_PASSED));
+        if (ok) {
+            pw |= P_PAIR | (right ? P_RIGHT : 0u) | ((sw & W_CSTATE) ? P_S1 : 0u);
+            nev = sm.cflip[t] < nev ? sm.cflip[t] : nev;
+        }
+    }
+    const long long nxf = sm.nxf[t];
+    const long long d = (nxf < nev ? nxf : nev) - (long long)s;
+    if (nxf < nev && d <= (long long)kLeftMax && !J.write_x) pw |= P_FRAME;
+    sm.nev[t] = nev;
+    sm.left[t] = (int)(d < (long long)kLeftMax ? d : (long long)kLeftMax);
+    sm.pw[t] = pw;
+}
+
+// Leaves a pair: the lane state as light crossings would have left it (the
+// ring entry of the cell first left, the transition-path clocks, and, in the
+// pair's other cell, the swapped barriers).
+template <bool DBL>
+__device__ __forceinline__ void unpair(const JobF& J, const SlotsDev& S, RareSm& sm, int t, int64_t slot, uint32_t pw) {
+    if (!(pw & P_CROSSED)) return;
+    const int cell = sm.cell[t], sw = sm.sw[t];
+    const int key = fkey(DBL, cell, sw & W_LB);
+    const int st = (pw & P_S0) ? 1 : 0;
+    const long long nf = sm.nflip[t];
+    S.ring[(int64_t)(key & (S.ring_slots - 1)) * S.nslots + slot] =
+        make_longlong2((long long)key, (nf << 1) | (long long)st);
+    if (J.evm & EV_TPT) {
+        const long long xs = sm.xs[t];
+        sm.bits[t] &= ~(B_TPT_UP | B_TPT2_UP);
+        sm.tpt[t] = xs;
+        sm.tpt2[t] = xs;
+        sm.tpt2w[t] = cell - ((pw & P_RIGHT) ? 0 : 1);
+    }
+    if (pw & P_SWAP) {
+        sm.cell[t] = cell + ((pw & P_RIGHT) ? 1 : -1);
+        sm.state[t] = (pw & P_S1) ? 1 : 0;
+        sm.ckey[t] = key;
+        sm.nflip[t] = sm.cflip[t];
+        sm.cflip[t] = nf;
+        sm.sw[t] = (DBL ? ((sw & W_LB) ^ W_LB) : (sw & W_LB)) | W_CVALID | (st ? W_CSTATE : 0);
+    }
+}
+
+// A special step that is not a quick one: out of line, on the lane state in
+// shared memory, so that the hot loop's registers do not carry its working
+// set.  sm.left: 0 when the countdown ends at s.
+template <bool DBL, bool OVER>
+__device__ __noinline__ void special_step(const JobF* jobs, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
+                                          uint64_t s) {
+    RareSm& sm = *smp;
+    const SlotsDev& S = *Sp;
+    const int job = sm.job[t];
+    if (job < 0) {
+        sm.left[t] = kLeftMax;
+        return;
+    }
+    const JobF& J = jobs[job];
+    unpair<DBL>(J, S, sm, t, slot, sm.pw[t]);
+    float xp = sm.xp[t], lo = sm.lo[t], hi = sm.hi[t], F = sm.F[t];
+    if (light_step<DBL>(J, S, sm, t, slot, sm.traj[t], s, sm.left[t] == 0, xp, lo, hi, F)) {
+        sm.xp[t] = xp;
+        sm.lo[t] = lo;
+        sm.hi[t] = hi;
+        sm.F[t] = F;
+    } else {
+        general_step<DBL, OVER>(jobs, Sp, smp, t, slot, s);
+        if (sm.job[t] < 0) return;
+        xp = sm.xp[t];
+    }
+    settle<DBL>(J, sm, t, s, xp);
+}
+
+// The quick steps: the commonest special steps, in the hot loop, with the
+// state a light step leaves (unpair fills in what a pair's crossings leave
+// open).  Returns false when the step needs special_step.
+//  * A frame, the position inside its band.
+//  * A band change inside the cell (a flank entered or left) that changes
+//    neither the well nor the local barrier.
+//  * A crossing of the pair's edge into the flat band of the other cell: the
+//    barriers change places.
+template <bool DBL>
+__device__ __forceinline__ bool quick_step(const JobF& J, RareSm& sm, int t, uint64_t s, bool countdown, float& xp,
+                                           float& lo, float& hi, float& F, int& left, uint32_t& pw) {
+    const uint32_t swapped = pw & P_SWAP;
+    if (countdown) {
+        if (!(pw & P_FRAME) || !(xp > lo && xp < hi)) return false;
+        const int fidx = sm.fidx[t];
+        int cell = sm.cell[t];
+        if (swapped) cell += (pw & P_RIGHT) ? 1 : -1;
+        if (fidx < J.nframe && J.fx) J.fx[(int64_t)fidx * J.ntraj + sm.traj[t]] = (double)cell * J.Ld + (double)xp;
+        sm.fidx[t] = fidx + 1;
+        const long long nxf = sm.nxf[t] + (long long)J.freq_save, nev = sm.nev[t];
+        sm.nxf[t] = nxf;
+        const long long d = (nxf < nev ? nxf : nev) - (long long)s;
+        if (!(nxf < nev && d <= (long long)kLeftMax)) pw &= ~P_FRAME;
+        left = (int)(d < (long long)kLeftMax ? d : (long long)kLeftMax);
+        return true;
+    }
+    if (!(pw & P_FAST)) return false;
+    const float hL = J.halfL;
+    const int st = (swapped ? pw & P_S1 : pw & P_S0) ? 1 : 0;
+    if (fabsf(xp) < hL) {
+        if ((xp < 0.0f) != (lo < 0.0f)) return false;
+        if (!DBL) {
+            const float a = fabsf(xp), w = J.w;
+            if (a == w || a == 0.0f) return false;
+            const bool in = a < w, neg = xp < 0.0f;
+            const float m0 = in ? 0.0f : w, m1 = in ? w : hL;
+            lo = neg ? -m1 : m0;
+            hi = neg ? -m0 : m1;
+            F = in ? copysignf(J.slope[st], xp) : 0.0f;
+        } else {
+            const float xc = J.xc;
+            if ((xp < xc) != (lo < xc)) return false;   // lo < xc: local barrier 0
+            float l2, h2;
+            band_of<DBL>(J, xp, &l2, &h2);
+            if (!(xp > l2 && xp < h2)) return false;
+            lo = l2;
+            hi = h2;
+            F = force_of<DBL>(J, xp, st);
+        }
+        return true;
+    }
+    if (!(pw & P_PAIR)) return false;
+    const bool right = ((pw & P_RIGHT) != 0u) != (swapped != 0u);   // the pair's other cell is the right neighbour
+    const float xn = right ? xp - J.L : xp + J.L;
+    const float e1 = right ? -hL : J.edge_hi, e2 = right ? J.edge_lo : hL;
+    if (!(right ? xp >= hL : xp < -hL) || !(xn > e1 && xn < e2)) return false;
+    pw = (pw ^ P_SWAP) | P_CROSSED;
+    sm.xs[t] = (long long)s;
+    if (((pw & P_S0) != 0u) != ((pw & P_S1) != 0u)) {
+        if (st) sm.sc1[t] += (long long)s - sm.since[t];
+        else sm.since[t] = (long long)s;
+    }
+    xp = xn;
+    lo = e1;
+    hi = e2;
+    F = 0.0f;
+    return true;
+}
+
+// One step's move.
+template <bool OVER>
+__device__ __forceinline__ void f_move(float& xp, float& rv, float F, float c1, float c2, float c3, float nz) {
+    if (OVER) {
+        xp = fmaf(F, c1, xp);
+        xp = xp + nz;
+        xp = xp + rv;
+        rv = nz;
+    } else {
+        rv = fmaf(F, c1, rv);
+        xp = fmaf(rv, c2, xp);
+        rv = fmaf(c3, rv, nz);
+        xp = fmaf(rv, c2, xp);
+    }
+}
+
+// One lane's steps 4j+1+h .. 4j+4 one by one, step 4j+1+h a special one that
+// is moved already; the block's noise is drawn again.  Out of line, on the
+// lane state in shared memory.
+template <bool DBL, bool OVER>
+__device__ __noinline__ void slow_steps(const JobF* jobs, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
+                                        uint64_t j, int h) {
+    RareSm& sm = *smp;
+    const float kn = __uint_as_float(sm.fixk[t].y);
+    const Words w = philox_step((uint32_t)j, sm.fix[t], sm.fixk[t].x);
+    float n[4];
+    noise_pair(w.w0, w.w1, kn, &n[0], &n[1]);
+    noise_pair(w.w2, w.w3, kn, &n[2], &n[3]);
+    int job = sm.job[t];
+    bool moved = true;
+#pragma unroll 1
+    for (; h < 4; ++h) {
+        const JobF& J = jobs[job < 0 ? 0 : job];
+        const float c1 = OVER ? J.c_drift : J.hdt_invM;
+        if (!moved && job >= 0) {
+            float xp = sm.xp[t], rv = sm.rv[t];
+            f_move<OVER>(xp, rv, sm.F[t], c1, J.hdt, J.expg, h == 1 ? n[1] : h == 2 ? n[2] : n[3]);
+            sm.xp[t] = xp;
+            sm.rv[t] = rv;
+            sm.left[t] -= 1;
+        }
+        const float xp = sm.xp[t];
+        if (moved || !(xp > sm.lo[t] && xp < sm.hi[t]) || sm.left[t] == 0) {
+            special_step<DBL, OVER>(jobs, Sp, smp, t, slot, 4 * j + 1 + h);
+            job = sm.job[t];
+            if (job < 0) {
+                sm.rv[t] = 0.f;
+                return;
+            }
+        }
+        if (!OVER) sm.rv[t] = fmaf(sm.F[t], c1, sm.rv[t]);
+        moved = false;
+    }
+}
+
+// Lowest and highest of four, NaN if one is.
+__device__ __forceinline__ void range4(float a, float b, float c, float d, float* mn, float* mx) {
+    float u, v;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(u) : "f"(a), "f"(b), "f"(c));
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(a), "f"(b), "f"(c));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(*mn) : "f"(u), "f"(d));
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(*mx) : "f"(v), "f"(d));
 }
 
 }  // namespace
@@ -832,222 +1136,281 @@ __device__ __forceinline__ int light_step(const JobF* jobs, const SlotsDev& S, R
 #define LDP_FP32_MIN_BLOCKS 3
 #endif
 
+namespace {
+
+// A lane's per-job constants, band, force and countdown from its position
+// (sm.xp) and statistics state; s: its next step.
+template <bool DBL>
+__device__ __forceinline__ void bind_lane(const JobF& J, RareSm& sm, int t, uint32_t traj, uint64_t s) {
+    sm.traj[t] = traj;
+    sm.j[t] = (uint32_t)((s - 1) >> 2);
+    bind_block(J, sm, t, s - 1);
+    const float xp = sm.xp[t];
+    float lo, hi;
+    band_of<DBL>(J, xp, &lo, &hi);
+    sm.lo[t] = lo;
+    sm.hi[t] = hi;
+    sm.F[t] = force_of<DBL>(J, xp, sm.state[t]);
+    settle<DBL>(J, sm, t, s - 1, xp);
+}
+
+// The state a slot kept since the last launch, into sm.
+template <bool DBL>
+__device__ __noinline__ void load_slot(const QueueDev* qp, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot) {
+    const SlotsDev& S = *Sp;
+    RareSm& sm = *smp;
+    idle_lane(sm, t);
+    const int job = (slot < S.nslots) ? S.job[slot] : -1;
+    if (job < 0) return;
+    const JobF& J = qp->jobs[job];
+    const uint32_t traj = (uint32_t)S.traj[slot];
+    const uint64_t s = (uint64_t)S.step[slot];
+    sm.job[t] = job;
+    sm.xp[t] = S.xp[slot];
+    sm.rv[t] = S.rv[slot];
+    sm.cell[t] = S.cell[slot];
+    const int st = S.st[slot];
+    sm.state[t] = st & 1;
+    sm.sw[t] = st >> 1;
+    sm.bits[t] = (uint32_t)J.bits[traj];
+    sm.init0[t] = J.init_idx0[traj];
+    sm.idx2[t] = J.idx2_0[traj];
+    sm.tpt2w[t] = J.tpt2_well[traj];
+    sm.fpt[t] = J.fpt_last[traj];
+    sm.fpt2[t] = J.fpt2_last[traj];
+    sm.tpt[t] = J.tpt_last[traj];
+    sm.tpt2[t] = J.tpt2_last[traj];
+    sm.ckey[t] = S.ckey[slot];
+    sm.cflip[t] = S.cflip[slot];
+    sm.sc1[t] = S.sc1[slot];
+    sm.since[t] = S.since[slot];
+    sm.cgw[t] = S.cgw[slot];
+    sm.fidx[t] = S.fidx[slot];
+    sm.nxf[t] = S.nxf[slot];
+    sm.nflip[t] = S.nflip[slot];
+    bind_lane<DBL>(J, sm, t, traj, s);
+}
+
+// A lane's state into its slot, until the next launch.
+template <bool DBL>
+__device__ __noinline__ void save_slot(const QueueDev* qp, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot) {
+    const SlotsDev& S = *Sp;
+    RareSm& sm = *smp;
+    if (slot >= S.nslots) return;
+    const int job = sm.job[t];
+    S.job[slot] = job;
+    if (job < 0) return;
+    const JobF& J = qp->jobs[job];
+    const uint32_t traj = sm.traj[t];
+    unpair<DBL>(J, S, sm, t, slot, sm.pw[t]);
+    S.traj[slot] = traj;
+    S.step[slot] = (int64_t)(((uint64_t)sm.jh[t] << 34 | (uint64_t)sm.j[t] << 2) + 1);
+    S.xp[slot] = sm.xp[t];
+    S.rv[slot] = sm.rv[t];
+    S.cell[slot] = sm.cell[t];
+    S.st[slot] = sm.state[t] | (sm.sw[t] << 1);
+    S.ckey[slot] = sm.ckey[t];
+    S.cflip[slot] = sm.cflip[t];
+    S.sc1[slot] = sm.sc1[t];
+    S.since[slot] = sm.since[t];
+    S.cgw[slot] = sm.cgw[t];
+    S.fidx[slot] = sm.fidx[t];
+    S.nxf[slot] = sm.nxf[t];
+    S.nflip[slot] = sm.nflip[t];
+    J.bits[traj] = (int32_t)sm.bits[t];
+    J.init_idx0[traj] = sm.init0[t];
+    J.idx2_0[traj] = sm.idx2[t];
+    J.tpt2_well[traj] = sm.tpt2w[t];
+    J.fpt_last[traj] = sm.fpt[t];
+    J.fpt2_last[traj] = sm.fpt2[t];
+    J.tpt_last[traj] = sm.tpt[t];
+    J.tpt2_last[traj] = sm.tpt2[t];
+}
+
+// Warp-aggregated refill of the warp's idle lanes (all lanes call): lanes
+// with `need` claim trajectories from the queue.  Returns whether the queue
+// had fewer than the lanes wanted.
+template <bool DBL, bool OVER>
+__device__ __noinline__ bool refill(const QueueDev* qp, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
+                                    bool need) {
+    const QueueDev& q = *qp;
+    const SlotsDev& S = *Sp;
+    RareSm& sm = *smp;
+    const unsigned m = __ballot_sync(kFull, need);
+    if (!m) return false;
+    const unsigned lane = t & 31u;
+    const int leader = __ffs(m) - 1;
+    unsigned long long base = 0, got = 0;
+    if ((int)lane == leader) {
+        // One fetch-and-add per warp.  A claim that runs past the
+        // tail gets the part below it; the overshoot of head is
+        // clamped back to the tail when more work is published
+        // (fp32_publish_kernel, stream-ordered between launches).
+        const unsigned long long tail = *(volatile unsigned long long*)q.tail;
+        if (*(volatile unsigned long long*)q.head < tail) {
+            const unsigned long long want = (unsigned long long)__popc(m);
+            const unsigned long long old = atomicAdd(q.head, want);
+            if (old < tail) {
+                base = old;
+                got = min(want, tail - old);
+            }
+        }
+    }
+    base = __shfl_sync(kFull, base, leader);
+    got = __shfl_sync(kFull, got, leader);
+    const unsigned rank = __popc(m & ((1u << lane) - 1u));
+    if (need && rank < got) {
+        int job;
+        const uint32_t traj = (uint32_t)f_resolve(q.range_end, q.range_job, q.range_first, q.nranges,
+                                                  (int64_t)(base + rank), &job);
+        const JobF* Jn = &q.jobs[job];
+        f_start<DBL, OVER>(Jn, S.ring, S.nslots, S.ring_slots, slot, traj, &sm, t);
+        sm.job[t] = job;
+        bind_lane<DBL>(*Jn, sm, t, traj, Jn->step0);
+        if (Jn->nsteps == 0) {
+            retire_lane<OVER>(*Jn, S.retired, sm, t, 0, sm.xp[t], sm.rv[t], 0);
+            idle_lane(sm, t);
+        }
+    }
+    return got < (unsigned long long)__popc(m);
+}
+
+}  // namespace
+
 // The persistent loop of one model type for the calling warp: its slots'
 // trajectories (and new ones claimed from queue q) for up to quad_budget
 // blocks of four steps.  Returns the blocks run; *drained is set when it
 // stopped early because every lane of the warp was idle and the queue had
 // nothing left for it.  Slot state is loaded at entry and saved at exit.
+//
+// The hot lane state is in registers inside the loop and in sm across the
+// out-of-line calls, so that no register lives across one (the loop spilled
+// with them).
 template <bool DBL, bool OVER>
 __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const SlotsDev& S, RareSm& sm,
                                                    uint32_t quad_budget, bool* drained) {
     const int t = threadIdx.x;
     const int64_t slot = (int64_t)blockIdx.x * blockDim.x + t;
-    const unsigned lane = t & 31u;
-    const float kInf = __int_as_float(0x7f800000);
 
-    // ---- hot lane state (registers); the rest lives in sm ----
-    int job = (slot < S.nslots) ? S.job[slot] : -1;
-    uint64_t j = 0;                 // next block of four steps: 4j+1 .. 4j+4
-    float xp = 0.f, rv = 0.f, F = 0.f, lo = -kInf, hi = kInf;
-    int left = kLeftMax;
+    int job, left;
+    uint32_t j;   // low word
+    float xp, rv, F, lo, hi;
     float c1 = 0.f, c2 = 0.f, c3 = 0.f;
-    sm.job[t] = job;
-
-    // Per-job constants into registers; band, force and countdown from the
-    // position.  s = next step.
-    auto bind = [&](uint32_t traj, uint64_t s) {
-        const JobF& J = q.jobs[job];
-        if (OVER) c1 = J.c_drift;
-        else { c1 = J.hdt_invM; c2 = J.hdt; c3 = J.expg; }
-        sm.c1[t] = c1;
-        sm.traj[t] = traj;
-        sm.kn[t] = J.bm_k;
-        sm.key0[t] = J.key0;
-        sm.key1[t] = J.key1;
-        sm.gtraj[t] = traj + J.g0;
-        const int state = sm.state[t];
-        band_of<DBL>(J, xp, &lo, &hi);
-        F = force_of<DBL>(J, xp, state);
-        left = steps_to_special(J, s - 1, sm.nxf[t], sm.nflip[t]);
-        j = (s - 1) >> 2;
+    uint32_t pw;
+    auto load = [&]() {
+        job = sm.job[t];
+        xp = sm.xp[t];
+        rv = sm.rv[t];
+        F = sm.F[t];
+        lo = sm.lo[t];
+        hi = sm.hi[t];
+        left = sm.left[t];
+        pw = sm.pw[t];
+        j = sm.j[t];
+        c1 = c2 = c3 = 0.f;
+        if (job >= 0) {
+            const JobF& J = q.jobs[job];
+            if (OVER) c1 = J.c_drift;
+            else { c1 = J.hdt_invM; c2 = J.hdt; c3 = J.expg; }
+        }
     };
-
-    if (job >= 0) {
-        const JobF& J = q.jobs[job];
-        const uint32_t traj = (uint32_t)S.traj[slot];
-        const uint64_t s = (uint64_t)S.step[slot];
-        xp = S.xp[slot];
-        rv = S.rv[slot];
-        sm.cell[t] = S.cell[slot];
-        const int st = S.st[slot];
-        sm.state[t] = st & 1;
-        sm.sw[t] = st >> 1;
-        sm.bits[t] = (uint32_t)J.bits[traj];
-        sm.init0[t] = J.init_idx0[traj];
-        sm.idx2[t] = J.idx2_0[traj];
-        sm.tpt2w[t] = J.tpt2_well[traj];
-        sm.fpt[t] = J.fpt_last[traj];
-        sm.fpt2[t] = J.fpt2_last[traj];
-        sm.tpt[t] = J.tpt_last[traj];
-        sm.tpt2[t] = J.tpt2_last[traj];
-        sm.ckey[t] = S.ckey[slot];
-        sm.cflip[t] = S.cflip[slot];
-        sm.sc1[t] = S.sc1[slot];
-        sm.since[t] = S.since[slot];
-        sm.cgw[t] = S.cgw[slot];
-        sm.fidx[t] = S.fidx[slot];
-        sm.nxf[t] = S.nxf[slot];
-        sm.nflip[t] = S.nflip[slot];
-        bind(traj, s);
-    }
+    auto save = [&]() {
+        sm.xp[t] = xp;
+        sm.rv[t] = rv;
+        sm.F[t] = F;
+        sm.lo[t] = lo;
+        sm.hi[t] = hi;
+        sm.left[t] = left;
+        sm.pw[t] = pw;
+        sm.j[t] = j;
+    };
+    load_slot<DBL>(&q, &S, &sm, t, slot);
+    load();
 
     bool dry = false;   // the queue had nothing left for this warp
     uint32_t it = 0;
     for (; it < quad_budget; ++it) {
-        // ---- warp-aggregated refill of idle lanes ----
-        const unsigned idle = __ballot_sync(kFull, job < 0);
-        if (__builtin_expect(idle != 0, 0)) {
+        if (__builtin_expect(__any_sync(kFull, job < 0), 0)) {
             const bool need = job < 0 && !dry && slot < S.nslots;
-            const unsigned m = __ballot_sync(kFull, need);
-            if (m) {
-                const int leader = __ffs(m) - 1;
-                unsigned long long base = 0, got = 0;
-                if ((int)lane == leader) {
-                    // One fetch-and-add per warp.  A claim that runs past the
-                    // tail gets the part below it; the overshoot of head is
-                    // clamped back to the tail when more work is published
-                    // (fp32_publish_kernel, stream-ordered between launches).
-                    const unsigned long long tail = *(volatile unsigned long long*)q.tail;
-                    if (*(volatile unsigned long long*)q.head < tail) {
-                        const unsigned long long want = (unsigned long long)__popc(m);
-                        const unsigned long long old = atomicAdd(q.head, want);
-                        if (old < tail) {
-                            base = old;
-                            got = min(want, tail - old);
-                        }
-                    }
-                }
-                base = __shfl_sync(kFull, base, leader);
-                got = __shfl_sync(kFull, got, leader);
-                if (got < (unsigned long long)__popc(m)) dry = true;
-                if (need) {
-                    const unsigned rank = __popc(m & ((1u << lane) - 1u));
-                    if (rank < got) {
-                        const uint32_t traj = (uint32_t)f_resolve(q.range_end, q.range_job, q.range_first, q.nranges,
-                                                   (int64_t)(base + rank), &job);
-                        const JobF* Jn = &q.jobs[job];
-                        f_start<DBL, OVER>(Jn, S.ring, S.nslots, S.ring_slots, slot, traj, &sm, t, &xp, &rv,
-                                           &sm.cell[t], &sm.state[t], &sm.sw[t]);
-                        sm.job[t] = job;
-                        bind(traj, Jn->step0);
-                        if (Jn->nsteps == 0) {
-                            retire_lane<OVER>(*Jn, S.retired, sm, t, 0, xp, rv, 0);
-                            job = -1;
-                            sm.job[t] = -1;
-                            lo = -kInf;
-                            hi = kInf;
-                            F = 0.f;
-                            left = kLeftMax;
-                        }
-                    }
-                }
+            const bool asked = __any_sync(kFull, need);
+            if (asked) {
+                save();
+                if (refill<DBL, OVER>(&q, &S, &sm, t, slot, need)) dry = true;
+                load();
             }
             if (__all_sync(kFull, job < 0)) {
-                if (dry || m == 0) {
+                if (dry || !asked) {
                     *drained = true;
                     break;
                 }
                 continue;
             }
-            if (job < 0) continue;
         }
 
         // ---- one Philox block, four steps ----
-        const Words w = philox_wide((uint32_t)j, (uint32_t)(j >> 32), sm.gtraj[t], TAG_STEP, sm.key0[t], sm.key1[t]);
-        const float kn = sm.kn[t];
+        const uint2 fk = sm.fixk[t];
+        const Words w = philox_step(j, sm.fix[t], fk.x);
+        const float kn = __uint_as_float(fk.y);
         float nq[4];
         noise_pair(w.w0, w.w1, kn, &nq[0], &nq[1]);
         noise_pair(w.w2, w.w3, kn, &nq[2], &nq[3]);
+        // The four steps without a test between them: when the whole warp's
+        // positions stayed inside their bands and no countdown ends, they
+        // stand; else its lanes take them again one by one, the special ones
+        // as quick steps where they can.
+        const float x0 = xp, rv0 = rv;
+        float xs[4];
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
-            const float nz = nq[h];
-            if (OVER) {
-                xp = fmaf(F, c1, xp);
-                xp = xp + nz;
-                xp = xp + rv;
-                rv = nz;
-            } else {
-                rv = fmaf(F, c1, rv);
-                xp = fmaf(rv, c2, xp);
-                rv = fmaf(c3, rv, nz);
-                xp = fmaf(rv, c2, xp);
-            }
-            // left counts from the quad's start: the countdown ends at this
-            // sub-step when it equals h + 1 (one decrement per quad)
-            if (__builtin_expect(!(xp > lo && xp < hi) || left == h + 1, 0)) {
-                const uint64_t s = 4 * j + 1 + h;
-                int lrel = 0;
-                const int lt = light_step<DBL>(q.jobs, S, sm, t, slot, job, sm.traj[t], s, left == h + 1, xp, lo, hi, F,
-                                               lrel);
-                if (lt == 2) {
-                    left = lrel + (h + 1);
-                } else if (lt == 0) {
-                    sm.xp[t] = xp;
-                    sm.rv[t] = rv;
-                    sm.F[t] = F;
-                    sm.left[t] = left - (h + 1);
-                    sm.lo[t] = lo;
-                    sm.hi[t] = hi;
-                    general_step<DBL, OVER>(q.jobs, &S, &sm, t, slot, s);
-                    xp = sm.xp[t];
-                    F = sm.F[t];
-                    lo = sm.lo[t];
-                    hi = sm.hi[t];
-                    left = sm.left[t] + (h + 1);
-                    job = sm.job[t];
-                }
-            }
+            f_move<OVER>(xp, rv, F, c1, c2, c3, nq[h]);
+            xs[h] = xp;
             if (!OVER) rv = fmaf(F, c1, rv);
         }
+        float xmin, xmax;
+        range4(xs[0], xs[1], xs[2], xs[3], &xmin, &xmax);
         left -= 4;
+        const bool bad = !(xmin > lo) | !(xmax < hi) | (left <= 0);
+        if (__any_sync(kFull, bad)) {
+            int hs = 4;   // the step that needs special_step (4: none)
+            if (bad) {
+                xp = x0;
+                rv = rv0;
+                left += 4;
+                const uint64_t s0 = (uint64_t)sm.jh[t] << 34 | (uint64_t)j << 2;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    if (hs < 4) continue;
+                    f_move<OVER>(xp, rv, F, c1, c2, c3, nq[h]);
+                    --left;
+                    if (!(xp > lo) | !(xp < hi) | (left == 0)) {
+                        if (job < 0 || !quick_step<DBL>(q.jobs[job], sm, t, s0 + 1 + h, left == 0, xp, lo, hi, F,
+                                                        left, pw)) {
+                            hs = h;
+                            continue;
+                        }
+                    }
+                    if (!OVER) rv = fmaf(F, c1, rv);
+                }
+            }
+            if (__any_sync(kFull, hs < 4)) {
+                save();
+                if (hs < 4) slow_steps<DBL, OVER>(q.jobs, &S, &sm, t, slot, (uint64_t)sm.jh[t] << 32 | j, hs);
+                __syncwarp();
+                load();
+            }
+        }
         ++j;
     }
-
-    if (slot >= S.nslots) return it;
-    S.job[slot] = job;
-    if (job >= 0) {
-        const JobF& J = q.jobs[job];
-        const uint32_t traj = sm.traj[t];
-        S.traj[slot] = traj;
-        S.step[slot] = (int64_t)(4 * j + 1);
-        S.xp[slot] = xp;
-        S.rv[slot] = rv;
-        S.cell[slot] = sm.cell[t];
-        S.st[slot] = sm.state[t] | (sm.sw[t] << 1);
-        S.ckey[slot] = sm.ckey[t];
-        S.cflip[slot] = sm.cflip[t];
-        S.sc1[slot] = sm.sc1[t];
-        S.since[slot] = sm.since[t];
-        S.cgw[slot] = sm.cgw[t];
-        S.fidx[slot] = sm.fidx[t];
-        S.nxf[slot] = sm.nxf[t];
-        S.nflip[slot] = sm.nflip[t];
-        J.bits[traj] = (int32_t)sm.bits[t];
-        J.init_idx0[traj] = sm.init0[t];
-        J.idx2_0[traj] = sm.idx2[t];
-        J.tpt2_well[traj] = sm.tpt2w[t];
-        J.fpt_last[traj] = sm.fpt[t];
-        J.fpt2_last[traj] = sm.fpt2[t];
-        J.tpt_last[traj] = sm.tpt[t];
-        J.tpt2_last[traj] = sm.tpt2[t];
-    }
+    save();
+    save_slot<DBL>(&q, &S, &sm, t, slot);
     return it;
 }
 
 template <bool DBL, bool OVER>
 __global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_persistent_kernel(
     const __grid_constant__ QueueDev q, const __grid_constant__ SlotsDev S, uint32_t quad_budget) {
-    __shared__ RareSm sm;
+    extern __shared__ uint4 sm_raw[];
+    RareSm& sm = *reinterpret_cast<RareSm*>(sm_raw);
     bool drained = false;
     persistent_run<DBL, OVER>(q, S, sm, quad_budget, &drained);
 }
@@ -1068,7 +1431,8 @@ __global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_persistent_kern
 template <int kUnused>
 __global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_mixed_kernel(const __grid_constant__ MixedDev m,
                                                                                uint32_t quad_budget) {
-    __shared__ RareSm sm;
+    extern __shared__ uint4 sm_raw[];
+    RareSm& sm = *reinterpret_cast<RareSm*>(sm_raw);
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int type = m.wtype[w];
     uint32_t left = quad_budget;
@@ -1143,8 +1507,12 @@ template <bool DBL, bool OVER>
 static cudaError_t fp32_kernel_attrs() {
     // The kernel reads little global memory: give shared memory the whole
     // carveout so that the occupancy the grid is sized for is resident.
-    return cudaFuncSetAttribute(fp32_persistent_kernel<DBL, OVER>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                (int)cudaSharedmemCarveoutMaxShared);
+    const cudaError_t e = cudaFuncSetAttribute(fp32_persistent_kernel<DBL, OVER>,
+                                               cudaFuncAttributePreferredSharedMemoryCarveout,
+                                               (int)cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(fp32_persistent_kernel<DBL, OVER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(RareSm));
 }
 
 int fp32_blocks_per_sm(bool dbl, bool over, int block) {
@@ -1153,10 +1521,10 @@ int fp32_blocks_per_sm(bool dbl, bool over, int block) {
     if (dbl) e = over ? fp32_kernel_attrs<true, true>() : fp32_kernel_attrs<true, false>();
     else e = over ? fp32_kernel_attrs<false, true>() : fp32_kernel_attrs<false, false>();
     if (e != cudaSuccess) return 0;
-    if (dbl) e = over ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<true, true>, block, 0)
-                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<true, false>, block, 0);
-    else e = over ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<false, true>, block, 0)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<false, false>, block, 0);
+    if (dbl) e = over ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<true, true>, block, sizeof(RareSm))
+                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<true, false>, block, sizeof(RareSm));
+    else e = over ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<false, true>, block, sizeof(RareSm))
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<false, false>, block, sizeof(RareSm));
     return e == cudaSuccess ? n : 0;
 }
 
@@ -1164,14 +1532,16 @@ int fp32_mixed_blocks_per_sm(int block) {
     int n = 0;
     cudaError_t e = cudaFuncSetAttribute(fp32_mixed_kernel<0>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_mixed_kernel<0>, block, 0);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fp32_mixed_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RareSm));
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_mixed_kernel<0>, block, sizeof(RareSm));
     return e == cudaSuccess ? n : 0;
 }
 
 int launch_fp32_mixed(const MixedDev& m, uint32_t pair_budget, int grid, int block, void* stream) {
     const uint32_t quad_budget = pair_budget > 1 ? pair_budget / 2 : 1;
     if (block != 256 || (int64_t)grid * block > m.S.nslots) return (int)cudaErrorInvalidValue;
-    fp32_mixed_kernel<0><<<grid, block, 0, (cudaStream_t)stream>>>(m, quad_budget);
+    fp32_mixed_kernel<0><<<grid, block, sizeof(RareSm), (cudaStream_t)stream>>>(m, quad_budget);
     return (int)cudaGetLastError();
 }
 
@@ -1181,11 +1551,11 @@ int launch_fp32_persistent(bool dbl, bool over, const QueueDev& q, const SlotsDe
     const uint32_t quad_budget = pair_budget > 1 ? pair_budget / 2 : 1;   // blocks of four steps
     if (block > kMaxBlock) return (int)cudaErrorInvalidValue;
     if (dbl) {
-        if (over) fp32_persistent_kernel<true, true><<<grid, block, 0, st>>>(q, s, quad_budget);
-        else fp32_persistent_kernel<true, false><<<grid, block, 0, st>>>(q, s, quad_budget);
+        if (over) fp32_persistent_kernel<true, true><<<grid, block, sizeof(RareSm), st>>>(q, s, quad_budget);
+        else fp32_persistent_kernel<true, false><<<grid, block, sizeof(RareSm), st>>>(q, s, quad_budget);
     } else {
-        if (over) fp32_persistent_kernel<false, true><<<grid, block, 0, st>>>(q, s, quad_budget);
-        else fp32_persistent_kernel<false, false><<<grid, block, 0, st>>>(q, s, quad_budget);
+        if (over) fp32_persistent_kernel<false, true><<<grid, block, sizeof(RareSm), st>>>(q, s, quad_budget);
+        else fp32_persistent_kernel<false, false><<<grid, block, sizeof(RareSm), st>>>(q, s, quad_budget);
     }
     return (int)cudaGetLastError();
 }
