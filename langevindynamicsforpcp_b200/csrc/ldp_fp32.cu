@@ -29,11 +29,12 @@
 //
 // What bounds it: instruction issue.  4 jobs x 65536 trajectories x 120000
 // steps, frames every 100: 76.8 ms with a test and a branch at each step and
-// light steps (an out-of-line call's worth of state around them), 63.0 ms
-// with this loop; 161 instead of 194 warp instructions a block of four steps.
-// Nothing lives in a register across an out-of-line call (the lane state is in
-// shared memory there): with calls inside the loop it spilled at each block
-// (71.4 ms).
+// light steps (an out-of-line call's worth of state around them), 59.6 ms
+// with this loop.
+// The loop is a function without calls (run_blocks, no spills at 48 registers
+// and more), the lane state in shared memory between it and the out-of-line
+// parts: with the calls inside it the loop kept three of its values on the
+// stack (63.7 ms, 59.6 ms without), or spilled at each block (71.4 ms).
 
 // Rare state lives in shared memory (statistics clocks and flags, the cached
 // state of the cell left last, the state-1 step count), counts and duration
@@ -71,7 +72,8 @@ enum : int32_t { W_LB = 1, W_EVICT = 2, W_CVALID = 4, W_CSTATE = 8 };
 // right neighbour; the two barriers' states; the countdown ends at a frame
 // and nothing else; the pair's edge was crossed at least once.
 enum : uint32_t {
-    P_FAST = 1, P_PAIR = 2, P_SWAP = 4, P_RIGHT = 8, P_S0 = 16, P_S1 = 32, P_FRAME = 64, P_CROSSED = 128
+    P_FAST = 1, P_PAIR = 2, P_SWAP = 4, P_RIGHT = 8, P_S0 = 16, P_S1 = 32, P_FRAME = 64, P_CROSSED = 128,
+    P_HALT = 256
 };
 
 // Per-thread rare state, structure of arrays (conflict-free by thread).
@@ -1227,18 +1229,49 @@ __device__ __noinline__ void save_slot(const QueueDev* qp, const SlotsDev* Sp, R
     J.tpt2_last[traj] = sm.tpt2[t];
 }
 
-// Warp-aggregated refill of the warp's idle lanes (all lanes call): lanes
-// with `need` claim trajectories from the queue.  Returns whether the queue
-// had fewer than the lanes wanted.
+// How a launch that finds fewer items than it has lanes shares them out
+// (avail: items unclaimed at the last publication): as few warps to each
+// scheduler of the GPU as hold them, all schedulers alike.  Returns the lanes
+// a warp fills at its first claim, 0 for a warp that leaves the items to
+// others, 32 where every lane is wanted.  (24000 steps, frames every 20, warps
+// filled one after the other / this way: 16000 trajectories 5.6 / 3.0 ms,
+// 32000 5.8 / 3.4, 60000 5.7 / 4.3 overdamped; 1024 2.5 / 1.9.  One warp to a
+// scheduler while 32 lanes hold the items: two half as full cost 3.8 ms at
+// 16000.)  A warp's turn goes by its SM and by
+// its block's rank among the SM's blocks: a count of arrivals, which need not
+// start at zero (launches add one block per SM and rank); block indices do
+// not tell the SM (6 of 148 SMs hold two of blocks 0-147, 6 none).  All
+// threads of the block call.
+__device__ __forceinline__ int first_claim(unsigned long long avail, const SlotsDev& S) {
+    __shared__ unsigned rank;
+    const unsigned sms = (unsigned)S.sms, wpb = blockDim.x >> 5, schedulers = sms * 4;
+    if (avail == 0 || avail > (unsigned long long)gridDim.x * blockDim.x) return 32;
+    unsigned smid;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+    if (threadIdx.x == 0) rank = atomicAdd(&S.sm_rank[smid & (unsigned)(kSmRanks - 1)], 1u);
+    __syncthreads();
+    const unsigned n = (unsigned)avail, k = (n + schedulers * 32 - 1) / (schedulers * 32);
+    const unsigned cap = min(32u, (n + schedulers * k - 1) / (schedulers * k));
+    const unsigned used = (n + cap - 1) / cap;   // warps that take cap items (the last one fewer)
+    const unsigned layer = rank % (gridDim.x / sms) * wpb + (threadIdx.x >> 5);
+    return layer * sms + smid % sms < used ? (int)cap : 0;
+}
+
+// Warp-aggregated refill of the warp's idle lanes (all lanes call): the
+// first `most` lanes with `need` claim trajectories from the queue.  Returns
+// whether the warp is done claiming: the queue had fewer than the lanes
+// wanted, or lanes were left out.
 template <bool DBL, bool OVER>
 __device__ __noinline__ bool refill(const QueueDev* qp, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
-                                    bool need) {
+                                    bool need, int most) {
     const QueueDev& q = *qp;
     const SlotsDev& S = *Sp;
     RareSm& sm = *smp;
-    const unsigned m = __ballot_sync(kFull, need);
-    if (!m) return false;
     const unsigned lane = t & 31u;
+    const unsigned all = __ballot_sync(kFull, need);
+    need = need && __popc(all & ((1u << lane) - 1u)) < most;
+    const unsigned m = __ballot_sync(kFull, need);
+    if (!m) return all != 0;
     const int leader = __ffs(m) - 1;
     unsigned long long base = 0, got = 0;
     if ((int)lane == leader) {
@@ -1272,81 +1305,29 @@ __device__ __noinline__ bool refill(const QueueDev* qp, const SlotsDev* Sp, Rare
             idle_lane(sm, t);
         }
     }
-    return got < (unsigned long long)__popc(m);
+    return got < (unsigned long long)__popc(m) || m != all;
 }
 
-}  // namespace
-
-// The persistent loop of one model type for the calling warp: its slots'
-// trajectories (and new ones claimed from queue q) for up to quad_budget
-// blocks of four steps.  Returns the blocks run; *drained is set when it
-// stopped early because every lane of the warp was idle and the queue had
-// nothing left for it.  Slot state is loaded at entry and saved at exit.
-//
-// The hot lane state is in registers inside the loop and in sm across the
-// out-of-line calls, so that no register lives across one (the loop spilled
-// with them).
+// The hot loop: blocks of four steps of the warp's lanes, from their state
+// in sm and back, until a lane needs the slow path or `most` blocks ran.
+// Returns the blocks run, the last one unfinished for lanes with a step h
+// that needs the slow path (P_HALT + h in their P_* word).  A function
+// without calls, so that nothing in it is held for one.
 template <bool DBL, bool OVER>
-__device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const SlotsDev& S, RareSm& sm,
-                                                   uint32_t quad_budget, bool* drained) {
-    const int t = threadIdx.x;
-    const int64_t slot = (int64_t)blockIdx.x * blockDim.x + t;
-
-    int job, left;
-    uint32_t j;   // low word
-    float xp, rv, F, lo, hi;
+__device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t, uint32_t most) {
+    RareSm& sm = *smp;
+    const int job = sm.job[t];
+    float xp = sm.xp[t], rv = sm.rv[t], F = sm.F[t], lo = sm.lo[t], hi = sm.hi[t];
+    int left = sm.left[t];
+    uint32_t pw = sm.pw[t], j = sm.j[t];
     float c1 = 0.f, c2 = 0.f, c3 = 0.f;
-    uint32_t pw;
-    auto load = [&]() {
-        job = sm.job[t];
-        xp = sm.xp[t];
-        rv = sm.rv[t];
-        F = sm.F[t];
-        lo = sm.lo[t];
-        hi = sm.hi[t];
-        left = sm.left[t];
-        pw = sm.pw[t];
-        j = sm.j[t];
-        c1 = c2 = c3 = 0.f;
-        if (job >= 0) {
-            const JobF& J = q.jobs[job];
-            if (OVER) c1 = J.c_drift;
-            else { c1 = J.hdt_invM; c2 = J.hdt; c3 = J.expg; }
-        }
-    };
-    auto save = [&]() {
-        sm.xp[t] = xp;
-        sm.rv[t] = rv;
-        sm.F[t] = F;
-        sm.lo[t] = lo;
-        sm.hi[t] = hi;
-        sm.left[t] = left;
-        sm.pw[t] = pw;
-        sm.j[t] = j;
-    };
-    load_slot<DBL>(&q, &S, &sm, t, slot);
-    load();
-
-    bool dry = false;   // the queue had nothing left for this warp
+    if (job >= 0) {
+        const JobF& J = jobs[job];
+        if (OVER) c1 = J.c_drift;
+        else { c1 = J.hdt_invM; c2 = J.hdt; c3 = J.expg; }
+    }
     uint32_t it = 0;
-    for (; it < quad_budget; ++it) {
-        if (__builtin_expect(__any_sync(kFull, job < 0), 0)) {
-            const bool need = job < 0 && !dry && slot < S.nslots;
-            const bool asked = __any_sync(kFull, need);
-            if (asked) {
-                save();
-                if (refill<DBL, OVER>(&q, &S, &sm, t, slot, need)) dry = true;
-                load();
-            }
-            if (__all_sync(kFull, job < 0)) {
-                if (dry || !asked) {
-                    *drained = true;
-                    break;
-                }
-                continue;
-            }
-        }
-
+    do {
         // ---- one Philox block, four steps ----
         const uint2 fk = sm.fixk[t];
         const Words w = philox_step(j, sm.fix[t], fk.x);
@@ -1369,9 +1350,10 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
         float xmin, xmax;
         range4(xs[0], xs[1], xs[2], xs[3], &xmin, &xmax);
         left -= 4;
+        ++it;
         const bool bad = !(xmin > lo) | !(xmax < hi) | (left <= 0);
         if (__any_sync(kFull, bad)) {
-            int hs = 4;   // the step that needs special_step (4: none)
+            bool halt = false;
             if (bad) {
                 xp = x0;
                 rv = rv0;
@@ -1379,40 +1361,101 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
                 const uint64_t s0 = (uint64_t)sm.jh[t] << 34 | (uint64_t)j << 2;
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
-                    if (hs < 4) continue;
+                    if (halt) continue;
                     f_move<OVER>(xp, rv, F, c1, c2, c3, nq[h]);
                     --left;
                     if (!(xp > lo) | !(xp < hi) | (left == 0)) {
-                        if (job < 0 || !quick_step<DBL>(q.jobs[job], sm, t, s0 + 1 + h, left == 0, xp, lo, hi, F,
-                                                        left, pw)) {
-                            hs = h;
+                        if (job < 0 || !quick_step<DBL>(jobs[job], sm, t, s0 + 1 + h, left == 0, xp, lo, hi, F, left,
+                                                        pw)) {
+                            halt = true;
+                            pw |= P_HALT * (1 + h);
                             continue;
                         }
                     }
                     if (!OVER) rv = fmaf(F, c1, rv);
                 }
             }
-            if (__any_sync(kFull, hs < 4)) {
-                save();
-                if (hs < 4) slow_steps<DBL, OVER>(q.jobs, &S, &sm, t, slot, (uint64_t)sm.jh[t] << 32 | j, hs);
-                __syncwarp();
-                load();
-            }
+            if (__any_sync(kFull, halt)) break;
         }
         ++j;
+    } while (it < most);
+    sm.xp[t] = xp;
+    sm.rv[t] = rv;
+    sm.F[t] = F;
+    sm.lo[t] = lo;
+    sm.hi[t] = hi;
+    sm.left[t] = left;
+    sm.pw[t] = pw;
+    sm.j[t] = j;
+    return it;
+}
+
+}  // namespace
+
+// The persistent loop of one model type for the calling warp: its slots'
+// trajectories (and new ones claimed from queue q) for up to quad_budget
+// blocks of four steps.  Returns the blocks run; *drained is set when it
+// stopped early because every lane of the warp was idle and the queue had
+// nothing left for it.  Slot state is loaded at entry and saved at exit.
+template <bool DBL, bool OVER, bool kSpread>
+__device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const SlotsDev& S, RareSm& sm,
+                                                   uint32_t quad_budget, bool* drained) {
+    const int t = threadIdx.x;
+    const int64_t slot = (int64_t)blockIdx.x * blockDim.x + t;
+    load_slot<DBL>(&q, &S, &sm, t, slot);
+
+    bool dry = false;   // the queue had nothing left for this warp
+    int most = kSpread ? first_claim(*q.avail, S) : 32;
+    uint32_t it = 0;
+    while (it < quad_budget) {
+        // lanes become idle in the slow path only
+        if (__any_sync(kFull, sm.job[t] < 0)) {
+            const bool need = sm.job[t] < 0 && !dry && slot < S.nslots;
+            const bool asked = __any_sync(kFull, need);
+            if (asked) {
+                if (kSpread && most == 0) {
+                    // leave the items to the warps that take them now; items
+                    // still there after that (warps that were to take them
+                    // have trajectories already) are claimed
+                    if (*(volatile unsigned long long*)q.head < *(volatile unsigned long long*)q.tail)
+                        __nanosleep(20000);
+                    most = 32;
+                }
+                if (refill<DBL, OVER>(&q, &S, &sm, t, slot, need, most)) dry = true;
+                most = 32;
+            }
+            if (__all_sync(kFull, sm.job[t] < 0)) {
+                if (dry || !asked) {
+                    *drained = true;
+                    break;
+                }
+                ++it;
+                continue;
+            }
+        }
+        it += run_blocks<DBL, OVER>(q.jobs, &sm, t, quad_budget - it);
+        const uint32_t halt = sm.pw[t] / P_HALT;
+        if (__any_sync(kFull, halt != 0)) {
+            if (halt) {
+                sm.pw[t] &= P_HALT - 1;
+                slow_steps<DBL, OVER>(q.jobs, &S, &sm, t, slot, (uint64_t)sm.jh[t] << 32 | sm.j[t], (int)halt - 1);
+            }
+            __syncwarp();
+            sm.j[t] += 1;
+        }
     }
-    save();
     save_slot<DBL>(&q, &S, &sm, t, slot);
     return it;
 }
 
 template <bool DBL, bool OVER>
 __global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_persistent_kernel(
+
     const __grid_constant__ QueueDev q, const __grid_constant__ SlotsDev S, uint32_t quad_budget) {
     extern __shared__ uint4 sm_raw[];
     RareSm& sm = *reinterpret_cast<RareSm*>(sm_raw);
     bool drained = false;
-    persistent_run<DBL, OVER>(q, S, sm, quad_budget, &drained);
+    persistent_run<DBL, OVER, true>(q, S, sm, quad_budget, &drained);
 }
 
 // All four model types in one persistent launch (the serving loop's).  A
@@ -1470,10 +1513,10 @@ __global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_mixed_kernel(co
         bool drained = false;
         uint32_t used;
         switch (type) {
-            case 0: used = persistent_run<false, false>(m.q[0], m.S, sm, left, &drained); break;
-            case 1: used = persistent_run<false, true>(m.q[1], m.S, sm, left, &drained); break;
-            case 2: used = persistent_run<true, false>(m.q[2], m.S, sm, left, &drained); break;
-            default: used = persistent_run<true, true>(m.q[3], m.S, sm, left, &drained); break;
+            case 0: used = persistent_run<false, false, false>(m.q[0], m.S, sm, left, &drained); break;
+            case 1: used = persistent_run<false, true, false>(m.q[1], m.S, sm, left, &drained); break;
+            case 2: used = persistent_run<true, false, false>(m.q[2], m.S, sm, left, &drained); break;
+            default: used = persistent_run<true, true, false>(m.q[3], m.S, sm, left, &drained); break;
         }
         left -= (used < left) ? used : left;
         if (drained) {
@@ -1490,16 +1533,17 @@ __global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_mixed_kernel(co
 
 // Publishes item ranges [.., new_tail): clamps the head (claims may have run
 // past the old tail) and moves the tail; one thread, between launches.
-__global__ void fp32_publish_kernel(unsigned long long* head, unsigned long long* tail, int32_t* nranges,
-                                    unsigned long long new_tail, int32_t new_nranges) {
+__global__ void fp32_publish_kernel(unsigned long long* head, unsigned long long* tail, unsigned long long* avail,
+                                    int32_t* nranges, unsigned long long new_tail, int32_t new_nranges) {
     const unsigned long long t = *tail;
     if (*head > t) *head = t;
     *tail = new_tail;
+    *avail = new_tail - *head;
     *nranges = new_nranges;
 }
 
 int launch_fp32_publish(const QueueDev& q, unsigned long long new_tail, int32_t new_nranges, void* stream) {
-    fp32_publish_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(q.head, q.tail, q.nranges, new_tail, new_nranges);
+    fp32_publish_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(q.head, q.tail, q.avail, q.nranges, new_tail, new_nranges);
     return (int)cudaGetLastError();
 }
 

@@ -96,9 +96,12 @@ struct QueueDev {
     int64_t* range_first;   // [kFp32MaxRanges] first trajectory of the range
     unsigned long long* head;  // claimed items
     unsigned long long* tail;  // published items (written by the host)
+    unsigned long long* avail; // unclaimed items at the last publication
     int32_t* nranges;       // published ranges (written by the host)
     JobF* jobs;             // [kFp32MaxJobs]
 };
+
+constexpr int kSmRanks = 1024;
 
 // Per-slot state saved between launches, [nslots].
 struct SlotsDev {
@@ -117,6 +120,8 @@ struct SlotsDev {
     longlong2* ring;        // [R][nslots] cell table: {key, stamp << 1 | state}
     unsigned long long* retired;   // total retired trajectories (all jobs)
     int32_t ring_slots;
+    int32_t sms;            // SMs the grid's blocks are spread over
+    uint32_t* sm_rank;      // [kSmRanks] blocks started on an SM so far
 };
 
 // The four model types' queues and one set of slots shared by them, for the

@@ -67,10 +67,10 @@ static int64_t* stage(Fp32Queue& Q) {
 
 // One set of persistent slots (their state between launches): nslots
 // slots with R cell-table ring entries each, every slot empty.
-static int slots_init(int64_t nslots, int R, SlotsDev* Sp, void** mem) {
+static int slots_init(int64_t nslots, int R, int sms, SlotsDev* Sp, void** mem) {
     size_t sb = al256(sizeof(int32_t) * nslots) * 6 + al256(sizeof(int64_t) * nslots) * 7 +
                 al256(sizeof(float) * nslots) * 2 + al256(sizeof(longlong2) * (size_t)R * nslots) +
-                al256(sizeof(unsigned long long));
+                al256(sizeof(unsigned long long)) + al256(sizeof(uint32_t) * kSmRanks);
     cudaError_t e = cudaMalloc(mem, sb);
     if (e != cudaSuccess) return (int)e;
     e = cudaMemset(*mem, 0, sb);
@@ -80,6 +80,7 @@ static int slots_init(int64_t nslots, int R, SlotsDev* Sp, void** mem) {
     SlotsDev& S = *Sp;
     S.nslots = nslots;
     S.ring_slots = R;
+    S.sms = sms;
     S.job = (int32_t*)(a + o); o += al256(sizeof(int32_t) * nslots);
     S.cell = (int32_t*)(a + o); o += al256(sizeof(int32_t) * nslots);
     S.st = (int32_t*)(a + o); o += al256(sizeof(int32_t) * nslots);
@@ -96,7 +97,8 @@ static int slots_init(int64_t nslots, int R, SlotsDev* Sp, void** mem) {
     S.xp = (float*)(a + o); o += al256(sizeof(float) * nslots);
     S.rv = (float*)(a + o); o += al256(sizeof(float) * nslots);
     S.ring = (longlong2*)(a + o); o += al256(sizeof(longlong2) * (size_t)R * nslots);
-    S.retired = (unsigned long long*)(a + o);
+    S.retired = (unsigned long long*)(a + o); o += al256(sizeof(unsigned long long));
+    S.sm_rank = (uint32_t*)(a + o);
     // every slot starts empty
     std::vector<int32_t> neg((size_t)nslots, -1);
     e = cudaMemcpy(S.job, neg.data(), sizeof(int32_t) * nslots, cudaMemcpyHostToDevice);
@@ -117,7 +119,7 @@ static int queue_init(ldp_ctx* ctx, Fp32Queue& Q, int type, int ring_slots) {
     const int64_t nslots = (int64_t)Q.grid * Q.block;
     // queue + job table
     size_t qb = al256(sizeof(int64_t) * kFp32MaxRanges) * 2 + al256(sizeof(int32_t) * kFp32MaxRanges) +
-                al256(sizeof(unsigned long long) * 2) + al256(sizeof(int32_t)) + al256(sizeof(JobF) * kFp32MaxJobs) +
+                al256(sizeof(unsigned long long) * 3) + al256(sizeof(int32_t)) + al256(sizeof(JobF) * kFp32MaxJobs) +
                 al256(sizeof(unsigned long long) * kFp32MaxJobs);
     cudaError_t e = cudaMalloc(&Q.qmem, qb);
     if (e != cudaSuccess) return (int)e;
@@ -130,11 +132,12 @@ static int queue_init(ldp_ctx* ctx, Fp32Queue& Q, int type, int ring_slots) {
     Q.q.range_job = (int32_t*)(a + o); o += al256(sizeof(int32_t) * kFp32MaxRanges);
     Q.q.head = (unsigned long long*)(a + o);
     Q.q.tail = Q.q.head + 1;
-    o += al256(sizeof(unsigned long long) * 2);
+    Q.q.avail = Q.q.head + 2;
+    o += al256(sizeof(unsigned long long) * 3);
     Q.q.nranges = (int32_t*)(a + o); o += al256(sizeof(int32_t));
     Q.q.jobs = (JobF*)(a + o); o += al256(sizeof(JobF) * kFp32MaxJobs);
     Q.rem = (unsigned long long*)(a + o);
-    e = (cudaError_t)slots_init(nslots, ring_slots, &Q.s, &Q.smem);
+    e = (cudaError_t)slots_init(nslots, ring_slots, ctx->sm_count, &Q.s, &Q.smem);
     if (e != cudaSuccess) return (int)e;
     e = cudaMallocHost((void**)&Q.h_stage, 4096 * Fp32Queue::kStageSlots);
     if (e != cudaSuccess) return (int)e;
@@ -281,7 +284,7 @@ int fp32_launch_mixed(ldp_ctx* ctx, uint32_t pair_budget, cudaStream_t st) {
         bps = std::max(bps, 1);
         R.mixed_grid = ctx->sm_count * bps;
         const int64_t nslots = (int64_t)R.mixed_grid * block;
-        int e = slots_init(nslots, ring, &R.mixed, &R.mixed_mem);
+        int e = slots_init(nslots, ring, ctx->sm_count, &R.mixed, &R.mixed_mem);
         if (e) return e;
         const size_t n = (size_t)(nslots / 32) + kMixedSmTypes;   // wtype, then sm_type
         cudaError_t ce = cudaMalloc((void**)&R.wtype, sizeof(int32_t) * n);

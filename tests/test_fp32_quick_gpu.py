@@ -113,3 +113,23 @@ def _header_bytes(b):
     of [LDP_NCOUNT = 30][3] 64-bit counts."""
     at = b.index(struct.pack("<Q", 30 * 3 * 8), 12)
     return at - 12
+
+
+def test_every_job_size_is_claimed():
+    # How a launch shares out few items: fewer than schedulers, one more than
+    # a warp to each, partly filled ones, one more than all lanes; alone, and
+    # published while another job's trajectories hold part of the lanes.
+    p = params("single_over", 1050, freq_save=1)
+    keys = ("counts", "sums", "x_final", "state_final")
+    with ldp.Context(0) as c:
+        def job(n, job_id=3):
+            return ldp.Job(c, p, lanes=n, precision=ldp.PREC_FP32_BATCHED, job_id=job_id)
+        with job(113_665) as j:
+            whole = j.run().results(frames=False)
+        for n in (1, 593, 18_945, 40_001, 113_664):
+            with job(5_000, 4) as a, job(n) as b:
+                a.submit()
+                r = b.submit().wait().results(frames=False)
+                for k in keys:
+                    np.testing.assert_array_equal(r[k], whole[k][..., :n], err_msg=f"{n} {k}")
+                a.wait()
