@@ -259,17 +259,16 @@ ldp_status  ldp_ctx_mark(ldp_ctx *ctx, int mark);
 ldp_status  ldp_ctx_elapsed_ms(ldp_ctx *ctx, int mark_a, int mark_b, double *ms);
 ldp_status  ldp_ctx_synchronize(ldp_ctx *ctx);
 /* FP64 plain jobs in fixed-step mode with at most max_traj trajectories run
- * in latency mode: one CTA of two warps per trajectory, one warp drawing
- * the Gaussians and flip schedules of the next 32 steps while the other
- * integrates, for runs of few long trajectories (the reference's sample:
- * 16-32 trajectories x 3e9 steps), whose per-step dependency chain bounds
- * them.  Results are the same bit for bit either way.  0 disables it;
- * default 2048.  No reference counterpart. */
+ * in latency mode: some warps step the trajectories, as few to a warp as give
+ * every scheduler of the GPU one such warp, while others draw their noise (and
+ * flips, when they are frequent) ahead, for runs of few long trajectories (the
+ * reference's sample: 16-32 trajectories x 3e9 steps), whose per-step
+ * dependency chain bounds them.  Results are the same bit for bit either way.
+ * 0 disables it; default 2048.  No reference counterpart. */
 ldp_status  ldp_ctx_set_fp64_latency(ldp_ctx *ctx, int64_t max_traj);
 /* FP64 plain fixed-step jobs above the latency-mode limit and of at most
- * max_traj trajectories run in group mode: a CTA of 32 trajectories, a
- * consumer warp stepping them (lane l one trajectory) while producer warps
- * draw their Gaussians and flip schedules ahead, for runs of a few thousand
+ * max_traj trajectories run in group mode: as latency mode, with at least
+ * eight trajectories to a stepping warp, for runs of a few thousand
  * trajectories.  Results are the same bit for bit.  0 disables it;
  * default 16384.  No reference counterpart. */
 ldp_status  ldp_ctx_set_fp64_group(ldp_ctx *ctx, int64_t max_traj);

@@ -13,6 +13,8 @@
 // fma(), as in the reference's intrinsics (the only fused step is the
 // overdamped drift, _mmSIMD_fmadd_pd at S.h:2868).
 #include <cuda_runtime.h>
+#include <algorithm>
+#include <cmath>
 #include "ldp_device.cuh"
 #include "ldp_engine.h"
 
@@ -77,6 +79,22 @@ __device__ __forceinline__ void ring_store(const KConst& k, const TrajState& st,
     if (old != ck && old != INT64_MIN) st.counts[(int64_t)LDP_C_EVICT * st.n + i] += 1;
     st.ring_tag[o] = ck;
     st.ring_data[o] = (nflip << 1) | (int64_t)state;
+}
+
+// ring_store of the barrier left, then ring_load of the one entered, with all
+// their loads issued together: one memory latency instead of three in a row.
+template <bool DBL>
+__device__ __forceinline__ void ring_swap(const KConst& k, const TrajState& st, int64_t i, uint32_t g, int64_t left,
+                                          int state, int64_t nflip, int64_t ck, int* ps, int64_t* nb, bool* found) {
+    const int64_t mask = (int64_t)(k.slots - 1);
+    const int64_t o = (left & mask) * st.n + i, e = (ck & mask) * st.n + i;
+    const int64_t old = st.ring_tag[o], tag = st.ring_tag[e], d = st.ring_data[e];
+    if (old != left && old != INT64_MIN) st.counts[(int64_t)LDP_C_EVICT * st.n + i] += 1;
+    st.ring_tag[o] = left;
+    st.ring_data[o] = (nflip << 1) | (int64_t)state;
+    *found = tag == ck && o != e;   // o == e: the entry stored just now, of another barrier
+    *ps = *found ? (int)(d & 1) : default_state<DBL>(k, g, ck);
+    *nb = *found ? d >> 1 : 0;
 }
 
 // EnergyAndForce, S.h:1292-1324 / D.h:1464-1522.
@@ -166,10 +184,11 @@ __device__ __forceinline__ bool cg_hit(int64_t well, int size) { return ((int)we
 // Appends an event duration to list `list` of trajectory i (the reference's
 // push_back on its per-lane vectors, S.h:2391, 2447, 2504, 2524, 2580); c is
 // the list's count before the event.  A full list flags the trajectory.
-__device__ __noinline__ void ev_push(const KConst& k, const TrajState& st, int list, int64_t i, int64_t c, double d,
-                                     uint32_t* flags) {
-    if (c < k.ev_cap) st.ev[((int64_t)list * st.n + i) * k.ev_cap + c] = d;
-    else *flags |= LDP_FLAG_EVENT_OVERFLOW;
+__device__ __noinline__ uint32_t ev_push(const KConst& k, const TrajState& st, int list, int64_t i, int64_t c,
+                                         double d) {
+    if (c >= k.ev_cap) return LDP_FLAG_EVENT_OVERFLOW;
+    st.ev[((int64_t)list * st.n + i) * k.ev_cap + c] = d;
+    return 0u;
 }
 
 __device__ __forceinline__ void record(const KConst& k, const TrajState& st, const T64& t, int64_t i,
@@ -276,15 +295,16 @@ struct FlipDraw {
 // One step s of a trajectory (Integrate's loop body, S.h:1403-1511):
 // IntegrateStepEta / IntegrateStep (S.h:1654-1706, 2833-2886; D.h:1973-2024,
 // 3448-3505) followed by UpdateStatistics (S.h:2334-2592, D.h:2931-3209).
-// z is the step's Gaussian; src supplies the flip schedule of a flip at s.
-// Returns 0 to continue, 1 when the trajectory stops before completing s
-// (non-finite position), 2 when it stops after s (first passage reached).
+// src supplies the flip schedule of a flip at s.  Returns 0 to continue, 1
+// when the trajectory stops before completing s (non-finite position), 2 when
+// it stops after s (first passage reached).
+//
 // The position (and velocity) update of a step, IntegrateStepEta's first
-// part (S.h:1680-1695, 2860-2870).
+// part (S.h:1680-1695, 2860-2870).  rf: the step's noise, its Gaussian times
+// sig_r (overdamped) or sig_v.
 template <bool OVER>
-__device__ __forceinline__ void fp64_move(const KConst& k, T64& t, double z) {
+__device__ __forceinline__ void fp64_move(const KConst& k, T64& t, double rf) {
     if (OVER) {
-        const double rf = k.sig_r * z;
         t.x = fma(t.F, k.c_drift, t.x);
         t.x = t.x + rf;
         t.x = t.x + t.rprev;
@@ -292,21 +312,41 @@ __device__ __forceinline__ void fp64_move(const KConst& k, T64& t, double z) {
     } else {
         t.v = t.v + (k.invM * t.F) * k.hdt;
         t.x = t.x + t.v * k.hdt;
-        t.v = k.expg * t.v + k.sig_v * z;
+        t.v = k.expg * t.v + rf;
         t.x = t.x + t.v * k.hdt;
     }
 }
 
+// A barrier in state `state` whose flip at step `base` was missed, entered
+// at step s: its state then (S.h:2025-2068) and its new pending flip.
+__device__ __forceinline__ void catch_up(const KConst& k, uint32_t g, uint64_t s, int64_t base, int state,
+                                         const Words* wf, int* now, int64_t* nflip) {
+    const double lap = (double)((int64_t)s - base);
+    const double pl = k.c_lap[k.eq ? 0 : state] * -expm1_f64(k.a_lap * lap);
+    const uint64_t Tl = prob_to_u64(pl);
+    const Words wc = philox_at(s, g, TAG_CATCHUP, k.key0, k.key1);
+    const uint64_t U = ((uint64_t)wc.w0 << 32) | wc.w1;
+    *now = (U < Tl) ? (state ^ 1) : state;
+    *nflip = flip_schedule(s, wf->w2, wf->w3, k.ln1m[*now]);
+}
+
+// The barrier (cell, or in the double model local barrier) that a step left:
+// its state and pending flip, as stored in the cell table.
+struct LeftKey {
+    int64_t nflip;
+    int state;
+};
+
 // The rest of step s after fp64_move: indices, barrier flips and cell
-// entries, the state count, the force, the statistics and the frame.
-// cell_prev, well_prev, lb_prev: the indices before the move.
+// entries, the state count, the force and the statistics (the frame is the
+// caller's).  cell_prev, well_prev, lb_prev: the indices before the move; lk:
+// the barrier left, when one was.
 template <bool DBL, bool OVER, bool ETA, class Src>
 __device__ __forceinline__ int fp64_after_move(const KConst& k, const TrajState& st, int64_t i, uint32_t g, T64& t,
-                                               uint64_t s, const Src& src, int64_t& nflip, int64_t& sc0,
-                                               int64_t& sc1, uint32_t& flags, uint64_t& nxf, int64_t cell_prev,
-                                               int64_t well_prev, int lb_prev) {
+                                               uint64_t s, const Src& src, int64_t& nflip, int64_t& sc1,
+                                               uint32_t& flags, int64_t cell_prev, int64_t well_prev, int lb_prev,
+                                               LeftKey& lk) {
     const int64_t n = st.n;
-    const uint64_t fs = k.freq_save;
     if (!isfinite(t.x)) {
         flags |= LDP_FLAG_NONFINITE;
         t.bits |= B_DONE;
@@ -334,39 +374,33 @@ __device__ __forceinline__ int fp64_after_move(const KConst& k, const TrajState&
             nflip = src.schedule(k, g, s, t.state, &wf, &have_wf);
         }
         if (dKey) {
-            ring_store(k, st, i, cell_key<DBL>(cell_prev, lb_prev), t.state, nflip);
+            lk = LeftKey{nflip, t.state};
             int ps;
             int64_t nb;
             bool found;
-            ring_load<DBL>(k, st, i, g, cell_key<DBL>(t.cell, t.lb), &ps, &nb, &found);
+            ring_swap<DBL>(k, st, i, g, cell_key<DBL>(cell_prev, lb_prev), t.state, nflip,
+                           cell_key<DBL>(t.cell, t.lb), &ps, &nb, &found);
             if (found && nb > (int64_t)s) {
                 t.state = ps;
                 nflip = nb;
             } else {
-                const int64_t base = found ? nb : 0;
-                const int sb = found ? (ps ^ 1) : ps;
-                const double lap = (double)((int64_t)s - base);
-                const double pl = k.c_lap[k.eq ? 0 : sb] * -expm1_f64(k.a_lap * lap);
-                const uint64_t Tl = prob_to_u64(pl);
-                const Words wc = philox_at(s, g, TAG_CATCHUP, k.key0, k.key1);
-                const uint64_t U = ((uint64_t)wc.w0 << 32) | wc.w1;
-                t.state = (U < Tl) ? (sb ^ 1) : sb;
                 if (!have_wf) wf = philox_at(s, g, TAG_FLIP, k.key0, k.key1);
-                nflip = flip_schedule(s, wf.w2, wf.w3, k.ln1m[t.state]);
+                catch_up(k, g, s, found ? nb : 0, found ? (ps ^ 1) : ps, &wf, &t.state, &nflip);
             }
         }
     } else {
         // UpdateBarrierState (TAU == 0), S.h:1933-1997 / D.h:2299-2434.
         if (dKey) {
-            ring_store(k, st, i, cell_key<DBL>(cell_prev, lb_prev), t.state, nflip);
+            lk = LeftKey{nflip, t.state};
             int ps;
             int64_t nb;
             bool found;
-            ring_load<DBL>(k, st, i, g, cell_key<DBL>(t.cell, t.lb), &ps, &nb, &found);
+            ring_swap<DBL>(k, st, i, g, cell_key<DBL>(cell_prev, lb_prev), t.state, nflip,
+                           cell_key<DBL>(t.cell, t.lb), &ps, &nb, &found);
             t.state = ps;
         }
     }
-    if (t.state) ++sc1; else ++sc0;   // UpdateBarrierStateEtaParamter
+    sc1 += t.state;   // UpdateBarrierStateEtaParamter
     energy_force<DBL>(k, t);
     if (!OVER) t.v = t.v + (k.invM * t.F) * k.hdt;
 
@@ -399,7 +433,7 @@ __device__ __forceinline__ int fp64_after_move(const KConst& k, const TrajState&
                     const bool ib = ((double)t.cell == (double)t.init_idx0) ? ((t.bits & B_INIT0) != 0)
                                                                             : ((t.bits & B_INIT1) != 0);
                     if (k.ev_cap) {
-                        ev_push(k, st, LDP_E_FPT, i, c, now - t.fpt_last, &flags);
+                        flags |= ev_push(k, st, LDP_E_FPT, i, c, now - t.fpt_last);
                         if (c < k.ev_cap) st.ev_st[i * k.ev_cap + c] = (uint8_t)((t.state ? 1 : 0) | (ib ? 2 : 0));
                     }
                     st.counts[(int64_t)(ib ? LDP_C_INIT1 : LDP_C_INIT0) * n + i] += 1;
@@ -416,7 +450,7 @@ __device__ __forceinline__ int fp64_after_move(const KConst& k, const TrajState&
                 if (c == 0) st.sums[(int64_t)LDP_S_FIRST_FPT2 * n + i] = now - t.fpt2_last;
                 st.sums[(int64_t)LDP_S_FPT2 * n + i] += now - t.fpt2_last;
                 st.counts[(int64_t)LDP_C_FPT2 * n + i] = c + 1;
-                if (k.ev_cap) ev_push(k, st, LDP_E_FPT2, i, c, now - t.fpt2_last, &flags);
+                if (k.ev_cap) flags |= ev_push(k, st, LDP_E_FPT2, i, c, now - t.fpt2_last);
                 t.fpt2_last = now;
                 fpt2_set_idx(t);
                 if (k.fp_mode) t.bits |= B_DONE;   // first passage reached
@@ -430,7 +464,7 @@ __device__ __forceinline__ int fp64_after_move(const KConst& k, const TrajState&
                 if (c == 0) st.sums[(int64_t)LDP_S_FIRST_TPT * n + i] = now - t.tpt_last;
                 st.sums[(int64_t)LDP_S_TPT * n + i] += now - t.tpt_last;
                 st.counts[(int64_t)LDP_C_TPT * n + i] = c + 1;
-                if (k.ev_cap) ev_push(k, st, LDP_E_TPT, i, c, now - t.tpt_last, &flags);
+                if (k.ev_cap) flags |= ev_push(k, st, LDP_E_TPT, i, c, now - t.tpt_last);
             }
             if (dCell) {
                 if (t.bits & B_TPT2_UP) t.bits &= ~B_TPT2_UP;
@@ -439,7 +473,7 @@ __device__ __forceinline__ int fp64_after_move(const KConst& k, const TrajState&
                     if (c == 0) st.sums[(int64_t)LDP_S_FIRST_TPT2 * n + i] = now - t.tpt2_last;
                     st.sums[(int64_t)LDP_S_TPT2 * n + i] += now - t.tpt2_last;
                     st.counts[(int64_t)LDP_C_TPT2 * n + i] = c + 1;
-                    if (k.ev_cap) ev_push(k, st, LDP_E_TPT2, i, c, now - t.tpt2_last, &flags);
+                    if (k.ev_cap) flags |= ev_push(k, st, LDP_E_TPT2, i, c, now - t.tpt2_last);
                 }
                 t.tpt2_last = now;
                 t.tpt2_well = t.well;
@@ -457,7 +491,7 @@ __device__ __forceinline__ int fp64_after_move(const KConst& k, const TrajState&
                         st.sums[(int64_t)(LDP_S_CG0 + jj) * n + i] += now - st.cg_last[o];
                         const int64_t c = st.counts[(int64_t)(LDP_C_CG0 + jj) * n + i];
                         st.counts[(int64_t)(LDP_C_CG0 + jj) * n + i] = c + 1;
-                        if (k.ev_cap) ev_push(k, st, LDP_E_CG0 + jj, i, c, now - st.cg_last[o], &flags);
+                        if (k.ev_cap) flags |= ev_push(k, st, LDP_E_CG0 + jj, i, c, now - st.cg_last[o]);
                         st.cg_last[o] = now;
                         st.cg_well[o] = t.well;
                     }
@@ -465,23 +499,8 @@ __device__ __forceinline__ int fp64_after_move(const KConst& k, const TrajState&
             }
         }
     }
-    if (!k.fp_mode && s == nxf) {
-        record(k, st, t, i, (int64_t)(s / fs));
-        nxf += fs;
-    }
     if (t.bits & B_DONE) return 2;
     return 0;
-}
-
-template <bool DBL, bool OVER, bool ETA, class Src>
-__device__ __forceinline__ int fp64_step(const KConst& k, const TrajState& st, int64_t i, uint32_t g, T64& t,
-                                         uint64_t s, double z, const Src& src, int64_t& nflip, int64_t& sc0,
-                                         int64_t& sc1, uint32_t& flags, uint64_t& nxf) {
-    const int64_t cell_prev = t.cell, well_prev = t.well;
-    const int lb_prev = t.lb;
-    fp64_move<OVER>(k, t, z);
-    return fp64_after_move<DBL, OVER, ETA>(k, st, i, g, t, s, src, nflip, sc0, sc1, flags, nxf, cell_prev, well_prev,
-                                           lb_prev);
 }
 
 // The open interval of positions (absolute x) in which a step cannot change
@@ -533,574 +552,602 @@ __device__ __forceinline__ void band_forces(const KConst& k, const T64& t, doubl
     *f1 = a.F;
 }
 
-// Steps s_begin .. s_end-1 of the hot loop, one trajectory per thread, each
-// drawing its own Gaussians (one Philox block per four steps) and flips.
+// ---------------------------------------------------------------------------
+// Steps of a lane
+//
+// A lane steps one trajectory; all lanes of a launch are at the same step.
+// Steps are taken in blocks without a test between them (quiet_block): they
+// stand when the position stayed in the quiet band and, with rare flips, no
+// flip was pending in the block.  The lanes whose block does not stand take
+// its steps one by one (one_step): quiet; quick (the flank of the barrier
+// entered or left, or the edge between the cells of a pair crossed); or full
+// (fp64_after_move).  Same operations on the same values in every case, so
+// the results are those of full steps throughout, bit for bit.
+// ---------------------------------------------------------------------------
+enum : uint32_t {
+    Q_PAIR = 1,    // the lane's cell and a neighbour are a pair: see full_step
+    Q_RIGHT = 2,   // ... the right neighbour
+    Q_TAGGED = 4,  // the cell table has an entry of the lane's cell
+    Q_RUN = 8,     // the trajectory goes on
+    Q_FORCE = 16   // the quiet band has a force in some state
+};
+
+struct Lane {
+    T64 t;
+    double mid, bF0, bF1;   // quiet band: its middle, the force in it for either state
+    int half;               // ... high word of its half width (0: empty)
+    int pstate;             // the pair's other barrier: state ...
+    int64_t pnflip;         // ... and pending flip
+    int64_t nflip, sc1;
+    uint32_t q, flags;
+};
+
+// |x - mid| below the band's half width, by the high words: true only when it
+// is (NaN and infinity are not).
+__device__ __forceinline__ int off_band(const Lane& a, double x) {
+    return __double2hiint(x - a.mid) & 0x7fffffff;
+}
+
+template <bool DBL>
+__device__ __forceinline__ void set_band(const KConst& k, Lane& a, double mid, int half) {
+    a.mid = mid;
+    a.half = half;
+    band_forces<DBL>(k, a.t, &a.bF0, &a.bF1);
+    a.q = (a.q & ~Q_FORCE) | (a.bF0 != 0.0 || a.bF1 != 0.0 ? Q_FORCE : 0u);
+}
+
+template <bool DBL>
+__device__ __forceinline__ void open_band(const KConst& k, Lane& a) {
+    double lo, hi;
+    quiet_band<DBL>(k, a.t, &lo, &hi);
+    const double h = 0.5 * (hi - lo);
+    set_band<DBL>(k, a, 0.5 * (lo + hi), (h > 0.0) ? __double2hiint(h) : 0);
+}
+
+template <bool DBL, bool OVER>
+__device__ __forceinline__ void load_lane(const KConst& k, const TrajState& st, int64_t i, bool mine, Lane& a) {
+    a.q = 0;
+    a.flags = 0;
+    a.half = 0;
+    a.mid = a.bF0 = a.bF1 = 0.0;
+    a.pstate = 0;
+    a.pnflip = a.nflip = a.sc1 = 0;
+    a.t = T64{};
+    if (!mine) return;
+    load_traj(st, a.t, i);
+    if (a.t.bits & B_DONE) return;
+    a.q = Q_RUN;
+    a.sc1 = st.counts[(int64_t)LDP_C_STATE1 * st.n + i];
+    a.nflip = st.nflip[i];
+    energy_force<DBL>(k, a.t);   // not stored between launches
+}
+
+// s: the first step not integrated; before: the launch's first.
+__device__ __forceinline__ void store_lane(const KConst& k, const TrajState& st, int64_t i, const Lane& a, uint64_t s,
+                                           uint64_t before, uint64_t s_end) {
+    const int64_t n = st.n;
+    const int64_t sc1 = st.counts[(int64_t)LDP_C_STATE1 * n + i];
+    st.counts[(int64_t)LDP_C_STATE1 * n + i] = a.sc1;
+    st.counts[(int64_t)LDP_C_STATE0 * n + i] += (int64_t)(s - before) - (a.sc1 - sc1);
+    st.counts[(int64_t)LDP_C_STEPS * n + i] = (int64_t)s - 1;
+    uint32_t flags = a.flags;
+    if (k.fp_mode && !(a.t.bits & B_DONE) && s_end > k.step_cap) flags |= LDP_FLAG_CENSORED;
+    if (flags) st.counts[(int64_t)LDP_C_FLAGS * n + i] |= (int64_t)flags;
+    st.nflip[i] = a.nflip;
+    store_traj(st, a.t, i);
+}
+
+// A full step after its move.  When it crossed a cell edge and no statistic
+// is left waiting for a crossing, the cell left and the cell entered are a
+// pair: crossing their edge again, in this well, changes the barrier and
+// restarts the transition clocks, and nothing else, as long as the well stays
+// the same (the other barrier caught up when its pending flip has come).
+template <bool DBL, bool OVER, bool ETA, class Src>
+__device__ __forceinline__ int full_step(const KConst& k, const TrajState& st, int64_t i, uint32_t g, Lane& a,
+                                         uint64_t s, const Src& src) {
+    const int64_t cell = a.t.cell, well = a.t.well;
+    const int lb = a.t.lb;
+    LeftKey lk{};
+    const int r = fp64_after_move<DBL, OVER, ETA>(k, st, i, g, a.t, s, src, a.nflip, a.sc1, a.flags, cell, well, lb,
+                                                  lk);
+    a.q &= Q_RUN;
+    if (r) {
+        a.q = 0;
+        a.half = 0;
+        return r;
+    }
+    open_band<DBL>(k, a);
+    const int64_t d = cell - a.t.cell;
+    if ((d == 1 || d == -1) && a.t.well == well && (!DBL || a.t.lb != lb)) {
+        const bool fpt = !DBL && k.fpt && !k.fp_mode, fpt2 = k.fpt || k.fp_mode;
+        const bool ok = !(fpt && (a.t.bits & B_FPT_UP)) &&
+                        !(fpt2 && ((a.t.bits & B_FPT2_UP) || a.t.idx2_0 != well || a.t.idx2_1 != well + 1)) &&
+                        !(!DBL && k.wt && !k.fp_mode && (a.t.bits & B_WT_PASSED));
+        if (ok) {
+            a.q |= Q_PAIR | (d == 1 ? Q_RIGHT : 0u);
+            a.pstate = lk.state;
+            a.pnflip = lk.nflip;
+        }
+    }
+    return 0;
+}
+
+// A quick step after its move (not at the barrier's pending flip); false when
+// the step must be a full one.
+template <bool DBL, bool ETA>
+__device__ __forceinline__ bool quick_step(const KConst& k, const TrajState& st, int64_t i, uint32_t g, Lane& a,
+                                           uint64_t s) {
+    T64& t = a.t;
+    const bool right = t.well == t.cell;   // the half of the cell
+    const double hL = 0.5 * k.L, m = 1e-8 * (1.0 + fabs(t.x));   // beyond quiet_band's margins
+    const double xp = t.x - (double)t.cell * k.L;
+    if (!(fabs(xp) < k.L)) return false;   // not finite, or far
+    const bool leaves = right ? xp > hL : xp < -hL;
+    if (!leaves) {
+        // inside the cell: the same half and local barrier
+        if (!(right ? xp > m : xp < -m)) return false;
+        if (DBL && (t.lb ? !(xp > k.xc + m) : !(xp < k.xc - m))) return false;
+    } else {
+        if (!(a.q & Q_PAIR) || ((a.q & Q_RIGHT) != 0u) != right) return false;
+        t.cell += right ? 1 : -1;
+        if (DBL) t.lb ^= 1;
+    }
+    double lo, hi;
+    quiet_band<DBL>(k, t, &lo, &hi);
+    bool ok = t.x > lo && t.x < hi;
+    if (leaves) {
+        const double xn = t.x - (double)t.cell * k.L;
+        ok = ok && (right ? xn < -m : xn > m) && (!DBL || (t.lb ? xn > k.xc + m : xn < k.xc - m));
+        const int64_t left = t.cell - (right ? 1 : -1);
+        if (!ok) {
+            t.cell = left;
+            if (DBL) t.lb ^= 1;
+            return false;
+        }
+        const int64_t ck = cell_key<DBL>(left, t.lb ^ 1);
+        const int64_t o = (ck & (int64_t)(k.slots - 1)) * st.n + i;
+        if (a.q & Q_TAGGED) st.ring_data[o] = (a.nflip << 1) | (int64_t)t.state;
+        else ring_store(k, st, i, ck, t.state, a.nflip);
+        const int st0 = t.state;
+        const int64_t nf = a.nflip;
+        if (ETA && a.pnflip <= (int64_t)s) {
+            const Words wf = philox_at(s, g, TAG_FLIP, k.key0, k.key1);
+            catch_up(k, g, s, a.pnflip, a.pstate ^ 1, &wf, &t.state, &a.nflip);
+        } else {
+            t.state = a.pstate;
+            a.nflip = a.pnflip;
+        }
+        a.pstate = st0;
+        a.pnflip = nf;
+        a.q = (a.q ^ Q_RIGHT) | Q_TAGGED;
+        if (!DBL && k.tpt && !k.fp_mode) {
+            const double now = k.dt * (double)s;
+            t.bits &= ~(B_TPT_UP | B_TPT2_UP);
+            t.tpt_last = now;
+            t.tpt2_last = now;
+            t.tpt2_well = t.well;
+        }
+    }
+    if (!ok) return false;
+    set_band<DBL>(k, a, 0.5 * (lo + hi), __double2hiint(0.5 * (hi - lo)));
+    t.F = t.state ? a.bF1 : a.bF0;
+    a.sc1 += t.state;
+    return true;
+}
+
+// The rest of a lane's step s after its move, when it is not a quiet step
+// (off: the position is outside the band).
+template <bool DBL, bool OVER, bool ETA, class Src>
+__device__ __forceinline__ void special_step(const KConst& k, const TrajState& st, int64_t i, uint32_t g, Lane& a,
+                                             uint64_t s, bool off, const Src& src) {
+    const bool flip = ETA && (int64_t)s == a.nflip;
+    if (!off) {
+        // the current barrier's flip and nothing else
+        a.t.state ^= 1;
+        Words wf;
+        bool have = false;
+        a.nflip = src.schedule(k, g, s, a.t.state, &wf, &have);
+        a.t.F = a.t.state ? a.bF1 : a.bF0;
+        a.sc1 += a.t.state;
+    } else if (flip || !quick_step<DBL, ETA>(k, st, i, g, a, s)) {
+        full_step<DBL, OVER, ETA>(k, st, i, g, a, s, src);
+        return;   // the velocity's second half-kick included
+    }
+    if (!OVER) a.t.v = a.t.v + (k.invM * a.t.F) * k.hdt;
+}
+
+// A saved frame (after its step, a multiple of FREQSAVE); the energy and the
+// barrier height are those of the position, whatever kind of step led there.
+template <bool DBL>
+__device__ __forceinline__ void save_frame(const KConst& k, const TrajState& st, int64_t i, Lane& a, int64_t frame) {
+    if (k.write_x) energy_force<DBL>(k, a.t);
+    record(k, st, a.t, i, frame);
+}
+
+// N steps from the band, rf[m] their noise; true and the lane (one that wants
+// to) moved on when they stand.  FLAT: no lane of the warp has a force (fma(0, c, x) is x).
+template <bool OVER, bool FLAT, int N>
+__device__ __forceinline__ bool quiet_moves(const KConst& k, Lane& a, bool want, const double* rf) {
+    double x = a.t.x;
+    int far = 0;
+    if (OVER) {
+        double r = a.t.rprev;
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            if (!FLAT) x = fma(a.t.F, k.c_drift, x);
+            x = x + rf[m];
+            x = x + r;
+            r = rf[m];
+            far = max(far, off_band(a, x));
+        }
+        want = want && far < a.half;
+        if (want) {
+            a.t.x = x;
+            a.t.rprev = r;
+        }
+    } else {
+        const double kick = (k.invM * a.t.F) * k.hdt;
+        double v = a.t.v;
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            v = v + kick;
+            x = x + v * k.hdt;
+            v = k.expg * v + rf[m];
+            x = x + v * k.hdt;
+            v = v + kick;
+            far = max(far, off_band(a, x));
+        }
+        want = want && far < a.half;
+        if (want) {
+            a.t.x = x;
+            a.t.v = v;
+        }
+    }
+    if (want) a.sc1 += N * a.t.state;
+    return want;
+}
+
+// Steps s_begin .. s_end-1, one trajectory per thread, each drawing its own
+// noise: one Philox block and two Box-Muller pairs for four steps.
 template <bool DBL, bool OVER, bool ETA>
 __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, const TrajState st, int64_t g0,
                                                          uint64_t s_begin, uint64_t s_end) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= st.n) return;
     const uint32_t g = (uint32_t)(g0 + i);
-    T64 t;
-    load_traj(st, t, i);
-    if (t.bits & B_DONE) return;
-    const int64_t n = st.n;
-    int64_t sc0 = st.counts[(int64_t)LDP_C_STATE0 * n + i];
-    int64_t sc1 = st.counts[(int64_t)LDP_C_STATE1 * n + i];
-    // Force at the current position (not stored between launches).
-    energy_force<DBL>(k, t);
-    int64_t nflip = st.nflip[i];
-    uint32_t flags = 0;
-    uint64_t s = s_begin;
+    Lane a;
+    load_lane<DBL, OVER>(k, st, i, i < st.n, a);
+    const bool active = (a.q & Q_RUN) != 0u;
     const uint64_t fs = k.freq_save;
-    // Next frame step (a multiple of FREQSAVE), so that no step divides.
-    uint64_t nxf = (s_begin + fs - 1) / fs * fs;
-    // One Philox block serves steps 4a+1 .. 4a+4: words 0,1 the first
-    // Gaussian pair, words 2,3 (kept) the second.
-    double za = 0, zb = 0;
-    uint32_t wc2 = 0, wc3 = 0;
+    uint64_t s = s_begin, s_done = s_end;   // s_done: this lane's first step not integrated
+    // next frame step (a multiple of FREQSAVE), so that no step divides
+    int64_t frame = (int64_t)((s_begin + fs - 1) / fs);
+    uint64_t nxf = k.fp_mode ? ~0ull : (uint64_t)frame * fs;
+    const double sig = OVER ? k.sig_r : k.sig_v;
     const FlipDraw src;
-    // quiet band (empty: the first step takes the full path) and the force
-    // in it for either barrier state
-    double blo = 1.0, bhi = 0.0, bF0 = 0.0, bF1 = 0.0;
-    for (; s < s_end; ++s) {
-        const int q = (int)((s - 1) & 3);
-        if (q == 0 || s == s_begin) {
-            const Words w = philox_at((s - 1) >> 2, g, TAG_STEP, k.key0, k.key1);
-            wc2 = w.w2;
-            wc3 = w.w3;
-            if (q < 2) gauss_pair_f64(w.w0, w.w1, &za, &zb);
-            else gauss_pair_f64(w.w2, w.w3, &za, &zb);
-        } else if (q == 2) {
-            gauss_pair_f64(wc2, wc3, &za, &zb);
-        }
-        const double z = (q & 1) ? zb : za;
-        const int64_t cell_prev = t.cell, well_prev = t.well;
-        const int lb_prev = t.lb;
-        fp64_move<OVER>(k, t, z);
-        if (t.x > blo && t.x < bhi && (int64_t)s != (int64_t)nxf) {
-            // a quiet step (see quiet_band): same indices, no frame, no
-            // event; a flip draws its schedule and takes the band's force
-            if (ETA && (int64_t)s == nflip) {
-                t.state ^= 1;
-                Words wf;
-                bool have = false;
-                nflip = src.schedule(k, g, s, t.state, &wf, &have);
-                t.F = t.state ? bF1 : bF0;
+    while (s < s_end && __any_sync(0xffffffffu, (a.q & Q_RUN) != 0u)) {
+        const Words w = philox_at((s - 1) >> 2, g, TAG_STEP, k.key0, k.key1);
+        double rf[4];
+        gauss_pair_f64(w.w0, w.w1, &rf[0], &rf[1]);
+        gauss_pair_f64(w.w2, w.w3, &rf[2], &rf[3]);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) rf[m] = sig * rf[m];
+        const int m0 = (int)((s - 1) & 3), m1 = s_end - s < (uint64_t)(4 - m0) ? m0 + (int)(s_end - s) : 4;
+        bool stands = false;
+        if (m0 == 0 && m1 == 4 && nxf >= s + 3)
+            stands = quiet_moves<OVER, false, 4>(k, a, !ETA || a.nflip >= (int64_t)s + 4, rf);
+        if (__any_sync(0xffffffffu, !stands)) {
+#pragma unroll 1
+            for (int m = m0; m < m1; ++m) {
+                const uint64_t sm = s + (uint64_t)(m - m0);
+                const double z = m == 0 ? rf[0] : m == 1 ? rf[1] : m == 2 ? rf[2] : rf[3];
+                if (!stands && (a.q & Q_RUN)) {
+                    fp64_move<OVER>(k, a.t, z);
+                    const bool off = !(off_band(a, a.t.x) < a.half);
+                    if (off || (ETA && (int64_t)sm == a.nflip)) {
+                        special_step<DBL, OVER, ETA>(k, st, i, g, a, sm, off, src);
+                        if (!(a.q & Q_RUN)) s_done = sm + ((a.flags & LDP_FLAG_NONFINITE) ? 0 : 1);
+                    } else {
+                        a.sc1 += a.t.state;
+                        if (!OVER) a.t.v = a.t.v + (k.invM * a.t.F) * k.hdt;
+                    }
+                }
+                __syncwarp();
+                if (nxf == sm && m + 1 < m1) {
+                    // (a frame after the block's last step is saved below)
+                    if (a.q & Q_RUN) save_frame<DBL>(k, st, i, a, frame);
+                    nxf += fs;
+                    ++frame;
+                }
             }
-            if (t.state) ++sc1; else ++sc0;
-            if (!OVER) t.v = t.v + (k.invM * t.F) * k.hdt;
-            continue;
         }
-        const int r = fp64_after_move<DBL, OVER, ETA>(k, st, i, g, t, s, src, nflip, sc0, sc1, flags, nxf, cell_prev,
-                                                      well_prev, lb_prev);
-        if (r == 1) break;
-        if (r == 2) { ++s; break; }
-        quiet_band<DBL>(k, t, &blo, &bhi);
-        band_forces<DBL>(k, t, &bF0, &bF1);
+        s += (uint64_t)(m1 - m0);
+        if (nxf == s - 1) {
+            if (a.q & Q_RUN) save_frame<DBL>(k, st, i, a, frame);
+            nxf += fs;
+            ++frame;
+        }
     }
-    // s is the first step not integrated.
-    st.counts[(int64_t)LDP_C_STATE0 * n + i] = sc0;
-    st.counts[(int64_t)LDP_C_STATE1 * n + i] = sc1;
-    st.counts[(int64_t)LDP_C_STEPS * n + i] = (int64_t)s - 1;
-    if (k.fp_mode && !(t.bits & B_DONE) && s_end > k.step_cap) flags |= LDP_FLAG_CENSORED;
-    if (flags) st.counts[(int64_t)LDP_C_FLAGS * n + i] |= (int64_t)flags;
-    st.nflip[i] = nflip;
-    store_traj(st, t, i);
+    if (active) store_lane(k, st, i, a, s_done, s_begin, s_end);
 }
 
 // ---------------------------------------------------------------------------
-// Latency mode: few long trajectories (the reference's own sample runs 16-32
-// trajectories for 3e9 steps).  One trajectory per thread leaves a step's
-// whole dependency chain -- Philox rounds, the FP64 logarithm and sincos of
-// Box-Muller, the flip's logarithm and division -- on one thread, ~1800
-// cycles per step.  Here a trajectory gets a CTA of two warps:
-//  * the producer warp computes, for a block of 32 steps, lane l the inputs
-//    of step s0 + l that do not depend on the position: its Gaussian (the
-//    same Philox block and Box-Muller pair the thread-per-trajectory kernel
-//    uses) and, when barriers flip, the flip schedule a flip at that step
-//    would give for either new state (its TAG_FLIP words, one logarithm,
-//    the two geometric waiting times);
-//  * lane 0 of the consumer warp runs the steps with fp64_step, taking those
-//    inputs from shared memory, so its chain is the position update,
-//    indices, flip selection and force.
-// Two buffers of 32 steps alternate; named barriers 1-2 ("full") and 3-4
-// ("empty") hand them over, every arrival matched by one wait (the producer
-// waits for the last two buffers' release before it exits).  Every input is
-// the same FP64 value, so results equal the thread-per-trajectory kernel's
-// (and the oracle's) bit for bit.
+// Group mode
+//
+// What bounds a run of few trajectories is the chain of a step, not the GPU:
+// a Gaussian alone (Philox rounds, the FP64 logarithm and sincos, a square
+// root) takes ~1000 cycles in one thread.  So the noise is drawn ahead by
+// other warps: a CTA has nc consumer warps, T lanes of each stepping a
+// trajectory, and producer warps that draw the noise of the CTA's M = nc T
+// trajectories, B steps a buffer, one Philox block and two Box-Muller pairs
+// for four steps of a trajectory.  A consumer's chain of a quiet step is then
+// two additions (three operations where there is a force).  Two buffers
+// alternate; named barriers 1-2 ("full") and 3-4 ("empty") over all the CTA's
+// warps hand them over, every arrival matched by one wait, with no spin loop.
+//
+// T is chosen so that every scheduler of the GPU has one consumer warp
+// (launch_fp64_group): a warp waits for each of its lanes' special steps, so
+// fewer lanes a warp step faster, and warps beyond one a scheduler slow each
+// other and the producers down.
+//
+// Within a buffer each lane is at its own step: after a special step it goes
+// on with a new block of kGrpSteps steps, so a special step costs its warp
+// itself and the steps walked up to it (1000-1800 cycles in all), not the
+// block's remaining steps one by one as well (5000).
+//
+// DENSE: barriers flip so often that a lane could not draw its flips as they
+// come.  Producers then also draw the wait of a flip at every step for both
+// states (its TAG_FLIP words, one logarithm), in 16 bits: -ln(2^-64) /
+// -ln(1 - p) < 2^16 for p >= 1/1024.  A flip drawn by the consumer costs its
+// warp ~1000 cycles, the waits of all steps ~25 cycles a step and a longer
+// chain in the block: dense from p T = 1/40 on.
+//
+// What it measured (ns a step; one CTA a trajectory, or of 32 trajectories,
+// with a producer warp or four, flips drawn for every step / this): the
+// sample input, 32 trajectories, p = 1/2: 62.3 / 40.8; rare flips, 592: 91 /
+// 45, 2000: 312 / 68, 5003 underdamped: 235 / 60, 16000: 503 / 202.
 // ---------------------------------------------------------------------------
-constexpr int kLatBlock = 32;   // steps per buffer
+constexpr int kGrpConsumers = 4;   // consumer warps of a CTA at most: one to a scheduler
+constexpr int kGrpProducers = 8;   // producer warps (4: 16000 trajectories 263 ns a step, 12: 197)
+constexpr int kGrpSteps = 8;       // steps of a consumer's block (16: 5 % slower at 2 lanes a warp, 10 % faster at 1)
+constexpr int kGrpItems = 8;       // items (four steps of a trajectory) of a producer lane in a buffer (4: 219 ns)
+constexpr int kGrpBuffer = 256;    // steps of a buffer at most
+__device__ __forceinline__ void bar_sync(int id, int n) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
 
-constexpr int kLatSub = 8;       // steps per speculative sub-block (see the consumer)
-struct LatBuf {
-    double z[2][kLatBlock];
-    int64_t cand[2][2][kLatBlock];   // [buffer][new state][step]
-};
-
-// The flip schedule of a flip at step s for both new states, from the words
-// (hi, lo) of TAG_FLIP at s: flip_schedule of either state, with the
-// logarithm evaluated once.
-__device__ __forceinline__ void flip_schedule_both(uint64_t s, uint32_t hi, uint32_t lo, const double ln1m[2],
-                                                   int64_t* c0, int64_t* c1) {
+// Waits of a flip at step s into state 0 (low half) and 1: flip_wait for
+// either state, the logarithm evaluated once.
+__device__ __forceinline__ uint32_t dense_waits(const KConst& k, uint32_t hi, uint32_t lo) {
     const double u = ((double)(((uint64_t)hi << 32) | lo) + 1.0) * 0x1p-64;
     const double lu = log_f64(u);
-    int64_t c[2];
-#pragma unroll
-    for (int st = 0; st < 2; ++st) {
-        uint64_t wt = 0xffffffffffffffffull;
-        if (ln1m[st] < 0.0) {
-            const double q = lu / ln1m[st];
-            if (q < 0x1p62) wt = 1ull + (uint64_t)floor(q);
-        }
-        c[st] = (wt >= (uint64_t)kNeverFlip - s) ? kNeverFlip : (int64_t)(s + wt);
-    }
-    *c0 = c[0];
-    *c1 = c[1];
+    const uint32_t w0 = 1u + (uint32_t)floor(lu / k.ln1m[0]);
+    const uint32_t w1 = k.ln1m[1] == k.ln1m[0] ? w0 : 1u + (uint32_t)floor(lu / k.ln1m[1]);
+    return w0 | (w1 << 16);
 }
 
-// The consumer's flip schedule source: the producer's candidates for step s.
+// The consumer's flip schedule source with DENSE: the producer's waits.
 struct FlipFromBuffer {
-    const int64_t* c0;
-    const int64_t* c1;
-    __device__ __forceinline__ int64_t schedule(const KConst&, uint32_t, uint64_t, int state, Words*, bool*) const {
-        return state ? *c1 : *c0;
+    uint32_t w;
+    __device__ __forceinline__ int64_t schedule(const KConst&, uint32_t, uint64_t s, int state, Words*, bool*) const {
+        return (int64_t)s + (state ? (w >> 16) : (w & 0xffffu));
     }
 };
 
-__device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
-__device__ __forceinline__ void named_arrive(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
-
-template <bool DBL, bool OVER, bool ETA>
-__global__ void __launch_bounds__(64, 4) fp64_latency_kernel(const KConst k, const TrajState st, int64_t g0,
-                                                          uint64_t s_begin, uint64_t s_end) {
-    __shared__ LatBuf buf;
-    const int64_t i = blockIdx.x;
-    if (i >= st.n) return;   // whole CTA: no barrier is reached
-    const uint32_t g = (uint32_t)(g0 + i);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint64_t nblk = (s_end > s_begin) ? (s_end - s_begin + kLatBlock - 1) / kLatBlock : 0;
-    if (warp == 1) {
-        // ---- producer ----
-        for (uint64_t b = 0; b < nblk; ++b) {
-            const int u = (int)(b & 1);
-            if (b >= 2) named_sync(3 + u);   // buffer u released by the consumer
-            const uint64_t s = s_begin + b * kLatBlock + (uint64_t)lane;
-            if (s < s_end) {
-                const int q = (int)((s - 1) & 3);
-                const Words w = philox_at((s - 1) >> 2, g, TAG_STEP, k.key0, k.key1);
-                double za, zb;
-                if (q < 2) gauss_pair_f64(w.w0, w.w1, &za, &zb);
-                else gauss_pair_f64(w.w2, w.w3, &za, &zb);
-                buf.z[u][lane] = (q & 1) ? zb : za;
-                if (ETA) {
-                    const Words wf = philox_at(s, g, TAG_FLIP, k.key0, k.key1);
-                    flip_schedule_both(s, wf.w0, wf.w1, k.ln1m, &buf.cand[u][0][lane], &buf.cand[u][1][lane]);
-                }
-            }
-            __syncwarp();
-            named_arrive(1 + u);             // buffer u full
-        }
-        // the consumer's release of the last two buffers
-        for (uint64_t b = (nblk > 2 ? nblk - 2 : 0); b < nblk; ++b) named_sync(3 + (int)(b & 1));
-        return;
-    }
-    // ---- consumer ----
-    T64 t;
-    int64_t sc0 = 0, sc1 = 0, nflip = 0;
-    uint32_t flags = 0;
-    uint64_t s = s_begin, nxf = 0;
-    bool run = false, active = false;
-    // quiet band (empty: the first step takes the full path) and the force
-    // in it for either barrier state
-    double blo = 1.0, bhi = 0.0, bF0 = 0.0, bF1 = 0.0;
-    if (lane == 0) {
-        load_traj(st, t, i);
-        active = run = !(t.bits & B_DONE);
-        sc0 = st.counts[(int64_t)LDP_C_STATE0 * st.n + i];
-        sc1 = st.counts[(int64_t)LDP_C_STATE1 * st.n + i];
-        energy_force<DBL>(k, t);
-        nflip = st.nflip[i];
-        const uint64_t fs = k.freq_save;
-        nxf = (s_begin + fs - 1) / fs * fs;
-    }
-    for (uint64_t b = 0; b < nblk; ++b) {
-        const int u = (int)(b & 1);
-        named_sync(1 + u);                   // buffer u full
-        if (lane == 0 && run) {
-            const uint64_t s1 = (s_begin + (b + 1) * kLatBlock < s_end) ? s_begin + (b + 1) * kLatBlock : s_end;
-            const int nl = (int)(s1 - s);
-            // the next step's Gaussian and flip schedules are loaded one step
-            // ahead, so their shared-memory latency is off the chain (zn,
-            // cn0, cn1 hold step pf's)
-            double zn = buf.z[u][0];
-            int64_t cn0 = 0, cn1 = 0;
-            if (ETA) {
-                cn0 = buf.cand[u][0][0];
-                cn1 = buf.cand[u][1][0];
-            }
-            int pf = 0;
-            for (int l = 0; l < nl;) {
-                // Speculative sub-block: the next kLatSub steps run as quiet
-                // steps without the per-step band test, keeping the lowest
-                // and highest position; when every position stayed inside
-                // the quiet band (and no frame falls in the sub-block) they
-                // were quiet steps and stand, else the state at the
-                // sub-block's start is restored and the steps run one by one.
-                // x turning NaN stays NaN to the end, which the final test
-                // catches.
-                if (l + kLatSub <= nl && (l & (kLatSub - 1)) == 0 && (int64_t)nxf >= (int64_t)s + kLatSub &&
-                    t.x > blo && t.x < bhi) {
-                    double zb[kLatSub];
-                    int64_t c0b[kLatSub], c1b[kLatSub];
+// quiet_moves with flips taken from the producer's waits w[m]; l the first
+// step's place in the buffer, flip that of the pending flip.
+template <bool OVER, int N>
+__device__ __forceinline__ bool dense_block(const KConst& k, Lane& a, bool want, int& flip, int l, const double* rf,
+                                            const uint32_t* w) {
+    double x = a.t.x, r = a.t.rprev, v = a.t.v, F = a.t.F;
+    int nf = flip - l, state = a.t.state, n1 = 0, far = 0;
 #pragma unroll
-                    for (int m = 0; m < kLatSub; ++m) {
-                        zb[m] = buf.z[u][l + m];
-                        if (ETA) {
-                            c0b[m] = buf.cand[u][0][l + m];
-                            c1b[m] = buf.cand[u][1][l + m];
-                        }
-                    }
-                    const double x0 = t.x, v0 = t.v, F0 = t.F, r0 = t.rprev;
-                    const int st0 = t.state;
-                    const int64_t nflip0 = nflip;
-                    int n1 = 0;
-                    double xmin = t.x, xmax = t.x;
-#pragma unroll
-                    for (int m = 0; m < kLatSub; ++m) {
-                        fp64_move<OVER>(k, t, zb[m]);
-                        xmin = fmin(xmin, t.x);
-                        xmax = fmax(xmax, t.x);
-                        if (ETA) {
-                            // flips by selects (t.F is the band's force of
-                            // the state throughout), so the steps form one
-                            // chain in x
-                            const bool f = (int64_t)s + m == nflip;
-                            t.state ^= (int)f;
-                            const int64_t cn = t.state ? c1b[m] : c0b[m];
-                            nflip = f ? cn : nflip;
-                            t.F = t.state ? bF1 : bF0;
-                        }
-                        n1 += t.state;
-                        if (!OVER) t.v = t.v + (k.invM * t.F) * k.hdt;
-                    }
-                    if (xmin > blo && xmax < bhi && t.x > blo) {
-                        sc1 += n1;
-                        sc0 += kLatSub - n1;
-                        s += kLatSub;
-                        l += kLatSub;
-                        continue;
-                    }
-                    t.x = x0;
-                    t.v = v0;
-                    t.F = F0;
-                    t.rprev = r0;
-                    t.state = st0;
-                    nflip = nflip0;
-                }
-                double z;
-                int64_t ca0 = 0, ca1 = 0;
-                if (pf == l) {
-                    z = zn;
-                    ca0 = cn0;
-                    ca1 = cn1;
-                } else {
-                    z = buf.z[u][l];
-                    if (ETA) {
-                        ca0 = buf.cand[u][0][l];
-                        ca1 = buf.cand[u][1][l];
-                    }
-                }
-                if (l + 1 < nl) {
-                    zn = buf.z[u][l + 1];
-                    if (ETA) {
-                        cn0 = buf.cand[u][0][l + 1];
-                        cn1 = buf.cand[u][1][l + 1];
-                    }
-                    pf = l + 1;
-                }
-                const int64_t cell_prev = t.cell, well_prev = t.well;
-                const int lb_prev = t.lb;
-                fp64_move<OVER>(k, t, z);
-                if (t.x > blo && t.x < bhi && (int64_t)s != (int64_t)nxf) {
-                    // a quiet step: same indices, no frame, no event; a flip
-                    // toggles the state, takes its new schedule and the
-                    // band's force for that state (the rest of the full step)
-                    if (ETA && (int64_t)s == nflip) {
-                        t.state ^= 1;
-                        nflip = t.state ? ca1 : ca0;
-                        t.F = t.state ? bF1 : bF0;
-                    }
-                    if (t.state) ++sc1; else ++sc0;
-                    if (!OVER) t.v = t.v + (k.invM * t.F) * k.hdt;
-                    ++s;
-                    ++l;
-                    continue;
-                }
-                const FlipFromBuffer src{&buf.cand[u][0][l], &buf.cand[u][1][l]};
-                const int r = fp64_after_move<DBL, OVER, ETA>(k, st, i, g, t, s, src, nflip, sc0, sc1, flags, nxf,
-                                                              cell_prev, well_prev, lb_prev);
-                if (r == 1) { run = false; break; }
-                if (r == 2) { ++s; run = false; break; }
-                quiet_band<DBL>(k, t, &blo, &bhi);
-                band_forces<DBL>(k, t, &bF0, &bF1);
-                ++s;
-                ++l;
-            }
+    for (int m = 0; m < N; ++m) {
+        if (OVER) {
+            x = fma(F, k.c_drift, x);
+            x = x + rf[m];
+            x = x + r;
+            r = rf[m];
+        } else {
+            v = v + (k.invM * F) * k.hdt;
+            x = x + v * k.hdt;
+            v = k.expg * v + rf[m];
+            x = x + v * k.hdt;
         }
-        __syncwarp();
-        named_arrive(3 + u);                 // buffer u released
+        far = max(far, off_band(a, x));
+        if (nf == m) {
+            state ^= 1;
+            nf = m + (int)__byte_perm(w[m], 0, state ? 0x4432 : 0x4410);
+        }
+        F = state ? a.bF1 : a.bF0;
+        n1 += state;
+        if (!OVER) v = v + (k.invM * F) * k.hdt;
     }
-    if (lane != 0 || !active) return;   // a trajectory done before the launch keeps its state
-    // s is the first step not integrated
-    const int64_t n = st.n;
-    st.counts[(int64_t)LDP_C_STATE0 * n + i] = sc0;
-    st.counts[(int64_t)LDP_C_STATE1 * n + i] = sc1;
-    st.counts[(int64_t)LDP_C_STEPS * n + i] = (int64_t)s - 1;
-    if (k.fp_mode && !(t.bits & B_DONE) && s_end > k.step_cap) flags |= LDP_FLAG_CENSORED;
-    if (flags) st.counts[(int64_t)LDP_C_FLAGS * n + i] |= (int64_t)flags;
-    st.nflip[i] = nflip;
-    store_traj(st, t, i);
+    if (!(want && far < a.half)) return false;
+    a.t.x = x;
+    a.t.rprev = r;
+    a.t.v = v;
+    a.t.F = F;
+    a.t.state = state;
+    flip = l + nf;
+    a.sc1 += n1;
+    return true;
 }
 
-// ---------------------------------------------------------------------------
-// Group mode: mid-size runs (a few thousand trajectories).  Latency mode
-// gives each trajectory a CTA and saturates near 7e9 particle-steps/s; one
-// trajectory per thread leaves a few warps per SM, each waiting on its own
-// draws.  Here a CTA runs 32 trajectories: a consumer warp, lane l the
-// trajectory 32 blockIdx + l, steps them with latency mode's consumer code
-// (quiet steps, speculative sub-blocks, full steps through fp64_after_move),
-// and P producer warps draw their Gaussians and flip schedules for the
-// next 4 P steps into shared memory (producer lane p: the trajectory p mod
-// 32, the four consecutive steps 4 (p / 32) .. 4 (p / 32) + 3 of the block,
-// one Philox block and two Box-Muller pairs for them when the block starts
-// on a Philox block).  Two buffers alternate, handed over with named
-// barriers 5-6 ("full") and 7-8 ("empty") over all the CTA's warps; every
-// arrival is matched by one wait, with no spin loop.  Same inputs, same operations:
-// results equal the other kernels' and the oracle's bit for bit.
-// ---------------------------------------------------------------------------
-// P producer warps per CTA, 4 P steps per buffer (four consecutive steps
-// per producer lane); P = 4 up to kGrpWideMin trajectories, P = 2 above
-// (fewer warps per group, more groups per SM).
-constexpr int64_t kGrpWideMin = 8192;
-template <int P>
-struct GrpBuf {
-    double z[2][4 * P][32];          // [buffer][step][trajectory]
-    int64_t cand[2][2][4 * P][32];   // [buffer][new state][step][trajectory]
-};
-
-template <int P>
-__device__ __forceinline__ void grp_sync(int id) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(32 * (1 + P)) : "memory");
-}
-template <int P>
-__device__ __forceinline__ void grp_arrive(int id) {
-    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(32 * (1 + P)) : "memory");
-}
-
-template <bool DBL, bool OVER, bool ETA, int P>
-__global__ void __launch_bounds__(32 * (1 + P), 2) fp64_group_kernel(const KConst k, const TrajState st, int64_t g0,
-                                                                     uint64_t s_begin, uint64_t s_end) {
-    constexpr int kGrpBlock = 4 * P, kGrpProducers = P;
-    __shared__ GrpBuf<P> buf;
+template <bool DBL, bool OVER, bool ETA, bool DENSE>
+__global__ void __launch_bounds__(32 * (kGrpConsumers + kGrpProducers), 1) fp64_group_kernel(const KConst k, const TrajState st, int64_t g0,
+                                                            uint64_t s_begin, uint64_t s_end, int nc, int T, int B) {
+    // noise [2][M][R], then with DENSE waits [2][M][R]; rows of an odd length,
+    // so that lanes at the same step are in different banks
+    constexpr int N = kGrpSteps;
+    extern __shared__ double buf[];
+    const int M = nc * T, R = B + 1, nthreads = blockDim.x;
+    uint32_t* waits = (uint32_t*)(buf + 2 * R * M);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint64_t nblk = (s_end > s_begin) ? (s_end - s_begin + kGrpBlock - 1) / kGrpBlock : 0;
-    if (warp >= 1) {
+    const int64_t i0 = (int64_t)blockIdx.x * M;
+    const uint64_t a0 = (s_begin - 1) >> 2;           // the first buffer starts on a Philox block
+    const uint64_t sb = 4 * a0 + 1;
+    const uint64_t nblk = s_end > s_begin ? (s_end - sb + B - 1) / B : 0;
+    if (warp >= nc) {
         // ---- producers ----
-        const int p = (warp - 1) * 32 + lane;
-        const int tl = p & 31;               // the trajectory's lane
-        const int e0 = (p >> 5) * (kGrpBlock / kGrpProducers);   // its steps e0 .. e0 + 3 of each block
-        const int64_t ip = (int64_t)blockIdx.x * 32 + tl;
-        const uint32_t g = (uint32_t)(g0 + ip);
-        // the last Philox block's four Gaussians (a block serves four steps;
-        // a lane's four steps share one when the block start is aligned)
-        uint64_t aq = ~0ull;
-        double z0 = 0.0, z1 = 0.0, z2 = 0.0, z3 = 0.0;
+        const int p = (warp - nc) * 32 + lane, np = nthreads - 32 * nc;
+        const double sig = OVER ? k.sig_r : k.sig_v;
         for (uint64_t b = 0; b < nblk; ++b) {
             const int u = (int)(b & 1);
-            if (b >= 2) grp_sync<P>(7 + u);     // buffer u released by the consumer
-            for (int e = e0; e < e0 + kGrpBlock / kGrpProducers; ++e) {
-                const uint64_t s = s_begin + b * kGrpBlock + (uint64_t)e;
-                if (ip >= st.n || s >= s_end) continue;
-                const uint64_t a = (s - 1) >> 2;
-                if (a != aq) {
-                    const Words w = philox_at(a, g, TAG_STEP, k.key0, k.key1);
-                    gauss_pair_f64(w.w0, w.w1, &z0, &z1);
-                    gauss_pair_f64(w.w2, w.w3, &z2, &z3);
-                    aq = a;
-                }
-                const int q = (int)((s - 1) & 3);
-                buf.z[u][e][tl] = (q == 0) ? z0 : (q == 1) ? z1 : (q == 2) ? z2 : z3;
-                if (ETA) {
-                    const Words wf = philox_at(s, g, TAG_FLIP, k.key0, k.key1);
-                    flip_schedule_both(s, wf.w0, wf.w1, k.ln1m, &buf.cand[u][0][e][tl], &buf.cand[u][1][e][tl]);
+            if (b >= 2) bar_sync(3 + u, nthreads);   // buffer u released by the consumers
+            double* z = buf + u * R * M;
+            for (int e = p; e < (B >> 2) * M; e += np) {
+                const int quad = e / M, tr = e - quad * M;
+                const uint64_t q = a0 + b * (uint64_t)(B >> 2) + (uint64_t)quad;
+                if (i0 + tr >= st.n || 4 * q + 1 >= s_end) continue;
+                const Words w = philox_at(q, (uint32_t)(g0 + i0 + tr), TAG_STEP, k.key0, k.key1);
+                double z0, z1, z2, z3;
+                gauss_pair_f64(w.w0, w.w1, &z0, &z1);
+                gauss_pair_f64(w.w2, w.w3, &z2, &z3);
+                double* o = z + tr * R + quad * 4;
+                o[0] = sig * z0;
+                o[1] = sig * z1;
+                o[2] = sig * z2;
+                o[3] = sig * z3;
+            }
+            if (DENSE) {
+                uint32_t* wt = waits + u * R * M;
+                for (int e = p; e < B * M; e += np) {
+                    const int step = e / M, tr = e - step * M;
+                    const uint64_t s = sb + b * (uint64_t)B + (uint64_t)step;
+                    if (i0 + tr >= st.n || s >= s_end) continue;
+                    const Words wf = philox_at(s, (uint32_t)(g0 + i0 + tr), TAG_FLIP, k.key0, k.key1);
+                    wt[tr * R + step] = dense_waits(k, wf.w0, wf.w1);
                 }
             }
             __syncwarp();
-            grp_arrive<P>(5 + u);               // buffer u full
+            bar_arrive(1 + u, nthreads);             // buffer u full
         }
-        // the consumer's release of the last two buffers
-        for (uint64_t b = (nblk > 2 ? nblk - 2 : 0); b < nblk; ++b) grp_sync<P>(7 + (int)(b & 1));
+        // the consumers' release of the last two buffers
+        for (uint64_t b = (nblk > 2 ? nblk - 2 : 0); b < nblk; ++b) bar_sync(3 + (int)(b & 1), nthreads);
         return;
     }
-    // ---- consumer: lane l runs trajectory 32 blockIdx + l ----
-    const int64_t i = (int64_t)blockIdx.x * 32 + lane;
+    // ---- consumers ----
+    const int tr = warp * T + lane;
+    const int64_t i = i0 + tr;
     const uint32_t g = (uint32_t)(g0 + i);
-    T64 t;
-    int64_t sc0 = 0, sc1 = 0, nflip = 0;
-    uint32_t flags = 0;
-    uint64_t s = s_begin, nxf = 0;
-    bool run = false, active = false;
-    // quiet band (empty: the first step takes the full path) and the force
-    // in it for either barrier state
-    double blo = 1.0, bhi = 0.0, bF0 = 0.0, bF1 = 0.0;
-    if (i < st.n) {
-        load_traj(st, t, i);
-        active = run = !(t.bits & B_DONE);
-        sc0 = st.counts[(int64_t)LDP_C_STATE0 * st.n + i];
-        sc1 = st.counts[(int64_t)LDP_C_STATE1 * st.n + i];
-        energy_force<DBL>(k, t);
-        nflip = st.nflip[i];
-        const uint64_t fs = k.freq_save;
-        nxf = (s_begin + fs - 1) / fs * fs;
-    }
+    Lane a;
+    load_lane<DBL, OVER>(k, st, i, lane < T && i < st.n, a);
+    const bool active = (a.q & Q_RUN) != 0u;
+    const uint64_t fs = k.freq_save;
+    uint64_t s_done = s_end;   // this lane's first step not integrated
+    int64_t frame = (int64_t)((s_begin + fs - 1) / fs);   // this lane's next frame
+    double* px = st.fx ? st.fx + frame * st.n + i : nullptr;
+    const int ifs = fs < (1u << 30) ? (int)fs : 1 << 30;
+    const int tl = lane < T ? tr : warp * T;   // idle lanes read a lane's noise
+    auto near = [](int64_t d) { return d < (1 << 30) ? (int)d : 1 << 30; };
     for (uint64_t b = 0; b < nblk; ++b) {
         const int u = (int)(b & 1);
-        grp_sync<P>(5 + u);                     // buffer u full
-        if (run) {
-            const uint64_t s1 = (s_begin + (b + 1) * kGrpBlock < s_end) ? s_begin + (b + 1) * kGrpBlock : s_end;
-            const int nl = (int)(s1 - s);
-            // the next step's Gaussian and flip schedules are loaded one step
-            // ahead, so their shared-memory latency is off the chain (zn,
-            // cn0, cn1 hold step pf's)
-            double zn = buf.z[u][0][lane];
-            int64_t cn0 = 0, cn1 = 0;
-            if (ETA) {
-                cn0 = buf.cand[u][0][0][lane];
-                cn1 = buf.cand[u][1][0][lane];
+        bar_sync(1 + u, nthreads);                   // buffer u full
+        const double* z = buf + (u * M + tl) * R;
+        const uint32_t* wt = waits + (u * M + tl) * R;
+        const uint64_t s0 = sb + b * (uint64_t)B;
+        // Steps s0 + l, l < n; each lane at its own l: a lane goes on from a
+        // special step with a new block, and its warp waits for it at the
+        // buffer's end only.
+        const int n = s_end - s0 < (uint64_t)B ? (int)(s_end - s0) : B;
+        int l = b == 0 ? (int)(s_begin - sb) : 0;
+        if (!(a.q & Q_RUN)) l = n;
+        // the places of the next frame and of the pending flip, and the last
+        // place a block can start at
+        int fr = k.fp_mode ? 1 << 30 : near(frame * (int64_t)fs - (int64_t)s0);
+        int flip = near(a.nflip - (int64_t)s0);
+        auto save = [&]() {
+            if (frame < k.nframe) {
+                if (k.write_x) save_frame<DBL>(k, st, i, a, frame);
+                else if (px) *px = a.t.x;
             }
-            int pf = 0;
-            for (int l = 0; l < nl;) {
-                // Speculative sub-block: the next kLatSub steps run as quiet
-                // steps without the per-step band test, keeping the lowest
-                // and highest position; when every position stayed inside
-                // the quiet band (and no frame falls in the sub-block) they
-                // were quiet steps and stand, else the state at the
-                // sub-block's start is restored and the steps run one by one.
-                // x turning NaN stays NaN to the end, which the final test
-                // catches.
-                if (l + kLatSub <= nl && (l & (kLatSub - 1)) == 0 && (int64_t)nxf >= (int64_t)s + kLatSub &&
-                    t.x > blo && t.x < bhi) {
-                    double zb[kLatSub];
-                    int64_t c0b[kLatSub], c1b[kLatSub];
+            px += st.n;
+            ++frame;
+            fr = min(fr + ifs, 1 << 30);
+        };
+        auto last_start = [&]() { return min(min(n, fr + 1), ETA && !DENSE ? flip : n) - N; };
+        int lim = last_start();
+        while (__any_sync(0xffffffffu, l < n)) {
+            bool failed = false;
+            if (!__any_sync(0xffffffffu, l < n && l > lim)) {
+                // blocks, until a lane cannot go on with one
+                const bool flat = OVER && !DENSE && !__any_sync(0xffffffffu, (a.q & Q_FORCE) != 0u);
+                bool on, stop;
+#pragma unroll 1
+                do {
+                    on = l <= lim;
+                    const int lc = on ? l : 0;
+                    double rf[N];
 #pragma unroll
-                    for (int m = 0; m < kLatSub; ++m) {
-                        zb[m] = buf.z[u][l + m][lane];
-                        if (ETA) {
-                            c0b[m] = buf.cand[u][0][l + m][lane];
-                            c1b[m] = buf.cand[u][1][l + m][lane];
-                        }
+                    for (int m = 0; m < N; ++m) rf[m] = z[lc + m];
+                    bool stands;
+                    if (DENSE) {
+                        uint32_t w[N];
+#pragma unroll
+                        for (int m = 0; m < N; ++m) w[m] = wt[lc + m];
+                        stands = dense_block<OVER, N>(k, a, on, flip, lc, rf, w);
+                    } else if (flat) {
+                        stands = quiet_moves<OVER, true, N>(k, a, on, rf);
+                    } else {
+                        stands = quiet_moves<OVER, false, N>(k, a, on, rf);
                     }
-                    const double x0 = t.x, v0 = t.v, F0 = t.F, r0 = t.rprev;
-                    const int st0 = t.state;
-                    const int64_t nflip0 = nflip;
+                    l += stands ? N : 0;
+                    failed = on && !stands;
+                    stop = on && (failed || l > lim);
+                } while (!__any_sync(0xffffffffu, stop));
+            }
+            if (l < n && (failed || l > lim)) {
+                if (l != fr + 1) {
+                    // one by one, to the first special step and over it, or
+                    // to the next place where blocks can go on
+                    const int end = min(failed ? l + N : n, fr + 1);
                     int n1 = 0;
-                    double xmin = t.x, xmax = t.x;
-#pragma unroll
-                    for (int m = 0; m < kLatSub; ++m) {
-                        fp64_move<OVER>(k, t, zb[m]);
-                        xmin = fmin(xmin, t.x);
-                        xmax = fmax(xmax, t.x);
-                        if (ETA) {
-                            // flips by selects (t.F is the band's force of
-                            // the state throughout), so the steps form one
-                            // chain in x
-                            const bool f = (int64_t)s + m == nflip;
-                            t.state ^= (int)f;
-                            const int64_t cn = t.state ? c1b[m] : c0b[m];
-                            nflip = f ? cn : nflip;
-                            t.F = t.state ? bF1 : bF0;
+                    bool off;
+                    do {
+                        fp64_move<OVER>(k, a.t, z[l]);
+                        off = !(off_band(a, a.t.x) < a.half);
+                        if (off || (ETA && !DENSE && l == flip)) break;
+                        if (DENSE && l == flip) {
+                            a.t.state ^= 1;
+                            flip = l + (int)__byte_perm(wt[l], 0, a.t.state ? 0x4432 : 0x4410);
+                            a.t.F = a.t.state ? a.bF1 : a.bF0;
                         }
-                        n1 += t.state;
-                        if (!OVER) t.v = t.v + (k.invM * t.F) * k.hdt;
-                    }
-                    if (xmin > blo && xmax < bhi && t.x > blo) {
-                        sc1 += n1;
-                        sc0 += kLatSub - n1;
-                        s += kLatSub;
-                        l += kLatSub;
-                        continue;
-                    }
-                    t.x = x0;
-                    t.v = v0;
-                    t.F = F0;
-                    t.rprev = r0;
-                    t.state = st0;
-                    nflip = nflip0;
-                }
-                double z;
-                int64_t ca0 = 0, ca1 = 0;
-                if (pf == l) {
-                    z = zn;
-                    ca0 = cn0;
-                    ca1 = cn1;
-                } else {
-                    z = buf.z[u][l][lane];
-                    if (ETA) {
-                        ca0 = buf.cand[u][0][l][lane];
-                        ca1 = buf.cand[u][1][l][lane];
+                        n1 += a.t.state;
+                        if (!OVER) a.t.v = a.t.v + (k.invM * a.t.F) * k.hdt;
+                    } while (++l < end);
+                    a.sc1 += n1;
+                    if (l < end) {
+                        if (DENSE) {
+                            a.nflip = (int64_t)s0 + flip;
+                            const FlipFromBuffer src{wt[l]};
+                            special_step<DBL, OVER, ETA>(k, st, i, g, a, s0 + l, off, src);
+                        } else {
+                            const FlipDraw src;
+                            special_step<DBL, OVER, ETA>(k, st, i, g, a, s0 + l, off, src);
+                        }
+                        flip = near(a.nflip - (int64_t)s0);
+                        ++l;
                     }
                 }
-                if (l + 1 < nl) {
-                    zn = buf.z[u][l + 1][lane];
-                    if (ETA) {
-                        cn0 = buf.cand[u][0][l + 1][lane];
-                        cn1 = buf.cand[u][1][l + 1][lane];
-                    }
-                    pf = l + 1;
+                if (!(a.q & Q_RUN)) {
+                    s_done = s0 + l - ((a.flags & LDP_FLAG_NONFINITE) ? 1 : 0);
+                    l = n;
+                } else if (l == fr + 1) {
+                    save();
                 }
-                const int64_t cell_prev = t.cell, well_prev = t.well;
-                const int lb_prev = t.lb;
-                fp64_move<OVER>(k, t, z);
-                if (t.x > blo && t.x < bhi && (int64_t)s != (int64_t)nxf) {
-                    // a quiet step: same indices, no frame, no event; a flip
-                    // toggles the state, takes its new schedule and the
-                    // band's force for that state (the rest of the full step)
-                    if (ETA && (int64_t)s == nflip) {
-                        t.state ^= 1;
-                        nflip = t.state ? ca1 : ca0;
-                        t.F = t.state ? bF1 : bF0;
-                    }
-                    if (t.state) ++sc1; else ++sc0;
-                    if (!OVER) t.v = t.v + (k.invM * t.F) * k.hdt;
-                    ++s;
-                    ++l;
-                    continue;
-                }
-                const FlipFromBuffer src{&buf.cand[u][0][l][lane], &buf.cand[u][1][l][lane]};
-                const int r = fp64_after_move<DBL, OVER, ETA>(k, st, i, g, t, s, src, nflip, sc0, sc1, flags, nxf,
-                                                              cell_prev, well_prev, lb_prev);
-                if (r == 1) { run = false; break; }
-                if (r == 2) { ++s; run = false; break; }
-                quiet_band<DBL>(k, t, &blo, &bhi);
-                band_forces<DBL>(k, t, &bF0, &bF1);
-                ++s;
-                ++l;
+                lim = last_start();
             }
+            __syncwarp();
         }
+        if (l == fr + 1 && (a.q & Q_RUN)) save();   // at the buffer's end
+        if (DENSE && (a.q & Q_RUN)) a.nflip = (int64_t)s0 + flip;
         __syncwarp();
-        grp_arrive<P>(7 + u);                   // buffer u released
+        bar_arrive(3 + u, nthreads);                 // buffer u released
     }
-    if (!active) return;   // a trajectory done before the launch keeps its state
-    // s is the first step not integrated
-    const int64_t n = st.n;
-    st.counts[(int64_t)LDP_C_STATE0 * n + i] = sc0;
-    st.counts[(int64_t)LDP_C_STATE1 * n + i] = sc1;
-    st.counts[(int64_t)LDP_C_STEPS * n + i] = (int64_t)s - 1;
-    if (k.fp_mode && !(t.bits & B_DONE) && s_end > k.step_cap) flags |= LDP_FLAG_CENSORED;
-    if (flags) st.counts[(int64_t)LDP_C_FLAGS * n + i] |= (int64_t)flags;
-    st.nflip[i] = nflip;
-    store_traj(st, t, i);
+    if (active) store_lane(k, st, i, a, s_done, s_begin, s_end);
 }
 
 template <bool DBL, bool OVER>
@@ -1126,52 +1173,50 @@ static int launch_steps_t(const KConst& k, const TrajState& st, int64_t g0, uint
 }
 
 template <bool DBL, bool OVER, bool ETA>
-static int launch_latency_t(const KConst& k, const TrajState& st, int64_t g0, uint64_t s0, uint64_t s1,
-                            cudaStream_t stream) {
-    fp64_latency_kernel<DBL, OVER, ETA><<<(unsigned)st.n, 64, 0, stream>>>(k, st, g0, s0, s1);
+static int launch_group_t(const KConst& k, const TrajState& st, int64_t g0, uint64_t s0, uint64_t s1, int nc, int T,
+                          int P, int B, bool dense, cudaStream_t stream) {
+    const int M = nc * T;
+    const int64_t grid = (st.n + M - 1) / M;
+    const size_t smem = (size_t)2 * (B + 1) * M * (dense ? 12 : 8);
+    auto* kern = fp64_group_kernel<DBL, OVER, ETA, false>;
+    if (ETA && dense) kern = fp64_group_kernel<DBL, OVER, ETA, ETA>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    kern<<<(unsigned)grid, 32 * (nc + P), smem, stream>>>(k, st, g0, s0, s1, nc, T, B);
     return (int)cudaGetLastError();
 }
 
-int launch_fp64_latency(const KConst& k, const TrajState& st, int64_t g0, uint64_t s_begin, uint64_t s_end,
-                        void* stream) {
+int launch_fp64_group(const KConst& k, const TrajState& st, int64_t g0, uint64_t s_begin, uint64_t s_end, int sms,
+                      int min_lanes, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     if (st.n <= 0) return 0;
-    const int sel = (k.dbl ? 4 : 0) | (k.over ? 2 : 0) | (k.eta ? 1 : 0);
-    switch (sel) {
-        case 0: return launch_latency_t<false, false, false>(k, st, g0, s_begin, s_end, s);
-        case 1: return launch_latency_t<false, false, true>(k, st, g0, s_begin, s_end, s);
-        case 2: return launch_latency_t<false, true, false>(k, st, g0, s_begin, s_end, s);
-        case 3: return launch_latency_t<false, true, true>(k, st, g0, s_begin, s_end, s);
-        case 4: return launch_latency_t<true, false, false>(k, st, g0, s_begin, s_end, s);
-        case 5: return launch_latency_t<true, false, true>(k, st, g0, s_begin, s_end, s);
-        case 6: return launch_latency_t<true, true, false>(k, st, g0, s_begin, s_end, s);
-        default: return launch_latency_t<true, true, true>(k, st, g0, s_begin, s_end, s);
+    // One consumer warp to each of the GPU's schedulers, with as many lanes
+    // as that takes.
+    int T = (int)std::min<int64_t>(32, (st.n + 4 * sms - 1) / (4 * sms));
+    T = std::max(T, min_lanes);
+    const int nc = (int)std::min<int64_t>(kGrpConsumers, (st.n + (int64_t)sms * T - 1) / ((int64_t)sms * T));
+    const int M = nc * T;
+    double p = 0.0, pmin = 1.0;
+    for (int b = 0; b < 2; ++b) {
+        const double f = k.eta ? -std::expm1(k.ln1m[b]) : 0.0;
+        p = std::max(p, f);
+        pmin = std::min(pmin, f);
     }
-}
-
-template <bool DBL, bool OVER, bool ETA>
-static int launch_group_t(const KConst& k, const TrajState& st, int64_t g0, uint64_t s0, uint64_t s1,
-                          cudaStream_t stream) {
-    const int64_t grid = (st.n + 31) / 32;
-    if (st.n > kGrpWideMin) fp64_group_kernel<DBL, OVER, ETA, 2><<<(unsigned)grid, 96, 0, stream>>>(k, st, g0, s0, s1);
-    else fp64_group_kernel<DBL, OVER, ETA, 4><<<(unsigned)grid, 160, 0, stream>>>(k, st, g0, s0, s1);
-    return (int)cudaGetLastError();
-}
-
-int launch_fp64_group(const KConst& k, const TrajState& st, int64_t g0, uint64_t s_begin, uint64_t s_end,
-                      void* stream) {
-    cudaStream_t s = (cudaStream_t)stream;
-    if (st.n <= 0) return 0;
+    const bool dense = k.eta && pmin >= 1.0 / 1024 && p * T > 1.0 / 40;
+    const int P = kGrpProducers;
+    int B = 8 * ((32 * P * kGrpItems * 4 / M + 7) / 8);
+    const int room = (200 << 10) / (2 * M * (dense ? 12 : 8)) - 1;   // shared memory
+    B = std::min(std::min(std::max(B, 16), kGrpBuffer), room / 8 * 8);
     const int sel = (k.dbl ? 4 : 0) | (k.over ? 2 : 0) | (k.eta ? 1 : 0);
     switch (sel) {
-        case 0: return launch_group_t<false, false, false>(k, st, g0, s_begin, s_end, s);
-        case 1: return launch_group_t<false, false, true>(k, st, g0, s_begin, s_end, s);
-        case 2: return launch_group_t<false, true, false>(k, st, g0, s_begin, s_end, s);
-        case 3: return launch_group_t<false, true, true>(k, st, g0, s_begin, s_end, s);
-        case 4: return launch_group_t<true, false, false>(k, st, g0, s_begin, s_end, s);
-        case 5: return launch_group_t<true, false, true>(k, st, g0, s_begin, s_end, s);
-        case 6: return launch_group_t<true, true, false>(k, st, g0, s_begin, s_end, s);
-        default: return launch_group_t<true, true, true>(k, st, g0, s_begin, s_end, s);
+        case 0: return launch_group_t<false, false, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
+        case 1: return launch_group_t<false, false, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
+        case 2: return launch_group_t<false, true, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
+        case 3: return launch_group_t<false, true, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
+        case 4: return launch_group_t<true, false, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
+        case 5: return launch_group_t<true, false, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
+        case 6: return launch_group_t<true, true, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
+        default: return launch_group_t<true, true, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
     }
 }
 
