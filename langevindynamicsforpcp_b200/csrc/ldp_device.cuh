@@ -40,24 +40,10 @@ enum : uint32_t { TAG_STEP = 0, TAG_INIT = 1, TAG_CATCHUP = 2, TAG_CELL = 3, TAG
 
 struct Words { uint32_t w0, w1, w2, w3; };
 
+// Philox4x32-10 with 32 x 32 -> 64-bit products (one wide multiply gives both
+// halves).
 __device__ __forceinline__ Words philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
                                         uint32_t k0, uint32_t k1) {
-#pragma unroll
-    for (int r = 0; r < 10; ++r) {
-        if (r) { k0 += 0x9E3779B9u; k1 += 0xBB67AE85u; }
-        const uint32_t lo0 = 0xD2511F53u * c0, hi0 = __umulhi(0xD2511F53u, c0);
-        const uint32_t lo1 = 0xCD9E8D57u * c2, hi1 = __umulhi(0xCD9E8D57u, c2);
-        const uint32_t n0 = hi1 ^ c1 ^ k0;
-        const uint32_t n2 = hi0 ^ c3 ^ k1;
-        c0 = n0; c1 = lo1; c2 = n2; c3 = lo0;
-    }
-    return Words{c0, c1, c2, c3};
-}
-
-// The same function written with 32 x 32 -> 64-bit products (one wide
-// multiply per product gives both halves); identical output.
-__device__ __forceinline__ Words philox_wide(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
-                                             uint32_t k0, uint32_t k1) {
 #pragma unroll
     for (int r = 0; r < 10; ++r) {
         if (r) { k0 += 0x9E3779B9u; k1 += 0xBB67AE85u; }

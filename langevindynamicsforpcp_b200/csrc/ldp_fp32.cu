@@ -23,14 +23,14 @@
 // countdown ended.  If not (about one block in five), the lanes concerned take
 // the block again step by step.  Their special steps are quick steps, inline
 // (a frame, a flank entered or left, the edge between the two cells of a pair
-// crossed), or take the slow path out of line: a light step, or the general
-// step, which follows the FP64 step exactly (wrap, indices, flip, cell-table
-// entry with lazy catch-up, force, renewal statistics, frame, end).
+// crossed, a flip where flips are frequent), or take the slow path out of line
+// (special_step): at last the general step, which follows the FP64 step
+// exactly (wrap, indices, flip, cell-table entry with lazy catch-up, force,
+// renewal statistics, frame, end).
 //
 // What bounds it: instruction issue.  4 jobs x 65536 trajectories x 120000
 // steps, frames every 100: 76.8 ms with a test and a branch at each step and
-// light steps (an out-of-line call's worth of state around them), 59.6 ms
-// with this loop.
+// ten dependent loads in each special step, 59.5 ms with this loop.
 // The loop is a function without calls (run_blocks, no spills at 48 registers
 // and more), the lane state in shared memory between it and the out-of-line
 // parts: with the calls inside it the loop kept three of its values on the
@@ -65,15 +65,23 @@ enum : uint32_t { B_HAS_FPT = 1u << 24, B_HAS_FPT2 = 1u << 25, B_HAS_TPT = 1u <<
 // the cell left last (valid, its state).
 enum : int32_t { W_LB = 1, W_EVICT = 2, W_CVALID = 4, W_CSTATE = 8 };
 
+// Model type K: 0-3 (double * 2 + overdamped), or 4, the job's, for code
+// that serves all four.
+template <int K>
+__device__ __forceinline__ bool is_double(const JobF& J) { return K < 4 ? (K & 2) != 0 : J.dbl != 0; }
+template <int K>
+__device__ __forceinline__ bool is_over(const JobF& J) { return K < 4 ? (K & 1) != 0 : J.over != 0; }
+
 // The word of a lane's quick steps (see quick_step), kept in a register by
 // the hot loop: quick steps allowed (the barrier flanks do not reach the cell
 // edges); the lane's cell and a neighbour form a pair whose shared edge it may
 // cross quickly; it is in the pair's other cell now; the other cell is the
 // right neighbour; the two barriers' states; the countdown ends at a frame
-// and nothing else; the pair's edge was crossed at least once.
+// and nothing else; the pair's edge was crossed at least once; the other
+// cell's pending flip has come.
 enum : uint32_t {
     P_FAST = 1, P_PAIR = 2, P_SWAP = 4, P_RIGHT = 8, P_S0 = 16, P_S1 = 32, P_FRAME = 64, P_CROSSED = 128,
-    P_HALT = 256
+    P_OVERDUE = 256, P_HALT = 512
 };
 
 // Per-thread rare state, structure of arrays (conflict-free by thread).
@@ -93,6 +101,7 @@ struct RareSm {
     // Lane state the hot loop hands to the general step and takes back, and
     // the lane state only the general step uses.
     float xp[kMaxBlock], rv[kMaxBlock], F[kMaxBlock], lo[kMaxBlock], hi[kMaxBlock];
+    float4 nz[kMaxBlock];         // noise of a block's steps after one that needs the slow path
     uint4 fix[kMaxBlock];         // Philox constants of the lane's step blocks (philox_fix) ...
     uint2 fixk[kMaxBlock];        // ... the first key word of its third round, and the noise scale (float bits)
     uint32_t traj[kMaxBlock];
@@ -196,8 +205,7 @@ __device__ __forceinline__ int f_ring_state(const JobF& J, const SlotsDev& S, in
 
 // FP32 force of state st at xp (EnergyAndForce, S.h:1292-1324 /
 // D.h:1464-1522).
-template <bool DBL>
-__device__ __forceinline__ float force_of(const JobF& J, float xp, int st) {
+__device__ __forceinline__ float force_of(const bool DBL, const JobF& J, float xp, int st) {
     if (!DBL) {
         const float a = fabsf(xp);
         return (a < J.w && a > 0.0f) ? copysignf(J.slope[st], xp) : 0.0f;
@@ -214,8 +222,7 @@ __device__ __forceinline__ float force_of(const JobF& J, float xp, int st) {
 // Open band (lo, hi) of consecutive breakpoints around xp; lo = hi = xp when
 // xp sits on a breakpoint, so that the next step takes the general path.
 // Single barrier: the breakpoints are -L/2, -w, 0, w (clamped to the cell).
-template <bool DBL>
-__device__ __forceinline__ void band_of(const JobF& J, float xp, float* lo, float* hi) {
+__device__ __forceinline__ void band_of(const bool DBL, const JobF& J, float xp, float* lo, float* hi) {
     if (!DBL) {
         const float w = J.w, hL = J.halfL, a = fabsf(xp);
         float l, h;
@@ -239,8 +246,7 @@ __device__ __forceinline__ void band_of(const JobF& J, float xp, float* lo, floa
     *hi = h;
 }
 
-template <bool DBL>
-__device__ void f_energy(const JobF& J, double xp, int s, double* E, double* B) {
+__device__ __forceinline__ void f_energy(const bool DBL, const JobF& J, double xp, int s, double* E, double* B) {
     if (!DBL) {
         const double sp = J.Hs[s] / J.wd, sn = -sp;
         double e = 0.0;
@@ -260,11 +266,10 @@ __device__ void f_energy(const JobF& J, double xp, int s, double* E, double* B) 
 }
 
 // WRITEX frame fields (velocity, force, barrier, energies, state).
-template <bool DBL>
-__device__ __noinline__ void f_record_extra(const JobF* Jp, int64_t o, float xp, float v, float F, int state) {
+__device__ __noinline__ void f_record_extra(bool DBL, const JobF* Jp, int64_t o, float xp, float v, float F, int state) {
     const JobF& J = *Jp;
     double E, B;
-    f_energy<DBL>(J, (double)xp, state, &E, &B);
+    f_energy(DBL, J, (double)xp, state, &E, &B);
     if (J.fv) J.fv[o] = (double)v;
     if (J.ff) J.ff[o] = (double)F;
     if (J.fb) J.fb[o] = B;
@@ -273,13 +278,12 @@ __device__ __noinline__ void f_record_extra(const JobF* Jp, int64_t o, float xp,
     if (J.fst) J.fst[o] = (double)state;
 }
 
-template <bool DBL>
-__device__ __forceinline__ void f_record(const JobF& J, uint32_t traj, int64_t frame, int cell, float xp, float v,
+__device__ __forceinline__ void f_record(const bool DBL, const JobF& J, uint32_t traj, int64_t frame, int cell, float xp, float v,
                                          float F, int state) {
     if (frame >= J.nframe) return;   // the frame arrays hold nframe rows
     const int64_t o = frame * J.ntraj + traj;
     if (J.fx) J.fx[o] = (double)cell * J.Ld + (double)xp;
-    if (J.write_x) f_record_extra<DBL>(&J, o, xp, v, F, state);
+    if (J.write_x) f_record_extra(DBL, &J, o, xp, v, F, state);
 }
 
 __device__ __forceinline__ bool cg_hit32(int well, int size) { return (well % size) == 0; }
@@ -287,10 +291,11 @@ __device__ __forceinline__ bool cg_hit32(int well, int size) { return (well % si
 // Step 0 of a trajectory (IntegrateStep0 + InitializeBarrierState +
 // InitializeStatistics), FP64 where it is cheap and exact, then the hot
 // state is rounded to FP32.  Writes the thread's rare state.
-template <bool DBL, bool OVER>
+template <int K>
 __device__ __noinline__ void f_start(const JobF* Jp, longlong2* ring, int64_t nslots, int ring_slots, int64_t slot,
                                      uint32_t traj, RareSm* sm, int t) {
     const JobF& J = *Jp;
+    const bool DBL = is_double<K>(J), OVER = is_over<K>(J);
     const uint32_t g = traj + J.g0;   // the trajectory's random streams
     float* xp = &sm->xp[t];
     float* rv = &sm->rv[t];
@@ -382,8 +387,8 @@ __device__ __noinline__ void f_start(const JobF* Jp, longlong2* ring, int64_t ns
     *sw = l ? W_LB : 0;
     *rv = OVER ? (float)(J.sig_r_d * zr) : (float)v;
     if (!J.fp_mode) {
-        const float F = force_of<DBL>(J, *xp, st);
-        f_record<DBL>(J, traj, 0, c, *xp, OVER ? 0.0f : (float)v, F, st);
+        const float F = force_of(DBL, J, *xp, st);
+        f_record(DBL, J, traj, 0, c, *xp, OVER ? 0.0f : (float)v, F, st);
     }
 }
 
@@ -432,9 +437,21 @@ __device__ __forceinline__ float one_minus_exp(float x) {
     return 1.0f - expf(x);
 }
 
+// State at step s of a barrier entered then that was in state sb after its
+// missed flip at step nb, and its new pending flip: flip with probability
+// c (1 - e^{a lap}) over the steps since, FP32, against the high word of the
+// same catch-up uniform the FP64 path draws.
+__device__ __forceinline__ int caught_up(const JobF& J, uint32_t g, uint64_t s, long long nb, int sb, const Words& wf,
+                                         long long* nf) {
+    const float pl = J.c_lapf[J.eq ? 0 : sb] * one_minus_exp(J.a_lapf * (float)((long long)s - nb));
+    const uint32_t w0 = philox_at(s, g, TAG_CATCHUP, J.key0, J.key1).w0;
+    const int sn = ((pl >= 1.0f) || (w0 < (uint32_t)(pl * 4294967296.0f))) ? (sb ^ 1) : sb;
+    *nf = flip_schedule(s, wf.w2, wf.w3, J.ln1m[sn]);
+    return sn;
+}
+
 // End of a trajectory after step `done` (v: velocity after that step).
-template <bool OVER>
-__device__ __forceinline__ void retire_lane(const JobF& J, unsigned long long* retired, RareSm& sm, int t,
+__device__ __forceinline__ void retire_lane(const bool OVER, const JobF& J, unsigned long long* retired, RareSm& sm, int t,
                                             uint64_t done, float xp, float v, uint32_t flags) {
     const int state = sm.state[t];
     const int64_t sc1 = sm.sc1[t] + (state ? (int64_t)done + 1 - sm.since[t] : 0);
@@ -485,21 +502,19 @@ __device__ __forceinline__ void idle_lane(RareSm& sm, int t) {
 // Ends a lane's trajectory after step `done` (general step): keeps its
 // continuation state when the job asks for it and the trajectory completed,
 // then retires it.  The lane's cell, state and slot word in sm are current.
-template <bool OVER>
-__device__ __noinline__ void f_end_lane(const JobF* Jp, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
+__device__ __noinline__ void f_end_lane(bool OVER, const JobF* Jp, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
                                         uint64_t done, float xp, float v, float rv, uint32_t flags) {
     const JobF& J = *Jp;
     RareSm& sm = *smp;
     if (J.ck_xp && !flags && done == J.nsteps)
         f_keep_state(Jp, Sp, smp, t, slot, sm.traj[t], xp, OVER ? rv : v, sm.cell[t], sm.sw[t]);
-    retire_lane<OVER>(J, Sp->retired, sm, t, done, xp, v, flags);
+    retire_lane(OVER, J, Sp->retired, sm, t, done, xp, v, flags);
 }
 
 // The general step s of one lane (position already advanced):
 // the FP64 step order of ldp_fp64.cu from the index update on, on the lane
 // state in shared memory.
-template <bool DBL, bool OVER>
-__device__ __forceinline__ void general_step(const JobF* jobs, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
+__device__ __forceinline__ void general_step(const bool DBL, const bool OVER, const JobF* jobs, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
                                           uint64_t s) {
     RareSm& sm = *smp;
     const SlotsDev& S = *Sp;
@@ -519,7 +534,7 @@ __device__ __forceinline__ void general_step(const JobF* jobs, const SlotsDev* S
         sm.cell[t] = cell;
         sm.state[t] = state;
         sm.sw[t] = sw;
-        f_end_lane<OVER>(&J, &S, &sm, t, slot, done, xp, v, rv, flags);
+        f_end_lane(OVER, &J, &S, &sm, t, slot, done, xp, v, rv, flags);
         idle_lane(sm, t);
     };
 
@@ -563,16 +578,8 @@ __device__ __forceinline__ void general_step(const JobF* jobs, const SlotsDev* S
             *nf = nb;
             return ps;
         }
-        // Flip with probability c (1 - e^{a lap}) over the steps since the
-        // missed flip, FP32, against the high word of the same catch-up
-        // uniform the FP64 path draws.
-        const int sb = found ? (ps ^ 1) : ps;
-        const float pl = J.c_lapf[J.eq ? 0 : sb] * one_minus_exp(J.a_lapf * (float)((long long)s - nb));
-        const uint32_t w0 = philox_at(s, gp, TAG_CATCHUP, J.key0, J.key1).w0;
-        const int sn = ((pl >= 1.0f) || (w0 < (uint32_t)(pl * 4294967296.0f))) ? (sb ^ 1) : sb;
         if (!have_wf) *wf = philox_at(s, gp, TAG_FLIP, J.key0, J.key1);
-        *nf = flip_schedule(s, wf->w2, wf->w3, J.ln1m[sn]);
-        return sn;
+        return caught_up(J, gp, s, nb, found ? (ps ^ 1) : ps, *wf, nf);
     };
 
     // Renewal statistics (UpdateStatistics, S.h:2334-2592 / D.h:2931-3209)
@@ -679,29 +686,12 @@ __device__ __forceinline__ void general_step(const JobF* jobs, const SlotsDev* S
         return done;
     };
 
-    if (J.eta && xp > lo && xp < hi && (long long)s == sm.nflip[t] && (long long)s != sm.nxf[t] &&
-        s != J.nsteps && (xp < 0.0f) == (lo < 0.0f) && (!DBL || (xp < J.xc ? 0 : W_LB) == (sw & W_LB))) {
-        // Only the current barrier's flip (no band exit, so the same cell,
-        // well and local barrier; no frame; not the last step): the path
-        // below with flip alone -- the new state and its schedule, the
-        // state-1 run, the state's force, the countdown.
-        const int st = state ^ 1;
-        const Words w = philox_at(s, gp, TAG_FLIP, J.key0, J.key1);
-        const long long nf = flip_schedule(s, w.w0, w.w1, J.ln1m[st]);
-        if (st) sm.since[t] = (long long)s;
-        else sm.sc1[t] += (long long)s - sm.since[t];
-        sm.state[t] = st;
-        sm.nflip[t] = nf;
-        sm.F[t] = force_of<DBL>(J, xp, st);
-        sm.left[t] = steps_to_special(J, s, sm.nxf[t], nf);
-        return;
-    }
     if (xp > lo && xp < hi && (long long)s != sm.nflip[t]) {
         // Only the countdown ran out: a frame and/or the last step.
         const float F = sm.F[t];
         const float vk = OVER ? 0.0f : fmaf(F, J.hdt_invM, rv);
         if ((long long)s == sm.nxf[t]) {
-            f_record<DBL>(J, traj, sm.fidx[t], cell, xp, vk, F, state);
+            f_record(DBL, J, traj, sm.fidx[t], cell, xp, vk, F, state);
             sm.fidx[t] += 1;
             sm.nxf[t] += (long long)J.freq_save;
         }
@@ -755,14 +745,14 @@ __device__ __forceinline__ void general_step(const JobF* jobs, const SlotsDev* S
         sm.nflip[t] = nf;
         left = 0;   // recompute the countdown below
     }
-    band_of<DBL>(J, xp, &lo, &hi);
-    const float F = force_of<DBL>(J, xp, state);
+    band_of(DBL, J, xp, &lo, &hi);
+    const float F = force_of(DBL, J, xp, state);
     bool finish = false;
     if (dCell || dWell) finish = events((int64_t)s, dWell, dCell, well);
     const float vk = OVER ? 0.0f : fmaf(F, J.hdt_invM, rv);
     if (left == 0) {
         if ((long long)s == sm.nxf[t]) {
-            f_record<DBL>(J, traj, sm.fidx[t], cell, xp, vk, F, state);
+            f_record(DBL, J, traj, sm.fidx[t], cell, xp, vk, F, state);
             sm.fidx[t] += 1;
             sm.nxf[t] += (long long)J.freq_save;
         }
@@ -780,111 +770,6 @@ __device__ __forceinline__ void general_step(const JobF* jobs, const SlotsDev* S
     if (finish) retire(s, vk, 0);
 }
 
-// The light step: special steps with few consequences, with the same result
-// the general step gives them.  Returns false when the step needs the general
-// step.
-//  * A frame step (the countdown ends at a frame, not at a flip or the last
-//    step), the position inside its band, no WRITEX series: the frame is
-//    written (FP64 cell * L + xp) and the countdown restarts.
-//  * A band exit inside the cell (a barrier flank entered or left), with no
-//    change of well (barrier top) or local barrier: new band and force.
-//  * A crossing of the cell edge into the flat band of the neighbour cell
-//    whose barrier is the cached one (the cell left last) and has not passed
-//    its pending flip, with no flip at this step and no renewal statistic
-//    firing (every statistic already holds this well): the barrier state,
-//    pending flip and state-1 run change as in the general step's cell
-//    entry, the ring is written through, the transition-path clocks restart.
-template <bool DBL>
-__device__ __forceinline__ bool light_step(const JobF& J, const SlotsDev& S, RareSm& sm, int t, int64_t slot,
-                                           uint32_t traj, uint64_t s, bool countdown, float& xp, float& lo, float& hi,
-                                           float& F) {
-    const long long nflip = sm.nflip[t];
-    if (countdown) {
-        const long long nxf = sm.nxf[t];
-        if (!(xp > lo && xp < hi) || (long long)s != nxf || (long long)s == nflip || s == J.nsteps || J.write_x)
-            return false;
-        const int fidx = sm.fidx[t];
-        if (fidx < J.nframe && J.fx) J.fx[(int64_t)fidx * J.ntraj + traj] = (double)sm.cell[t] * J.Ld + (double)xp;
-        sm.fidx[t] = fidx + 1;
-        sm.nxf[t] = nxf + (long long)J.freq_save;
-        return true;
-    }
-    if ((long long)s == nflip) return false;
-    const float hL = J.halfL;
-    int sw = sm.sw[t];
-    if (xp >= -hL && xp < hL) {
-        // inside the cell: a band change unless the well or the local
-        // barrier changes, or xp sits on a breakpoint
-        float l2, h2;
-        band_of<DBL>(J, xp, &l2, &h2);
-        if (!(xp > l2 && xp < h2)) return false;
-        if ((xp < 0.0f) != (lo < 0.0f)) return false;
-        if (DBL && ((xp < J.xc ? 0 : W_LB) != (sw & W_LB))) return false;
-        lo = l2;
-        hi = h2;
-        F = force_of<DBL>(J, xp, sm.state[t]);
-        return true;
-    }
-    if (!J.edge_flat || !J.eta) return false;
-    float xn;
-    int dc;
-    if (xp >= hL) {
-        xn = xp - J.L;
-        dc = 1;
-        if (!(xn > -hL && xn < J.edge_lo)) return false;
-    } else if (xp < -hL) {
-        xn = xp + J.L;
-        dc = -1;
-        if (!(xn > J.edge_hi && xn < hL)) return false;
-    } else {
-        return false;   // not finite
-    }
-    const int cell_prev = sm.cell[t], cell = cell_prev + dc;
-    const int well = cell - (xn < 0.0f ? 1 : 0);
-    if (well != cell_prev - (lo < 0.0f ? 1 : 0)) return false;
-    const int lb = DBL ? (xn < J.xc ? 0 : 1) : 0;
-    if (DBL && lb == (sw & W_LB)) return false;   // the general step enters a key only when lb changes
-    const int key_prev = fkey(DBL, cell_prev, sw & W_LB), key = fkey(DBL, cell, lb);
-    if (!(sw & W_CVALID) || sm.ckey[t] != key || sm.cflip[t] <= (long long)s) return false;
-    const uint32_t bits = sm.bits[t];
-    const int evm = J.evm;
-    if ((evm & EV_FPT) && (bits & B_FPT_UP)) return false;
-    if ((evm & EV_FPT2) && ((bits & B_FPT2_UP) || sm.idx2[t] != well)) return false;
-    if ((evm & EV_TPT) && !(bits & B_TPT2_UP) && sm.tpt2w[t] != well) return false;
-    if ((evm & EV_CG) && sm.cgw[t] != well) return false;
-    if ((evm & EV_WT) && (bits & B_WT_PASSED)) return false;
-    // leave key_prev (its eviction, if its entry displaced another cell's,
-    // is counted now), enter the cached key
-    const int st_prev = sm.state[t];
-    if (sw & W_EVICT) red_add(&J.counts[(int64_t)LDP_C_EVICT * J.ntraj + traj], 1);
-    S.ring[(int64_t)(key_prev & (S.ring_slots - 1)) * S.nslots + slot] =
-        make_longlong2((long long)key_prev, (nflip << 1) | (long long)st_prev);
-    const int ps = (sw & W_CSTATE) ? 1 : 0;
-    const long long nb = sm.cflip[t];
-    sm.ckey[t] = key_prev;
-    sm.cflip[t] = nflip;
-    sm.nflip[t] = nb;
-    sw = (DBL ? (lb ? W_LB : 0) : (sw & W_LB)) | W_CVALID | (st_prev ? W_CSTATE : 0);
-    sm.sw[t] = sw;
-    if (ps != st_prev) {
-        if (ps) sm.since[t] = (long long)s;
-        else sm.sc1[t] += (long long)s - sm.since[t];
-        sm.state[t] = ps;
-    }
-    sm.cell[t] = cell;
-    if (evm & EV_TPT) {
-        sm.bits[t] = bits & ~(B_TPT_UP | B_TPT2_UP);
-        sm.tpt[t] = (long long)s;
-        sm.tpt2[t] = (long long)s;
-        sm.tpt2w[t] = well;
-    }
-    xp = xn;
-    if (dc > 0) { lo = -hL; hi = J.edge_lo; }
-    else { lo = J.edge_hi; hi = hL; }
-    F = 0.0f;
-    return true;
-}
-
 // The last step after s whose block index has the same high word as the
 // next step's: a special step, since the lane's Philox constants hold it.
 __device__ __forceinline__ long long block_wrap(uint64_t s) { return (long long)(((s >> 34) + 1) << 34); }
@@ -897,22 +782,36 @@ __device__ __forceinline__ void bind_block(const JobF& J, RareSm& sm, int t, uin
     sm.fixk[t] = make_uint2(J.key0 + 2u * 0x9E3779B9u, __float_as_uint(J.bm_k));
 }
 
+// The countdown from step s to the next frame or to nev, the first step that
+// is special for another reason; the lane's P_* word.
+__device__ __forceinline__ void count_down(const JobF& J, RareSm& sm, int t, uint64_t s, long long nev, int& left,
+                                           uint32_t& pw) {
+    const long long nxf = sm.nxf[t];
+    long long d = (nxf < nev ? nxf : nev) - (long long)s;
+    d = d > 1 ? d : 1;   // (both lie after s)
+    if (nxf < nev && d <= (long long)kLeftMax && !J.write_x) pw |= P_FRAME;
+    sm.nev[t] = nev;
+    left = (int)(d < (long long)kLeftMax ? d : (long long)kLeftMax);
+}
+
 // After a special step s (or before the first step, s one less): the word of
 // the lane's quick steps and its countdown.  A pair is formed when a crossing
-// of the nearer cell edge would be a light crossing (light_step) and stays
+// of the nearer cell edge would change the barrier and restart the transition
+// clocks and nothing else, and stays
 // one, whatever the number of crossings, until the next special step: the
 // neighbour is the cached cell, no statistic fires, no eviction is pending.
 // The countdown also ends at the neighbour's pending flip, past which its
-// cached state is no longer known.
-template <bool DBL>
-__device__ __forceinline__ void settle(const JobF& J, RareSm& sm, int t, uint64_t s, float xp) {
+// cached state is no longer known (P_OVERDUE).
+__device__ __noinline__ void settle(bool DBL, const JobF* Jp, RareSm* smp, int t, uint64_t s, float xp) {
+    const JobF& J = *Jp;
+    RareSm& sm = *smp;
     const int state = sm.state[t], sw = sm.sw[t], cell = sm.cell[t];
     uint32_t pw = (state ? P_S0 : 0u) | (J.edge_flat ? P_FAST : 0u);
     long long nev = sm.nflip[t] < (long long)J.nsteps ? sm.nflip[t] : (long long)J.nsteps;
     const long long wrap = block_wrap(s);
     nev = wrap < nev ? wrap : nev;
     if ((s & ((1ull << 34) - 1)) == 0) bind_block(J, sm, t, s);   // a new high word from the next step on
-    if (J.edge_flat && J.eta && (sw & W_CVALID) && !(sw & W_EVICT) && sm.cflip[t] > (long long)s) {
+    if (J.edge_flat && J.eta && (sw & W_CVALID) && !(sw & W_EVICT)) {
         const bool right = !(xp < 0.0f);
         const int lb = sw & W_LB;
         const int well = cell - (right ? 0 : 1);
@@ -927,22 +826,46 @@ __device__ __forceinline__ void settle(const JobF& J, RareSm& sm, int t, uint64_
         ok = ok && !((evm & EV_WT) && (bits & B_WT_PASSED));
         if (ok) {
             pw |= P_PAIR | (right ? P_RIGHT : 0u) | ((sw & W_CSTATE) ? P_S1 : 0u);
-            nev = sm.cflip[t] < nev ? sm.cflip[t] : nev;
+            if (sm.cflip[t] <= (long long)s) pw |= P_OVERDUE;
+            else nev = sm.cflip[t] < nev ? sm.cflip[t] : nev;
         }
     }
-    const long long nxf = sm.nxf[t];
-    const long long d = (nxf < nev ? nxf : nev) - (long long)s;
-    if (nxf < nev && d <= (long long)kLeftMax && !J.write_x) pw |= P_FRAME;
-    sm.nev[t] = nev;
-    sm.left[t] = (int)(d < (long long)kLeftMax ? d : (long long)kLeftMax);
+    int left;
+    count_down(J, sm, t, s, nev, left, pw);
+    sm.left[t] = left;
     sm.pw[t] = pw;
 }
 
-// Leaves a pair: the lane state as light crossings would have left it (the
+// The current barrier's flip at step s and nothing else, the lane in its
+// pair's first cell: its new state and pending flip, the state-1 run, the
+// force, the countdown; a pair stays one.
+__device__ __forceinline__ bool only_flip(const JobF& J, const RareSm& sm, int t, uint64_t s, uint32_t pw) {
+    return (pw & P_FAST) && !(pw & P_CROSSED) && (long long)s == sm.nflip[t] && (long long)s < sm.nxf[t] &&
+           s < J.nsteps && (s & ((1ull << 34) - 1)) != 0;
+}
+__device__ __forceinline__ void flip_here(const bool DBL, const JobF& J, RareSm& sm, int t, uint64_t s, float xp,
+                                          float& F, int& left, uint32_t& pw) {
+    pw = (pw & ~P_FRAME) ^ P_S0;
+    const int st = (pw & P_S0) ? 1 : 0;
+    const Words w = philox_at(s, sm.traj[t] + J.g0, TAG_FLIP, J.key0, J.key1);
+    const long long nf = flip_schedule(s, w.w0, w.w1, J.ln1m[st]);
+    if (st) sm.since[t] = (long long)s;
+    else sm.sc1[t] += (long long)s - sm.since[t];
+    sm.state[t] = st;
+    sm.nflip[t] = nf;
+    F = force_of(DBL, J, xp, st);
+    long long nev = block_wrap(s);
+    nev = (long long)J.nsteps < nev ? (long long)J.nsteps : nev;
+    nev = nf < nev ? nf : nev;
+    if (sm.cflip[t] <= (long long)s) pw |= P_OVERDUE;
+    if ((pw & (P_PAIR | P_OVERDUE)) == P_PAIR) nev = sm.cflip[t] < nev ? sm.cflip[t] : nev;
+    count_down(J, sm, t, s, nev, left, pw);
+}
+
+// Leaves a pair: the lane state as general steps would have left it (the
 // ring entry of the cell first left, the transition-path clocks, and, in the
 // pair's other cell, the swapped barriers).
-template <bool DBL>
-__device__ __forceinline__ void unpair(const JobF& J, const SlotsDev& S, RareSm& sm, int t, int64_t slot, uint32_t pw) {
+__device__ __forceinline__ void unpair(const bool DBL, const JobF& J, const SlotsDev& S, RareSm& sm, int t, int64_t slot, uint32_t pw) {
     if (!(pw & P_CROSSED)) return;
     const int cell = sm.cell[t], sw = sm.sw[t];
     const int key = fkey(DBL, cell, sw & W_LB);
@@ -970,7 +893,7 @@ __device__ __forceinline__ void unpair(const JobF& J, const SlotsDev& S, RareSm&
 // A special step that is not a quick one: out of line, on the lane state in
 // shared memory, so that the hot loop's registers do not carry its working
 // set.  sm.left: 0 when the countdown ends at s.
-template <bool DBL, bool OVER>
+template <int K>
 __device__ __noinline__ void special_step(const JobF* jobs, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
                                           uint64_t s) {
     RareSm& sm = *smp;
@@ -981,35 +904,92 @@ __device__ __noinline__ void special_step(const JobF* jobs, const SlotsDev* Sp, 
         return;
     }
     const JobF& J = jobs[job];
-    unpair<DBL>(J, S, sm, t, slot, sm.pw[t]);
-    float xp = sm.xp[t], lo = sm.lo[t], hi = sm.hi[t], F = sm.F[t];
-    if (light_step<DBL>(J, S, sm, t, slot, sm.traj[t], s, sm.left[t] == 0, xp, lo, hi, F)) {
-        sm.xp[t] = xp;
-        sm.lo[t] = lo;
-        sm.hi[t] = hi;
-        sm.F[t] = F;
-    } else {
-        general_step<DBL, OVER>(jobs, Sp, smp, t, slot, s);
-        if (sm.job[t] < 0) return;
-        xp = sm.xp[t];
+    const bool DBL = is_double<K>(J), OVER = is_over<K>(J);
+    uint32_t pw = sm.pw[t];
+    unpair(DBL, J, S, sm, t, slot, pw);
+    if (pw & P_SWAP) {   // the lane's cell is its pair's first now
+        pw ^= P_RIGHT;
+        if (((pw & P_S0) != 0u) != ((pw & P_S1) != 0u)) pw ^= P_S0 | P_S1;
     }
-    settle<DBL>(J, sm, t, s, xp);
+    pw &= ~(P_SWAP | P_CROSSED);
+    const float xp = sm.xp[t], lo = sm.lo[t], hi = sm.hi[t];
+    if (sm.left[t] == 0 && xp > lo && xp < hi && only_flip(J, sm, t, s, pw)) {
+        float F;
+        int left;
+        flip_here(DBL, J, sm, t, s, xp, F, left, pw);
+        sm.F[t] = F;
+        sm.left[t] = left;
+        sm.pw[t] = pw;
+        return;
+    }
+    if ((pw & P_PAIR) && (pw & P_OVERDUE) && sm.left[t] != 0 &&
+        ((pw & P_RIGHT) ? xp >= J.halfL : xp < -J.halfL)) {
+        // The pair's edge crossed, the other cell's pending flip past: as a
+        // quick crossing, the barrier entered caught up from that flip.
+        const bool right = (pw & P_RIGHT) != 0u;
+        const float xn = right ? xp - J.L : xp + J.L;
+        const float e1 = right ? -J.halfL : J.edge_hi, e2 = right ? J.edge_lo : J.halfL;
+        if (xn > e1 && xn < e2) {
+            const int st = sm.state[t];
+            const uint32_t g = sm.traj[t] + J.g0;
+            long long nf;
+            const int now = caught_up(J, g, s, sm.cflip[t], (pw & P_S1) ? 0 : 1, philox_at(s, g, TAG_FLIP, J.key0, J.key1),
+                                      &nf);
+            pw = (pw | P_CROSSED | P_SWAP) & ~P_S1;
+            if (now) pw |= P_S1;
+            sm.cflip[t] = nf;
+            sm.xs[t] = (long long)s;
+            if (now != st) {
+                if (now) sm.since[t] = (long long)s;
+                else sm.sc1[t] += (long long)s - sm.since[t];
+            }
+            unpair(DBL, J, S, sm, t, slot, pw);   // into the cell entered
+            sm.xp[t] = xn;
+            sm.lo[t] = e1;
+            sm.hi[t] = e2;
+            sm.F[t] = 0.f;
+            settle(DBL, &J, &sm, t, s, xn);
+            return;
+        }
+    }
+    general_step(DBL, OVER, jobs, Sp, smp, t, slot, s);
+    if (sm.job[t] < 0) return;
+    settle(DBL, &J, &sm, t, s, sm.xp[t]);
 }
 
 // The quick steps: the commonest special steps, in the hot loop, with the
-// state a light step leaves (unpair fills in what a pair's crossings leave
+// state the general step leaves (unpair fills in what a pair's crossings leave
 // open).  Returns false when the step needs special_step.
 //  * A frame, the position inside its band.
 //  * A band change inside the cell (a flank entered or left) that changes
 //    neither the well nor the local barrier.
 //  * A crossing of the pair's edge into the flat band of the other cell: the
 //    barriers change places.
-template <bool DBL>
-__device__ __forceinline__ bool quick_step(const JobF& J, RareSm& sm, int t, uint64_t s, bool countdown, float& xp,
+__device__ __forceinline__ bool quick_step(const bool DBL, const bool flips, const JobF& J, RareSm& sm, int t,
+                                           uint64_t s, bool countdown, float& xp,
                                            float& lo, float& hi, float& F, int& left, uint32_t& pw) {
     const uint32_t swapped = pw & P_SWAP;
     if (countdown) {
-        if (!(pw & P_FRAME) || !(xp > lo && xp < hi)) return false;
+        if (!(xp > lo && xp < hi)) return false;
+        if (!(pw & P_FRAME)) {
+            if (flips && only_flip(J, sm, t, s, pw)) {
+                flip_here(DBL, J, sm, t, s, xp, F, left, pw);
+                return true;
+            }
+            // the other cell's pending flip, and nothing else: caught up with
+            // when the cell is entered
+            const bool other = (pw & (P_PAIR | P_OVERDUE)) == P_PAIR &&
+                               (swapped ? sm.nflip[t] : sm.cflip[t]) == (long long)s && s != J.nsteps;
+            const long long nxf = sm.nxf[t], own = swapped ? sm.cflip[t] : sm.nflip[t];
+            if (!other || (long long)s == nxf || (long long)s == own) return false;
+            long long nev = block_wrap(s - 1);
+            if (nev == (long long)s) return false;
+            nev = (long long)J.nsteps < nev ? (long long)J.nsteps : nev;
+            nev = own < nev ? own : nev;
+            pw |= P_OVERDUE;
+            count_down(J, sm, t, s, nev, left, pw);
+            return true;
+        }
         const int fidx = sm.fidx[t];
         int cell = sm.cell[t];
         if (swapped) cell += (pw & P_RIGHT) ? 1 : -1;
@@ -1039,15 +1019,15 @@ __device__ __forceinline__ bool quick_step(const JobF& J, RareSm& sm, int t, uin
             const float xc = J.xc;
             if ((xp < xc) != (lo < xc)) return false;   // lo < xc: local barrier 0
             float l2, h2;
-            band_of<DBL>(J, xp, &l2, &h2);
+            band_of(DBL, J, xp, &l2, &h2);
             if (!(xp > l2 && xp < h2)) return false;
             lo = l2;
             hi = h2;
-            F = force_of<DBL>(J, xp, st);
+            F = force_of(DBL, J, xp, st);
         }
         return true;
     }
-    if (!(pw & P_PAIR)) return false;
+    if ((pw & (P_PAIR | P_OVERDUE)) != P_PAIR) return false;
     const bool right = ((pw & P_RIGHT) != 0u) != (swapped != 0u);   // the pair's other cell is the right neighbour
     const float xn = right ? xp - J.L : xp + J.L;
     const float e1 = right ? -hL : J.edge_hi, e2 = right ? J.edge_lo : hL;
@@ -1066,8 +1046,7 @@ __device__ __forceinline__ bool quick_step(const JobF& J, RareSm& sm, int t, uin
 }
 
 // One step's move.
-template <bool OVER>
-__device__ __forceinline__ void f_move(float& xp, float& rv, float F, float c1, float c2, float c3, float nz) {
+__device__ __forceinline__ void f_move(const bool OVER, float& xp, float& rv, float F, float c1, float c2, float c3, float nz) {
     if (OVER) {
         xp = fmaf(F, c1, xp);
         xp = xp + nz;
@@ -1082,33 +1061,32 @@ __device__ __forceinline__ void f_move(float& xp, float& rv, float F, float c1, 
 }
 
 // One lane's steps 4j+1+h .. 4j+4 one by one, step 4j+1+h a special one that
-// is moved already; the block's noise is drawn again.  Out of line, on the
-// lane state in shared memory.
-template <bool DBL, bool OVER>
+// is moved already; the later steps' noise in sm.nz.  Out of line, on the lane
+// state in shared memory.
+template <int K>
 __device__ __noinline__ void slow_steps(const JobF* jobs, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
                                         uint64_t j, int h) {
     RareSm& sm = *smp;
-    const float kn = __uint_as_float(sm.fixk[t].y);
-    const Words w = philox_step((uint32_t)j, sm.fix[t], sm.fixk[t].x);
-    float n[4];
-    noise_pair(w.w0, w.w1, kn, &n[0], &n[1]);
-    noise_pair(w.w2, w.w3, kn, &n[2], &n[3]);
     int job = sm.job[t];
     bool moved = true;
+    float4 nz = sm.nz[t];
 #pragma unroll 1
     for (; h < 4; ++h) {
         const JobF& J = jobs[job < 0 ? 0 : job];
+        const bool OVER = is_over<K>(J);
         const float c1 = OVER ? J.c_drift : J.hdt_invM;
         if (!moved && job >= 0) {
             float xp = sm.xp[t], rv = sm.rv[t];
-            f_move<OVER>(xp, rv, sm.F[t], c1, J.hdt, J.expg, h == 1 ? n[1] : h == 2 ? n[2] : n[3]);
+            f_move(OVER, xp, rv, sm.F[t], c1, J.hdt, J.expg, nz.x);
+            nz.x = nz.y;
+            nz.y = nz.z;
             sm.xp[t] = xp;
             sm.rv[t] = rv;
             sm.left[t] -= 1;
         }
         const float xp = sm.xp[t];
         if (moved || !(xp > sm.lo[t] && xp < sm.hi[t]) || sm.left[t] == 0) {
-            special_step<DBL, OVER>(jobs, Sp, smp, t, slot, 4 * j + 1 + h);
+            special_step<K>(jobs, Sp, smp, t, slot, 4 * j + 1 + h);
             job = sm.job[t];
             if (job < 0) {
                 sm.rv[t] = 0.f;
@@ -1142,22 +1120,21 @@ namespace {
 
 // A lane's per-job constants, band, force and countdown from its position
 // (sm.xp) and statistics state; s: its next step.
-template <bool DBL>
-__device__ __forceinline__ void bind_lane(const JobF& J, RareSm& sm, int t, uint32_t traj, uint64_t s) {
+__device__ __forceinline__ void bind_lane(const bool DBL, const JobF& J, RareSm& sm, int t, uint32_t traj, uint64_t s) {
     sm.traj[t] = traj;
     sm.j[t] = (uint32_t)((s - 1) >> 2);
     bind_block(J, sm, t, s - 1);
     const float xp = sm.xp[t];
     float lo, hi;
-    band_of<DBL>(J, xp, &lo, &hi);
+    band_of(DBL, J, xp, &lo, &hi);
     sm.lo[t] = lo;
     sm.hi[t] = hi;
-    sm.F[t] = force_of<DBL>(J, xp, sm.state[t]);
-    settle<DBL>(J, sm, t, s - 1, xp);
+    sm.F[t] = force_of(DBL, J, xp, sm.state[t]);
+    settle(DBL, &J, &sm, t, s - 1, xp);
 }
 
 // The state a slot kept since the last launch, into sm.
-template <bool DBL>
+template <int K>
 __device__ __noinline__ void load_slot(const QueueDev* qp, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot) {
     const SlotsDev& S = *Sp;
     RareSm& sm = *smp;
@@ -1165,6 +1142,7 @@ __device__ __noinline__ void load_slot(const QueueDev* qp, const SlotsDev* Sp, R
     const int job = (slot < S.nslots) ? S.job[slot] : -1;
     if (job < 0) return;
     const JobF& J = qp->jobs[job];
+    const bool DBL = is_double<K>(J);
     const uint32_t traj = (uint32_t)S.traj[slot];
     const uint64_t s = (uint64_t)S.step[slot];
     sm.job[t] = job;
@@ -1190,11 +1168,11 @@ __device__ __noinline__ void load_slot(const QueueDev* qp, const SlotsDev* Sp, R
     sm.fidx[t] = S.fidx[slot];
     sm.nxf[t] = S.nxf[slot];
     sm.nflip[t] = S.nflip[slot];
-    bind_lane<DBL>(J, sm, t, traj, s);
+    bind_lane(DBL, J, sm, t, traj, s);
 }
 
 // A lane's state into its slot, until the next launch.
-template <bool DBL>
+template <int K>
 __device__ __noinline__ void save_slot(const QueueDev* qp, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot) {
     const SlotsDev& S = *Sp;
     RareSm& sm = *smp;
@@ -1203,8 +1181,9 @@ __device__ __noinline__ void save_slot(const QueueDev* qp, const SlotsDev* Sp, R
     S.job[slot] = job;
     if (job < 0) return;
     const JobF& J = qp->jobs[job];
+    const bool DBL = is_double<K>(J);
     const uint32_t traj = sm.traj[t];
-    unpair<DBL>(J, S, sm, t, slot, sm.pw[t]);
+    unpair(DBL, J, S, sm, t, slot, sm.pw[t]);
     S.traj[slot] = traj;
     S.step[slot] = (int64_t)(((uint64_t)sm.jh[t] << 34 | (uint64_t)sm.j[t] << 2) + 1);
     S.xp[slot] = sm.xp[t];
@@ -1261,7 +1240,7 @@ __device__ __forceinline__ int first_claim(unsigned long long avail, const Slots
 // first `most` lanes with `need` claim trajectories from the queue.  Returns
 // whether the warp is done claiming: the queue had fewer than the lanes
 // wanted, or lanes were left out.
-template <bool DBL, bool OVER>
+template <int K>
 __device__ __noinline__ bool refill(const QueueDev* qp, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
                                     bool need, int most) {
     const QueueDev& q = *qp;
@@ -1297,11 +1276,12 @@ __device__ __noinline__ bool refill(const QueueDev* qp, const SlotsDev* Sp, Rare
         const uint32_t traj = (uint32_t)f_resolve(q.range_end, q.range_job, q.range_first, q.nranges,
                                                   (int64_t)(base + rank), &job);
         const JobF* Jn = &q.jobs[job];
-        f_start<DBL, OVER>(Jn, S.ring, S.nslots, S.ring_slots, slot, traj, &sm, t);
+        const bool DBL = is_double<K>(*Jn), OVER = is_over<K>(*Jn);
+        f_start<K>(Jn, S.ring, S.nslots, S.ring_slots, slot, traj, &sm, t);
         sm.job[t] = job;
-        bind_lane<DBL>(*Jn, sm, t, traj, Jn->step0);
+        bind_lane(DBL, *Jn, sm, t, traj, Jn->step0);
         if (Jn->nsteps == 0) {
-            retire_lane<OVER>(*Jn, S.retired, sm, t, 0, sm.xp[t], sm.rv[t], 0);
+            retire_lane(OVER, *Jn, S.retired, sm, t, 0, sm.xp[t], sm.rv[t], 0);
             idle_lane(sm, t);
         }
     }
@@ -1313,8 +1293,9 @@ __device__ __noinline__ bool refill(const QueueDev* qp, const SlotsDev* Sp, Rare
 // Returns the blocks run, the last one unfinished for lanes with a step h
 // that needs the slow path (P_HALT + h in their P_* word).  A function
 // without calls, so that nothing in it is held for one.
-template <bool DBL, bool OVER>
+template <int K, bool kRoll>
 __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t, uint32_t most) {
+    constexpr bool DBL = (K & 2) != 0, OVER = (K & 1) != 0;
     RareSm& sm = *smp;
     const int job = sm.job[t];
     float xp = sm.xp[t], rv = sm.rv[t], F = sm.F[t], lo = sm.lo[t], hi = sm.hi[t];
@@ -1343,7 +1324,7 @@ __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t
         float xs[4];
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
-            f_move<OVER>(xp, rv, F, c1, c2, c3, nq[h]);
+            f_move(OVER, xp, rv, F, c1, c2, c3, nq[h]);
             xs[h] = xp;
             if (!OVER) rv = fmaf(F, c1, rv);
         }
@@ -1359,16 +1340,22 @@ __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t
                 rv = rv0;
                 left += 4;
                 const uint64_t s0 = (uint64_t)sm.jh[t] << 34 | (uint64_t)j << 2;
-#pragma unroll
+                float n0 = nq[0], n1 = nq[1], n2 = nq[2];
+                const float n3 = nq[3];
+#pragma unroll kRoll ? 1 : 4
                 for (int h = 0; h < 4; ++h) {
                     if (halt) continue;
-                    f_move<OVER>(xp, rv, F, c1, c2, c3, nq[h]);
+                    f_move(OVER, xp, rv, F, c1, c2, c3, n0);
+                    n0 = n1;
+                    n1 = n2;
+                    n2 = n3;
                     --left;
                     if (!(xp > lo) | !(xp < hi) | (left == 0)) {
-                        if (job < 0 || !quick_step<DBL>(jobs[job], sm, t, s0 + 1 + h, left == 0, xp, lo, hi, F, left,
-                                                        pw)) {
+                        if (job < 0 || !quick_step(DBL, kRoll, jobs[job], sm, t, s0 + 1 + h, left == 0, xp, lo, hi, F,
+                                                    left, pw)) {
                             halt = true;
                             pw |= P_HALT * (1 + h);
+                            sm.nz[t] = make_float4(n0, n1, n2, 0.f);
                             continue;
                         }
                     }
@@ -1397,15 +1384,17 @@ __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t
 // blocks of four steps.  Returns the blocks run; *drained is set when it
 // stopped early because every lane of the warp was idle and the queue had
 // nothing left for it.  Slot state is loaded at entry and saved at exit.
-template <bool DBL, bool OVER, bool kSpread>
+template <int K, bool kMixed>
 __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const SlotsDev& S, RareSm& sm,
                                                    uint32_t quad_budget, bool* drained) {
     const int t = threadIdx.x;
     const int64_t slot = (int64_t)blockIdx.x * blockDim.x + t;
-    load_slot<DBL>(&q, &S, &sm, t, slot);
+    // out-of-line parts of the model type, or of whichever type (kMixed)
+    constexpr int C = kMixed ? 4 : K;
+    load_slot<C>(&q, &S, &sm, t, slot);
 
     bool dry = false;   // the queue had nothing left for this warp
-    int most = kSpread ? first_claim(*q.avail, S) : 32;
+    int most = !kMixed ? first_claim(*q.avail, S) : 32;
     uint32_t it = 0;
     while (it < quad_budget) {
         // lanes become idle in the slow path only
@@ -1413,7 +1402,7 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
             const bool need = sm.job[t] < 0 && !dry && slot < S.nslots;
             const bool asked = __any_sync(kFull, need);
             if (asked) {
-                if (kSpread && most == 0) {
+                if (!kMixed && most == 0) {
                     // leave the items to the warps that take them now; items
                     // still there after that (warps that were to take them
                     // have trajectories already) are claimed
@@ -1421,7 +1410,7 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
                         __nanosleep(20000);
                     most = 32;
                 }
-                if (refill<DBL, OVER>(&q, &S, &sm, t, slot, need, most)) dry = true;
+                if (refill<C>(&q, &S, &sm, t, slot, need, most)) dry = true;
                 most = 32;
             }
             if (__all_sync(kFull, sm.job[t] < 0)) {
@@ -1433,18 +1422,27 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
                 continue;
             }
         }
-        it += run_blocks<DBL, OVER>(q.jobs, &sm, t, quad_budget - it);
+        // The unrolled loop is the faster one for the single barrier with rare
+        // flips (2 x 65536 x 48000, flip probability 1e-5 a step: 17.0 ms
+        // against 18.6 rolled; 2e-4: 22.0 against 20.1, 1e-3: 40 against 28:
+        // with the flips' code it no longer fits the instruction cache), the
+        // rolled one for the double barrier (1e-5: 21.2 against 21.7) and for
+        // warps of all types on one SM (mixed launches).
+        constexpr bool kOnlyRolled = kMixed || (K & 2) != 0;
+        const bool often = !kOnlyRolled && sm.job[t] >= 0 && q.jobs[sm.job[t]].flips_often != 0;
+        if (kOnlyRolled || __any_sync(kFull, often)) it += run_blocks<K, true>(q.jobs, &sm, t, quad_budget - it);
+        else it += run_blocks<K, kOnlyRolled>(q.jobs, &sm, t, quad_budget - it);
         const uint32_t halt = sm.pw[t] / P_HALT;
         if (__any_sync(kFull, halt != 0)) {
             if (halt) {
                 sm.pw[t] &= P_HALT - 1;
-                slow_steps<DBL, OVER>(q.jobs, &S, &sm, t, slot, (uint64_t)sm.jh[t] << 32 | sm.j[t], (int)halt - 1);
+                slow_steps<C>(q.jobs, &S, &sm, t, slot, (uint64_t)sm.jh[t] << 32 | sm.j[t], (int)halt - 1);
             }
             __syncwarp();
             sm.j[t] += 1;
         }
     }
-    save_slot<DBL>(&q, &S, &sm, t, slot);
+    save_slot<C>(&q, &S, &sm, t, slot);
     return it;
 }
 
@@ -1455,7 +1453,7 @@ __global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_persistent_kern
     extern __shared__ uint4 sm_raw[];
     RareSm& sm = *reinterpret_cast<RareSm*>(sm_raw);
     bool drained = false;
-    persistent_run<DBL, OVER, true>(q, S, sm, quad_budget, &drained);
+    persistent_run<(DBL ? 2 : 0) + (OVER ? 1 : 0), false>(q, S, sm, quad_budget, &drained);
 }
 
 // All four model types in one persistent launch (the serving loop's).  A
@@ -1513,10 +1511,10 @@ __global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_mixed_kernel(co
         bool drained = false;
         uint32_t used;
         switch (type) {
-            case 0: used = persistent_run<false, false, false>(m.q[0], m.S, sm, left, &drained); break;
-            case 1: used = persistent_run<false, true, false>(m.q[1], m.S, sm, left, &drained); break;
-            case 2: used = persistent_run<true, false, false>(m.q[2], m.S, sm, left, &drained); break;
-            default: used = persistent_run<true, true, false>(m.q[3], m.S, sm, left, &drained); break;
+            case 0: used = persistent_run<0, true>(m.q[0], m.S, sm, left, &drained); break;
+            case 1: used = persistent_run<1, true>(m.q[1], m.S, sm, left, &drained); break;
+            case 2: used = persistent_run<2, true>(m.q[2], m.S, sm, left, &drained); break;
+            default: used = persistent_run<3, true>(m.q[3], m.S, sm, left, &drained); break;
         }
         left -= (used < left) ? used : left;
         if (drained) {

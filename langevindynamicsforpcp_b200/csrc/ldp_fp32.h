@@ -32,6 +32,8 @@ enum : int32_t {
 // Per-job constants and output pointers (device resident, one per job).
 struct JobF {
     // model switches (jobs of one queue share dbl/over)
+    int32_t dbl, over;
+    int32_t flips_often, pad0;   // flips are frequent among the special steps (run_blocks)
     int32_t eta, eq, rs, rv, us, init_state, wt, fpt, tpt, cg, n_cg, write_x, at_bottom, fp_mode;
     int32_t lanes, nruns, slots_log2;
     int32_t evm;         // EV_* statistics switches of the event path
@@ -49,7 +51,7 @@ struct JobF {
     // The bands next to the cell edges, (-L/2, edge_lo) and (edge_hi, L/2),
     // and whether the force is zero in both (no barrier flank reaches the
     // cell edge): then a crossing of the cell edge lands in a known flat
-    // band (the hot loop's light step).
+    // band (the pairs of settle).
     float edge_lo, edge_hi;
     int32_t edge_flat, pad2;
     // FP64 constants (step 0, events, frames)

@@ -157,6 +157,8 @@ static void fill_jobf(const ldp_job* job, JobF* J) {
     const KConst& k = job->k;
     const TrajState& S = job->st;
     const int64_t n = job->ntraj;
+    J->dbl = k.dbl; J->over = k.over;
+    J->flips_often = k.eta && std::min(k.ln1m[0], k.ln1m[1]) < -1.5e-4;
     J->eta = k.eta; J->eq = k.eq; J->rs = k.rs; J->rv = k.rv; J->us = k.us; J->init_state = k.init_state;
     J->wt = k.wt; J->fpt = k.fpt; J->tpt = k.tpt; J->cg = k.cg; J->n_cg = k.n_cg; J->write_x = k.write_x;
     J->at_bottom = k.at_bottom; J->fp_mode = k.fp_mode; J->lanes = k.lanes; J->nruns = k.nruns;
