@@ -66,11 +66,13 @@ enum : uint32_t { B_HAS_FPT = 1u << 24, B_HAS_FPT2 = 1u << 25, B_HAS_TPT = 1u <<
 enum : int32_t { W_LB = 1, W_EVICT = 2, W_CVALID = 4, W_CSTATE = 8 };
 
 // Model type K: 0-3 (double * 2 + overdamped), or 4, the job's, for code
-// that serves all four.
+// that serves all four; plus K_WIDE in the wide kernels (their own copies of
+// the out-of-line parts, compiled for fewer registers).
+constexpr int K_ANY = 4, K_WIDE = 8;
 template <int K>
-__device__ __forceinline__ bool is_double(const JobF& J) { return K < 4 ? (K & 2) != 0 : J.dbl != 0; }
+__device__ __forceinline__ bool is_double(const JobF& J) { return (K & K_ANY) ? J.dbl != 0 : (K & 2) != 0; }
 template <int K>
-__device__ __forceinline__ bool is_over(const JobF& J) { return K < 4 ? (K & 1) != 0 : J.over != 0; }
+__device__ __forceinline__ bool is_over(const JobF& J) { return (K & K_ANY) ? J.over != 0 : (K & 1) != 0; }
 
 // The word of a lane's quick steps (see quick_step), kept in a register by
 // the hot loop: quick steps allowed (the barrier flanks do not reach the cell
@@ -101,10 +103,10 @@ struct RareSm {
     // Lane state the hot loop hands to the general step and takes back, and
     // the lane state only the general step uses.
     float xp[kMaxBlock], rv[kMaxBlock], F[kMaxBlock], lo[kMaxBlock], hi[kMaxBlock];
-    float4 nz[kMaxBlock];         // noise of a block's steps after one that needs the slow path
     uint4 fix[kMaxBlock];         // Philox constants of the lane's step blocks (philox_fix) ...
     uint2 fixk[kMaxBlock];        // ... the first key word of its third round, and the noise scale (float bits)
     uint32_t traj[kMaxBlock];
+    float nz[3][kMaxBlock];       // noise of a block's steps after one that needs the slow path
     long long nflip[kMaxBlock];   // step of the current barrier's next flip
     int32_t left[kMaxBlock], job[kMaxBlock], cell[kMaxBlock], state[kMaxBlock], sw[kMaxBlock];
     uint32_t pw[kMaxBlock];       // P_* word (quick steps)
@@ -112,7 +114,7 @@ struct RareSm {
     long long xs[kMaxBlock];      // step of the last quick crossing
     uint32_t j[kMaxBlock], jh[kMaxBlock];   // next block of four steps, 4j+1 .. 4j+4: j's low and high word
 };
-static_assert(sizeof(RareSm) <= 56 * 1024, "four blocks to an SM");
+static_assert(sizeof(RareSm) <= 55 * 1024, "four blocks to an SM");
 
 __device__ __forceinline__ void red_add(int64_t* p, int64_t v) {
     atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)v);
@@ -1069,7 +1071,7 @@ __device__ __noinline__ void slow_steps(const JobF* jobs, const SlotsDev* Sp, Ra
     RareSm& sm = *smp;
     int job = sm.job[t];
     bool moved = true;
-    float4 nz = sm.nz[t];
+    int next = 0;
 #pragma unroll 1
     for (; h < 4; ++h) {
         const JobF& J = jobs[job < 0 ? 0 : job];
@@ -1077,9 +1079,7 @@ __device__ __noinline__ void slow_steps(const JobF* jobs, const SlotsDev* Sp, Ra
         const float c1 = OVER ? J.c_drift : J.hdt_invM;
         if (!moved && job >= 0) {
             float xp = sm.xp[t], rv = sm.rv[t];
-            f_move(OVER, xp, rv, sm.F[t], c1, J.hdt, J.expg, nz.x);
-            nz.x = nz.y;
-            nz.y = nz.z;
+            f_move(OVER, xp, rv, sm.F[t], c1, J.hdt, J.expg, sm.nz[next++][t]);
             sm.xp[t] = xp;
             sm.rv[t] = rv;
             sm.left[t] -= 1;
@@ -1109,12 +1109,15 @@ __device__ __forceinline__ void range4(float a, float b, float c, float d, float
 
 }  // namespace
 
-#ifndef LDP_FP32_MIN_BLOCKS
-// Resident 256-thread blocks per SM the register budget is sized for: 3
-// gives the hot loop 80 registers without spills (measured faster than 4
-// blocks at 64 registers, which spill in the loop).
-#define LDP_FP32_MIN_BLOCKS 3
-#endif
+// Resident 256-thread blocks per SM the register budget is sized for.  Three
+// (80 registers) leave room on the SM for the finished jobs' mean-square
+// displacements and step their own lanes 3-4 % faster; four (64) hold 151552
+// trajectories instead of 113664 and hide more latency: 2 x 65536 x 48000 16.8
+// / 15.1 ms, 4 x 65536 x 120000 59.4 / 56.6, a graph of two times 80000 x 24000
+// 19.4 / 20.2, 20011 double 6.9 / 7.2.  So four where the trajectories of the
+// queue do not fit three blocks (Fp32Queue::wide).  (Four at 56 registers,
+// which leave that room too: 15.0, 56.4, 20.3, 7.8.)
+constexpr int kNarrowBlocks = 3, kWideBlocks = 4;
 
 namespace {
 
@@ -1355,7 +1358,9 @@ __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t
                                                     left, pw)) {
                             halt = true;
                             pw |= P_HALT * (1 + h);
-                            sm.nz[t] = make_float4(n0, n1, n2, 0.f);
+                            sm.nz[0][t] = n0;
+                            sm.nz[1][t] = n1;
+                            sm.nz[2][t] = n2;
                             continue;
                         }
                     }
@@ -1390,7 +1395,7 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
     const int t = threadIdx.x;
     const int64_t slot = (int64_t)blockIdx.x * blockDim.x + t;
     // out-of-line parts of the model type, or of whichever type (kMixed)
-    constexpr int C = kMixed ? 4 : K;
+    constexpr int C = kMixed ? K_ANY : K;
     load_slot<C>(&q, &S, &sm, t, slot);
 
     bool dry = false;   // the queue had nothing left for this warp
@@ -1446,14 +1451,13 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
     return it;
 }
 
-template <bool DBL, bool OVER>
-__global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_persistent_kernel(
-
+template <int K>
+__global__ void __launch_bounds__(256, (K & K_WIDE) ? kWideBlocks : kNarrowBlocks) fp32_persistent_kernel(
     const __grid_constant__ QueueDev q, const __grid_constant__ SlotsDev S, uint32_t quad_budget) {
     extern __shared__ uint4 sm_raw[];
     RareSm& sm = *reinterpret_cast<RareSm*>(sm_raw);
     bool drained = false;
-    persistent_run<(DBL ? 2 : 0) + (OVER ? 1 : 0), false>(q, S, sm, quad_budget, &drained);
+    persistent_run<K, false>(q, S, sm, quad_budget, &drained);
 }
 
 // All four model types in one persistent launch (the serving loop's).  A
@@ -1470,7 +1474,7 @@ __global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_persistent_kern
 // budget is spent, no queue has work, or eight type changes in a row found
 // nothing to claim (claims raced away by other warps).
 template <int kUnused>
-__global__ void __launch_bounds__(256, LDP_FP32_MIN_BLOCKS) fp32_mixed_kernel(const __grid_constant__ MixedDev m,
+__global__ void __launch_bounds__(256, kNarrowBlocks) fp32_mixed_kernel(const __grid_constant__ MixedDev m,
                                                                                uint32_t quad_budget) {
     extern __shared__ uint4 sm_raw[];
     RareSm& sm = *reinterpret_cast<RareSm*>(sm_raw);
@@ -1545,28 +1549,30 @@ int launch_fp32_publish(const QueueDev& q, unsigned long long new_tail, int32_t 
     return (int)cudaGetLastError();
 }
 
-template <bool DBL, bool OVER>
-static cudaError_t fp32_kernel_attrs() {
-    // The kernel reads little global memory: give shared memory the whole
-    // carveout so that the occupancy the grid is sized for is resident.
-    const cudaError_t e = cudaFuncSetAttribute(fp32_persistent_kernel<DBL, OVER>,
-                                               cudaFuncAttributePreferredSharedMemoryCarveout,
-                                               (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(fp32_persistent_kernel<DBL, OVER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(RareSm));
+using PersistentKernel = void (*)(QueueDev, SlotsDev, uint32_t);
+static PersistentKernel persistent_kernel(bool dbl, bool over, bool wide) {
+    switch ((wide ? 4 : 0) | (dbl ? 2 : 0) | (over ? 1 : 0)) {
+        case 0: return fp32_persistent_kernel<0>;
+        case 1: return fp32_persistent_kernel<1>;
+        case 2: return fp32_persistent_kernel<2>;
+        case 3: return fp32_persistent_kernel<3>;
+        case 4: return fp32_persistent_kernel<K_WIDE + 0>;
+        case 5: return fp32_persistent_kernel<K_WIDE + 1>;
+        case 6: return fp32_persistent_kernel<K_WIDE + 2>;
+        default: return fp32_persistent_kernel<K_WIDE + 3>;
+    }
 }
 
-int fp32_blocks_per_sm(bool dbl, bool over, int block) {
+int fp32_blocks_per_sm(bool dbl, bool over, bool wide, int block) {
+    const PersistentKernel kern = persistent_kernel(dbl, over, wide);
+    // The kernel reads little global memory: give shared memory the whole
+    // carveout so that the occupancy the grid is sized for is resident.
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         (int)cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RareSm));
     int n = 0;
-    cudaError_t e;
-    if (dbl) e = over ? fp32_kernel_attrs<true, true>() : fp32_kernel_attrs<true, false>();
-    else e = over ? fp32_kernel_attrs<false, true>() : fp32_kernel_attrs<false, false>();
-    if (e != cudaSuccess) return 0;
-    if (dbl) e = over ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<true, true>, block, sizeof(RareSm))
-                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<true, false>, block, sizeof(RareSm));
-    else e = over ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<false, true>, block, sizeof(RareSm))
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_persistent_kernel<false, false>, block, sizeof(RareSm));
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, sizeof(RareSm));
     return e == cudaSuccess ? n : 0;
 }
 
@@ -1587,18 +1593,11 @@ int launch_fp32_mixed(const MixedDev& m, uint32_t pair_budget, int grid, int blo
     return (int)cudaGetLastError();
 }
 
-int launch_fp32_persistent(bool dbl, bool over, const QueueDev& q, const SlotsDev& s, uint32_t pair_budget, int grid,
-                           int block, void* stream) {
-    cudaStream_t st = (cudaStream_t)stream;
+int launch_fp32_persistent(bool dbl, bool over, bool wide, const QueueDev& q, const SlotsDev& s, uint32_t pair_budget,
+                           int grid, int block, void* stream) {
     const uint32_t quad_budget = pair_budget > 1 ? pair_budget / 2 : 1;   // blocks of four steps
     if (block > kMaxBlock) return (int)cudaErrorInvalidValue;
-    if (dbl) {
-        if (over) fp32_persistent_kernel<true, true><<<grid, block, sizeof(RareSm), st>>>(q, s, quad_budget);
-        else fp32_persistent_kernel<true, false><<<grid, block, sizeof(RareSm), st>>>(q, s, quad_budget);
-    } else {
-        if (over) fp32_persistent_kernel<false, true><<<grid, block, sizeof(RareSm), st>>>(q, s, quad_budget);
-        else fp32_persistent_kernel<false, false><<<grid, block, sizeof(RareSm), st>>>(q, s, quad_budget);
-    }
+    persistent_kernel(dbl, over, wide)<<<grid, block, sizeof(RareSm), (cudaStream_t)stream>>>(q, s, quad_budget);
     return (int)cudaGetLastError();
 }
 

@@ -143,8 +143,8 @@ struct MixedDev {
 // Appends published work: clamps head to the old tail, sets tail and nranges.
 int launch_fp32_publish(const QueueDev& q, unsigned long long new_tail, int32_t new_nranges, void* stream);
 // Resident blocks per SM of the persistent kernel (0 on error).
-int fp32_blocks_per_sm(bool dbl, bool over, int block);
-int launch_fp32_persistent(bool dbl, bool over, const QueueDev& q, const SlotsDev& s, uint32_t pair_budget,
+int fp32_blocks_per_sm(bool dbl, bool over, bool wide, int block);
+int launch_fp32_persistent(bool dbl, bool over, bool wide, const QueueDev& q, const SlotsDev& s, uint32_t pair_budget,
                            int grid, int block, void* stream);
 // Resident 256-thread blocks per SM of the mixed kernel, and its launch.
 int fp32_mixed_blocks_per_sm(int block);

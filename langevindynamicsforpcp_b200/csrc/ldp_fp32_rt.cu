@@ -27,7 +27,15 @@ struct Fp32Queue {
     SlotsDev s{};
     void* qmem = nullptr;
     void* smem = nullptr;
-    int grid = 0, block = 256;
+    // Grid of the narrow kernels (three blocks to an SM) and of the wide ones
+    // (four; equal to it where the context asks for fewer).  Wide launches
+    // start where the trajectories of the unfinished jobs do not fit the
+    // narrow grid, each in its own lane, and go on until the queue has no
+    // unfinished job: until then slots past the narrow grid may hold some.
+    int grid = 0, wide_grid = 0, block = 256;
+    bool wide = false;
+    int cur_grid() const { return wide ? wide_grid : grid; }
+    int64_t lanes() const { return (int64_t)cur_grid() * block; }
     uint64_t pair_budget = 1 << 15;
     int64_t nranges = 0;
     unsigned long long tail = 0;
@@ -110,13 +118,16 @@ static int queue_init(ldp_ctx* ctx, Fp32Queue& Q, int type, int ring_slots) {
     if (Q.ready) return 0;
     Q.block = ctx->fp32_block ? ctx->fp32_block : 256;
     // A persistent grid never exceeds what is resident at once.
-    const int resident = fp32_blocks_per_sm(type >= 2, (type & 1) != 0, Q.block);
-    int bps = ctx->fp32_blocks_per_sm ? ctx->fp32_blocks_per_sm : resident;
-    if (resident > 0) bps = std::min(bps, resident);
-    bps = std::max(bps, 1);
-    Q.grid = ctx->sm_count * bps;
+    auto blocks = [&](bool wide) {
+        const int resident = fp32_blocks_per_sm(type >= 2, (type & 1) != 0, wide, Q.block);
+        int bps = ctx->fp32_blocks_per_sm ? ctx->fp32_blocks_per_sm : resident;
+        if (resident > 0) bps = std::min(bps, resident);
+        return std::max(bps, 1);
+    };
+    Q.grid = ctx->sm_count * blocks(false);
+    Q.wide_grid = std::max(Q.grid, ctx->sm_count * blocks(true));
     Q.pair_budget = ctx->fp32_pair_budget ? ctx->fp32_pair_budget : (1u << 15);
-    const int64_t nslots = (int64_t)Q.grid * Q.block;
+    const int64_t nslots = (int64_t)Q.wide_grid * Q.block;
     // queue + job table
     size_t qb = al256(sizeof(int64_t) * kFp32MaxRanges) * 2 + al256(sizeof(int32_t) * kFp32MaxRanges) +
                 al256(sizeof(unsigned long long) * 3) + al256(sizeof(int32_t)) + al256(sizeof(JobF) * kFp32MaxJobs) +
@@ -265,7 +276,7 @@ bool fp32_queue_quiet(ldp_ctx* ctx, int type) {
 int fp32_launch_type(ldp_ctx* ctx, int type, uint32_t pair_budget, cudaStream_t st) {
     Fp32Queue& Q = ctx->fp32->q[type];
     if (!Q.ready) return 0;
-    return launch_fp32_persistent(type >= 2, (type & 1) != 0, Q.q, Q.s, pair_budget, Q.grid, Q.block, st);
+    return launch_fp32_persistent(type >= 2, (type & 1) != 0, Q.wide, Q.q, Q.s, pair_budget, Q.cur_grid(), Q.block, st);
 }
 
 // One persistent launch over all four model types' queues (serving): the
@@ -320,7 +331,7 @@ int fp32_copy_remaining(ldp_ctx* ctx, int type, unsigned long long* host, unsign
 // Slots of a queue's persistent grid and items published so far (serving).
 int64_t fp32_nslots(ldp_ctx* ctx, int type) {
     const Fp32Queue& Q = ctx->fp32->q[type];
-    return Q.ready ? Q.s.nslots : 0;
+    return Q.ready ? (int64_t)Q.grid * Q.block : 0;
 }
 unsigned long long fp32_published(ldp_ctx* ctx, int type) {
     const Fp32Queue& Q = ctx->fp32->q[type];
@@ -343,6 +354,11 @@ int fp32_register(ldp_job* job, cudaStream_t stream, bool publish) {
     int e = queue_init(ctx, Q, type, ctx->fp32_ring_slots ? ctx->fp32_ring_slots : 64);
     if (e) return e;
     if (Q.free_slots.empty()) return (int)cudaErrorMemoryAllocation;
+    if (fp32_queue_quiet(ctx, type)) Q.wide = false;
+    int64_t items = job->ntraj;
+    for (const ldp_job* j : Q.table)
+        if (j && !j->done) items += j->ntraj;
+    if (items > (int64_t)Q.grid * Q.block) Q.wide = Q.wide_grid > Q.grid;
     const int slot = Q.free_slots.back();
     Q.free_slots.pop_back();
     Q.table[slot] = job;
@@ -398,7 +414,7 @@ int fp32_pump(ldp_job* job, int nlaunch) {
     const bool dbl = job->k.dbl, over = job->k.over;
     for (int i = 0; i < nlaunch; ++i) {
         const uint32_t pb = (uint32_t)std::min<uint64_t>(Q.pair_budget, 0xffffffffull);
-        int e = launch_fp32_persistent(dbl, over, Q.q, Q.s, pb, Q.grid, Q.block, ctx->stream);
+        int e = launch_fp32_persistent(dbl, over, Q.wide, Q.q, Q.s, pb, Q.cur_grid(), Q.block, ctx->stream);
         if (e) return e;
         ++job->launches;
     }
@@ -409,7 +425,7 @@ int fp32_pump(ldp_job* job, int nlaunch) {
 int fp32_estimate_launches(const ldp_job* job) {
     const Fp32Queue& Q = job->ctx->fp32->q[job->fp32_type];
     const double pairs = (double)job->ntraj * (double)((job->nsteps + 1) / 2);
-    const double cap = (double)Q.s.nslots * (double)Q.pair_budget;
+    const double cap = (double)Q.lanes() * (double)Q.pair_budget;
     // A trajectory's steps run in order in one slot: at least its own length
     // in launches, however many slots are free.
     const double serial = (double)((job->nsteps + 1) / 2) / (double)Q.pair_budget;
@@ -424,7 +440,7 @@ int fp32_estimate_launches(const ldp_job* job) {
 int fp32_launch_bound(ldp_ctx* ctx, int type, double total_pairs, double max_pairs) {
     const Fp32Queue& Q = ctx->fp32->q[type];
     const double pb = (double)std::min<uint64_t>(Q.pair_budget, 0xffffffffull);
-    const double n = std::ceil(total_pairs / ((double)Q.s.nslots * pb)) + std::ceil(max_pairs / pb) + 1.0;
+    const double n = std::ceil(total_pairs / ((double)Q.lanes() * pb)) + std::ceil(max_pairs / pb) + 1.0;
     return (int)std::min(n, 1.0e6);
 }
 

@@ -988,7 +988,8 @@ extern "C" ldp_status ldp_submit_batch(ldp_ctx* ctx, ldp_job** jobs, int njobs) 
     // jobs published so far (fp32_launch_bound of the prefix) holds per
     // job.  The post-processing then runs on a side stream beside the
     // later jobs' launches, in the registers and shared memory three
-    // persistent blocks leave on an SM.
+    // persistent blocks leave on an SM (four leave none: then between the
+    // launches, as blocks end).
     bool early[4];
     for (int t = 0; t < 4; ++t) early[t] = fp32_queue_quiet(ctx, t);
     for (int i = 0; i < njobs; ++i)   // first-passage jobs: no tight bound
@@ -1013,8 +1014,14 @@ extern "C" ldp_status ldp_submit_batch(ldp_ctx* ctx, ldp_job** jobs, int njobs) 
         job->submitted = true;
         CUDA_OR_FAIL(ctx, cudaEventRecord(job->ev[0], s));
         const int t = job->fp32_type;
-        launches[t] += fp32_estimate_launches(job);
         if (!first[t]) first[t] = job;
+    }
+    // All registered: the queues' launch shapes stand.
+    for (int i = 0; i < njobs; ++i) {
+        ldp_job* job = jobs[i];
+        if (job->o.precision != LDP_PREC_FP32_BATCHED) continue;
+        const int t = job->fp32_type;
+        launches[t] += fp32_estimate_launches(job);
         if (early[t]) {
             const double pairs = (double)((job->nsteps + 1) / 2);
             prefix[t] += pairs * (double)job->ntraj;
@@ -1097,6 +1104,10 @@ extern "C" ldp_status ldp_submit_batch_graph(ldp_ctx* ctx, ldp_job** jobs, int n
             return LDP_ERR_DEVICE;
         }
         job->submitted = true;
+    }
+    // All registered: the queues' launch shapes stand.
+    for (int i = 0; i < njobs; ++i) {
+        ldp_job* job = jobs[i];
         const int t = job->fp32_type;
         const double pairs = (double)((job->nsteps + 1) / 2);
         total[t] += pairs * (double)job->ntraj;

@@ -133,3 +133,34 @@ def test_every_job_size_is_claimed():
                 for k in keys:
                     np.testing.assert_array_equal(r[k], whole[k][..., :n], err_msg=f"{n} {k}")
                 a.wait()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_launches_of_four_blocks_to_an_sm(graph):
+    """Jobs that outgrow three resident blocks to an SM together get launches
+    of four: the same results as three blocks', also when trajectories are in
+    the slots already, and the queue is back at three afterwards."""
+    def outcome(blocks):
+        with ldp.Context(0) as c:
+            _tune.set_fp32_shape(c, blocks_per_sm=blocks, pair_budget=2500)
+            jobs = [ldp.Job(c, params("single_over", 24_000, freq_save=20, tau=1e-3), lanes=n,
+                            precision=ldp.PREC_FP32_BATCHED, job_id=i) for i, n in enumerate((lanes, 2000, 40, 9))]
+            if graph:
+                ldp.submit_batch(c, jobs[:3], graph=True)
+            else:
+                for j in jobs[:3]:
+                    j.submit()
+            for j in jobs[:3]:
+                j.wait()
+            jobs[3].run()
+            out = [j.results(frames=False) for j in jobs]
+            for j in jobs:
+                j.close()
+            return out, _tune.get_fp32_shape(c)["grid"]
+
+    lanes = 113_000                  # with 2000 more, past 3 x 256 x 148
+    three, grid = outcome(3)
+    assert lanes < grid * 256 < lanes + 2000
+    for a, b in zip(three, outcome(0)[0]):
+        for k in a:
+            np.testing.assert_array_equal(a[k], b[k], err_msg=k)
