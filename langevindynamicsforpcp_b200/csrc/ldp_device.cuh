@@ -66,67 +66,89 @@ constexpr double kLn2Lo = 2.31904681384629955842e-17;    // ln 2 - kLn2Hi
 constexpr double kTwoPiHi = 6.28318530717958623200e+00;  // nearest double to 2 pi
 constexpr double kTwoPiLo = 2.44929359829470635445e-16;  // 2 pi - kTwoPiHi
 
-// log(u) for positive normal u: u = m 2^e with m in [sqrt(1/2), sqrt(2)),
+// Whole numbers become doubles, and doubles whole numbers, by an addition of a
+// constant whose unit in the last place is the wanted one: exact, as every
+// sum here is representable, and one FP64 addition where the conversion
+// instructions of another pipe took one and two more operations.
+
+// log(u) for positive normal u, N at once (each constant, two moves, is then
+// set up once for N): u = m 2^e with m in [sqrt(1/2), sqrt(2)),
 // log m = 2 atanh((m-1)/(m+1)) by the odd power series of atanh.
+template <int N>
+__device__ __forceinline__ void log_f64(const double (&u)[N], double (&out)[N]) {
+    double f[N], f2[N], de[N], s[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const uint32_t hi = (uint32_t)__double2hiint(u[j]), lo = (uint32_t)__double2loint(u[j]), mh = hi & 0xfffffu;
+        const bool up = mh > 0x6a09eu || (mh == 0x6a09eu && lo > 0x667f3bcdu);   // above sqrt(2)
+        const double m = __hiloint2double((int)(mh | (up ? 0x3fe00000u : 0x3ff00000u)), (int)lo);
+        de[j] = __hiloint2double(0x43300000, (int)((hi >> 20) + (up ? 1u : 0u))) - (0x1p52 + 1023.0);   // e
+        f[j] = (m - 1.0) / (m + 1.0);
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        f2[j] = f[j] * f[j];
+        s[j] = 1.0 / 23.0;
+    }
+    constexpr double c[] = {1.0 / 21.0, 1.0 / 19.0, 1.0 / 17.0, 1.0 / 15.0, 1.0 / 13.0,
+                            1.0 / 11.0, 1.0 / 9.0,  1.0 / 7.0,  1.0 / 5.0,  1.0 / 3.0};
+#pragma unroll
+    for (int i = 0; i < 10; ++i)
+#pragma unroll
+        for (int j = 0; j < N; ++j) s[j] = fma(s[j], f2[j], c[i]);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const double logm = fma(2.0 * f[j] * f2[j], s[j], 2.0 * f[j]);
+        out[j] = fma(de[j], kLn2Hi, fma(de[j], kLn2Lo, logm));
+    }
+}
 __device__ __forceinline__ double log_f64(double u) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(u);
-    long long e = (long long)((b >> 52) & 0x7ff) - 1023;
-    double m = __longlong_as_double((long long)((b & 0x000fffffffffffffull) | 0x3ff0000000000000ull));
-    if (m > 1.41421356237309504880) { m = m * 0.5; e += 1; }
-    const double f = (m - 1.0) / (m + 1.0);
-    const double f2 = f * f;
-    double s = 1.0 / 23.0;
-    s = fma(s, f2, 1.0 / 21.0);
-    s = fma(s, f2, 1.0 / 19.0);
-    s = fma(s, f2, 1.0 / 17.0);
-    s = fma(s, f2, 1.0 / 15.0);
-    s = fma(s, f2, 1.0 / 13.0);
-    s = fma(s, f2, 1.0 / 11.0);
-    s = fma(s, f2, 1.0 / 9.0);
-    s = fma(s, f2, 1.0 / 7.0);
-    s = fma(s, f2, 1.0 / 5.0);
-    s = fma(s, f2, 1.0 / 3.0);
-    const double logm = fma(2.0 * f * f2, s, 2.0 * f);
-    const double de = (double)e;
-    return fma(de, kLn2Hi, fma(de, kLn2Lo, logm));
+    const double a[1] = {u};
+    double r[1];
+    log_f64(a, r);
+    return r[0];
 }
 
-// sin(2 pi t), cos(2 pi t), t in [0, 1): quadrant from rint(4t), Taylor
-// series of sin and cos on [-pi/4, pi/4].
-__device__ __forceinline__ void sincos2pi_f64(double t, double* sn, double* cs) {
-    const double q = rint(t * 4.0);
-    const double f = t - q * 0.25;
-    const double x = fma(f, kTwoPiHi, f * kTwoPiLo);
-    const double x2 = x * x;
-    double ps = -1.0 / 121645100408832000.0;
-    ps = fma(ps, x2, 1.0 / 355687428096000.0);
-    ps = fma(ps, x2, -1.0 / 1307674368000.0);
-    ps = fma(ps, x2, 1.0 / 6227020800.0);
-    ps = fma(ps, x2, -1.0 / 39916800.0);
-    ps = fma(ps, x2, 1.0 / 362880.0);
-    ps = fma(ps, x2, -1.0 / 5040.0);
-    ps = fma(ps, x2, 1.0 / 120.0);
-    ps = fma(ps, x2, -1.0 / 6.0);
-    const double s = fma(x * x2, ps, x);
-    double pc = 1.0 / 2432902008176640000.0;
-    pc = fma(pc, x2, -1.0 / 6402373705728000.0);
-    pc = fma(pc, x2, 1.0 / 20922789888000.0);
-    pc = fma(pc, x2, -1.0 / 87178291200.0);
-    pc = fma(pc, x2, 1.0 / 479001600.0);
-    pc = fma(pc, x2, -1.0 / 3628800.0);
-    pc = fma(pc, x2, 1.0 / 40320.0);
-    pc = fma(pc, x2, -1.0 / 720.0);
-    pc = fma(pc, x2, 1.0 / 24.0);
-    pc = fma(pc, x2, -0.5);
-    const double c = fma(x2, pc, 1.0);
-    const int qi = ((int)q) & 3;
-    double so, co;
-    if (qi == 0) { so = s; co = c; }
-    else if (qi == 1) { so = c; co = -s; }
-    else if (qi == 2) { so = -s; co = -c; }
-    else { so = -c; co = s; }
-    *sn = so;
-    *cs = co;
+// sin(2 pi t), cos(2 pi t), t in [0, 1), N at once: quadrant from t rounded
+// to quarters, Taylor series of sin and cos on [-pi/4, pi/4].
+template <int N>
+__device__ __forceinline__ void sincos2pi_f64(const double (&t)[N], double (&sn)[N], double (&cs)[N]) {
+    constexpr double kQuarters = 0x1.8p50;   // unit in the last place: 1/4
+    double x[N], x2[N], ps[N], pc[N];
+    uint32_t qi[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const double q = t[j] + kQuarters;
+        const double f = t[j] - (q - kQuarters);
+        qi[j] = (uint32_t)__double2loint(q);
+        x[j] = fma(f, kTwoPiHi, f * kTwoPiLo);
+        x2[j] = x[j] * x[j];
+        ps[j] = -1.0 / 121645100408832000.0;
+        pc[j] = 1.0 / 2432902008176640000.0;
+    }
+    constexpr double cp[] = {1.0 / 355687428096000.0, -1.0 / 1307674368000.0, 1.0 / 6227020800.0,
+                             -1.0 / 39916800.0,       1.0 / 362880.0,         -1.0 / 5040.0,
+                             1.0 / 120.0,             -1.0 / 6.0};
+    constexpr double cc[] = {-1.0 / 6402373705728000.0, 1.0 / 20922789888000.0, -1.0 / 87178291200.0,
+                             1.0 / 479001600.0,         -1.0 / 3628800.0,       1.0 / 40320.0,
+                             -1.0 / 720.0,              1.0 / 24.0,             -0.5};
+#pragma unroll
+    for (int i = 0; i < 9; ++i)
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            if (i < 8) ps[j] = fma(ps[j], x2[j], cp[i]);
+            pc[j] = fma(pc[j], x2[j], cc[i]);
+        }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const double s = fma(x[j] * x2[j], ps[j], x[j]);
+        const double c = fma(x2[j], pc[j], 1.0);
+        // quadrants 1 and 3 swap them; the sine is negative in 2 and 3, the
+        // cosine in 1 and 2
+        const double a = (qi[j] & 1u) ? c : s, b = (qi[j] & 1u) ? s : c;
+        sn[j] = __hiloint2double(__double2hiint(a) ^ (int)((qi[j] & 2u) << 30), __double2loint(a));
+        cs[j] = __hiloint2double(__double2hiint(b) ^ (int)(((qi[j] + 1u) & 2u) << 30), __double2loint(b));
+    }
 }
 
 // expm1(x), x <= 0: Cody-Waite reduction x = k ln2 + r, Taylor series for
@@ -181,15 +203,37 @@ __device__ __forceinline__ uint64_t prob_to_u64(double p) {
     return (uint64_t)ldexp(p, 64);
 }
 
-// Box-Muller pair from two 32-bit words, FP64.
+// N Box-Muller pairs from two 32-bit words each, FP64.
+template <int N>
+__device__ __forceinline__ void gauss_pairs_f64(const uint32_t (&wa)[N], const uint32_t (&wb)[N], double* z) {
+    double u1[N], u2[N], lg[N], sn[N], cs[N], r[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        // (wa + 1) / 2^32 and wb / 2^32: the words as the low bits of 2^20 + w / 2^32
+        u1[j] = __hiloint2double(0x41300000, (int)wa[j]) - (0x1p20 - 0x1p-32);
+        u2[j] = __hiloint2double(0x41300000, (int)wb[j]) - 0x1p20;
+    }
+    log_f64(u1, lg);
+#pragma unroll
+    for (int j = 0; j < N; ++j) r[j] = sqrt(-2.0 * lg[j]);
+    sincos2pi_f64(u2, sn, cs);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        z[2 * j] = r[j] * cs[j];
+        z[2 * j + 1] = r[j] * sn[j];
+    }
+}
 __device__ __forceinline__ void gauss_pair_f64(uint32_t wa, uint32_t wb, double* z0, double* z1) {
-    const double u1 = ((double)wa + 1.0) * 0x1p-32;
-    const double u2 = (double)wb * 0x1p-32;
-    const double r = sqrt(-2.0 * log_f64(u1));
-    double sn, cs;
-    sincos2pi_f64(u2, &sn, &cs);
-    *z0 = r * cs;
-    *z1 = r * sn;
+    const uint32_t a[1] = {wa}, b[1] = {wb};
+    double z[2];
+    gauss_pairs_f64(a, b, z);
+    *z0 = z[0];
+    *z1 = z[1];
+}
+// The four normals of a Philox block.
+__device__ __forceinline__ void gauss_block_f64(const Words& w, double* z) {
+    const uint32_t a[2] = {w.w0, w.w2}, b[2] = {w.w1, w.w3};
+    gauss_pairs_f64(a, b, z);
 }
 
 // Box-Muller pair from the same two words on the FP32 special-function units.

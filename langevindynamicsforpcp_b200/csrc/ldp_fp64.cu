@@ -827,8 +827,7 @@ __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, cons
     while (s < s_end && __any_sync(0xffffffffu, (a.q & Q_RUN) != 0u)) {
         const Words w = philox_at((s - 1) >> 2, g, TAG_STEP, k.key0, k.key1);
         double rf[4];
-        gauss_pair_f64(w.w0, w.w1, &rf[0], &rf[1]);
-        gauss_pair_f64(w.w2, w.w3, &rf[2], &rf[3]);
+        gauss_block_f64(w, rf);
 #pragma unroll
         for (int m = 0; m < 4; ++m) rf[m] = sig * rf[m];
         const int m0 = (int)((s - 1) & 3), m1 = s_end - s < (uint64_t)(4 - m0) ? m0 + (int)(s_end - s) : 4;
@@ -1003,14 +1002,11 @@ __global__ void __launch_bounds__(32 * (kGrpConsumers + kGrpProducers), 1) fp64_
                 const uint64_t q = a0 + b * (uint64_t)(B >> 2) + (uint64_t)quad;
                 if (i0 + tr >= st.n || 4 * q + 1 >= s_end) continue;
                 const Words w = philox_at(q, (uint32_t)(g0 + i0 + tr), TAG_STEP, k.key0, k.key1);
-                double z0, z1, z2, z3;
-                gauss_pair_f64(w.w0, w.w1, &z0, &z1);
-                gauss_pair_f64(w.w2, w.w3, &z2, &z3);
+                double n[4];
+                gauss_block_f64(w, n);
                 double* o = z + tr * R + quad * 4;
-                o[0] = sig * z0;
-                o[1] = sig * z1;
-                o[2] = sig * z2;
-                o[3] = sig * z3;
+#pragma unroll
+                for (int m = 0; m < 4; ++m) o[m] = sig * n[m];
             }
             if (DENSE) {
                 uint32_t* wt = waits + u * R * M;
