@@ -965,6 +965,14 @@ extern "C" ldp_status ldp_submit_batch(ldp_ctx* ctx, ldp_job** jobs, int njobs) 
             }
             CUDA_OR_FAIL(ctx, cudaEventCreateWithFlags(&ctx->f64fork, cudaEventDisableTiming));
         }
+        // The jobs' memory is allocated and cleared on the context's stream:
+        // before the fork, or the clearing could still run beside a job's
+        // first kernels.
+        for (int i = 0; i < njobs; ++i)
+            if (jobs[i]->o.precision != LDP_PREC_FP32_BATCHED && !jobs[i]->arena && job_arena(jobs[i], true) == 0) {
+                ldp_set_error(ctx, "cudaMalloc of %zu bytes failed", job_arena(jobs[i], false));
+                return LDP_ERR_NOMEM;
+            }
         CUDA_OR_FAIL(ctx, cudaEventRecord(ctx->f64fork, s));
         for (int k = 0; k < kCtxF64Streams; ++k) CUDA_OR_FAIL(ctx, cudaStreamWaitEvent(ctx->f64s[k], ctx->f64fork, 0));
         int k = 0;
