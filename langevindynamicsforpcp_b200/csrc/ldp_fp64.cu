@@ -807,68 +807,6 @@ __device__ __forceinline__ bool quiet_moves(const KConst& k, Lane& a, bool want,
     return want;
 }
 
-// Steps s_begin .. s_end-1, one trajectory per thread, each drawing its own
-// noise: one Philox block and two Box-Muller pairs for four steps.
-template <bool DBL, bool OVER, bool ETA>
-__global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, const TrajState st, int64_t g0,
-                                                         uint64_t s_begin, uint64_t s_end) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t g = (uint32_t)(g0 + i);
-    Lane a;
-    load_lane<DBL, OVER>(k, st, i, i < st.n, a);
-    const bool active = (a.q & Q_RUN) != 0u;
-    const uint64_t fs = k.freq_save;
-    uint64_t s = s_begin, s_done = s_end;   // s_done: this lane's first step not integrated
-    // next frame step (a multiple of FREQSAVE), so that no step divides
-    int64_t frame = (int64_t)((s_begin + fs - 1) / fs);
-    uint64_t nxf = k.fp_mode ? ~0ull : (uint64_t)frame * fs;
-    const double sig = OVER ? k.sig_r : k.sig_v;
-    const FlipDraw src;
-    while (s < s_end && __any_sync(0xffffffffu, (a.q & Q_RUN) != 0u)) {
-        const Words w = philox_at((s - 1) >> 2, g, TAG_STEP, k.key0, k.key1);
-        double rf[4];
-        gauss_block_f64(w, rf);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) rf[m] = sig * rf[m];
-        const int m0 = (int)((s - 1) & 3), m1 = s_end - s < (uint64_t)(4 - m0) ? m0 + (int)(s_end - s) : 4;
-        bool stands = false;
-        if (m0 == 0 && m1 == 4 && nxf >= s + 3)
-            stands = quiet_moves<OVER, false, 4>(k, a, !ETA || a.nflip >= (int64_t)s + 4, rf);
-        if (__any_sync(0xffffffffu, !stands)) {
-#pragma unroll 1
-            for (int m = m0; m < m1; ++m) {
-                const uint64_t sm = s + (uint64_t)(m - m0);
-                const double z = m == 0 ? rf[0] : m == 1 ? rf[1] : m == 2 ? rf[2] : rf[3];
-                if (!stands && (a.q & Q_RUN)) {
-                    fp64_move<OVER>(k, a.t, z);
-                    const bool off = !(off_band(a, a.t.x) < a.half);
-                    if (off || (ETA && (int64_t)sm == a.nflip)) {
-                        special_step<DBL, OVER, ETA>(k, st, i, g, a, sm, off, src);
-                        if (!(a.q & Q_RUN)) s_done = sm + ((a.flags & LDP_FLAG_NONFINITE) ? 0 : 1);
-                    } else {
-                        a.sc1 += a.t.state;
-                        if (!OVER) a.t.v = a.t.v + (k.invM * a.t.F) * k.hdt;
-                    }
-                }
-                __syncwarp();
-                if (nxf == sm && m + 1 < m1) {
-                    // (a frame after the block's last step is saved below)
-                    if (a.q & Q_RUN) save_frame<DBL>(k, st, i, a, frame);
-                    nxf += fs;
-                    ++frame;
-                }
-            }
-        }
-        s += (uint64_t)(m1 - m0);
-        if (nxf == s - 1) {
-            if (a.q & Q_RUN) save_frame<DBL>(k, st, i, a, frame);
-            nxf += fs;
-            ++frame;
-        }
-    }
-    if (active) store_lane(k, st, i, a, s_done, s_begin, s_end);
-}
-
 // ---------------------------------------------------------------------------
 // Group mode
 //
@@ -975,12 +913,176 @@ __device__ __forceinline__ bool dense_block(const KConst& k, Lane& a, bool want,
     return true;
 }
 
+// Where a lane's run of steps stands besides its Lane: the next frame and its
+// place, and the first step not integrated.
+struct Course {
+    int64_t frame;
+    double* px;
+    uint64_t s_done;
+    int every;   // steps between frames, 2^30 at most
+};
+
+__device__ __forceinline__ Course course(const KConst& k, const TrajState& st, int64_t i, uint64_t s_begin,
+                                         uint64_t s_end) {
+    const uint64_t fs = k.freq_save;
+    Course c;
+    c.frame = (int64_t)((s_begin + fs - 1) / fs);
+    c.px = st.fx ? st.fx + c.frame * st.n + i : nullptr;
+    c.s_done = s_end;
+    c.every = fs < (1u << 30) ? (int)fs : 1 << 30;
+    return c;
+}
+
+// Steps s0 + l .. s0 + n - 1 of a warp's lanes, their noise in z[l ..] (DENSE:
+// the waits of their flips in wt), in blocks of N.
+template <bool DBL, bool OVER, bool ETA, bool DENSE, int N>
+__device__ __forceinline__ void take_steps(const KConst& k, const TrajState& st, int64_t i, uint32_t g, Lane& a,
+                                           Course& c, uint64_t s0, int l, const int n, const double* z,
+                                           const uint32_t* wt) {
+    auto near = [](int64_t d) { return d < (1 << 30) ? (int)d : 1 << 30; };
+    // Steps s0 + l, l < n; each lane at its own l: a lane goes on from a
+    // special step with a new block, and its warp waits for it at the
+    // buffer's end only.
+    if (!(a.q & Q_RUN)) l = n;
+    // the places of the next frame and of the pending flip, and the last
+    // place a block can start at
+    int fr = k.fp_mode ? 1 << 30 : near(c.frame * (int64_t)k.freq_save - (int64_t)s0);
+    int flip = near(a.nflip - (int64_t)s0);
+    auto save = [&]() {
+        if (c.frame < k.nframe) {
+            if (k.write_x) save_frame<DBL>(k, st, i, a, c.frame);
+            else if (c.px) *c.px = a.t.x;
+        }
+        c.px += st.n;
+        ++c.frame;
+        fr = min(fr + c.every, 1 << 30);
+    };
+    auto last_start = [&]() { return min(min(n, fr + 1), ETA && !DENSE ? flip : n) - N; };
+    int lim = last_start();
+    while (__any_sync(0xffffffffu, l < n)) {
+        bool failed = false;
+        if (!__any_sync(0xffffffffu, l < n && l > lim)) {
+            // blocks, until a lane cannot go on with one
+            const bool flat = OVER && !DENSE && !__any_sync(0xffffffffu, (a.q & Q_FORCE) != 0u);
+            bool on, stop;
+#pragma unroll 1
+            do {
+                on = l <= lim;
+                const int lc = on ? l : 0;
+                double rf[N];
+#pragma unroll
+                for (int m = 0; m < N; ++m) rf[m] = z[lc + m];
+                bool stands;
+                if (DENSE) {
+                    uint32_t w[N];
+#pragma unroll
+                    for (int m = 0; m < N; ++m) w[m] = wt[lc + m];
+                    stands = dense_block<OVER, N>(k, a, on, flip, lc, rf, w);
+                } else if (flat) {
+                    stands = quiet_moves<OVER, true, N>(k, a, on, rf);
+                } else {
+                    stands = quiet_moves<OVER, false, N>(k, a, on, rf);
+                }
+                l += stands ? N : 0;
+                failed = on && !stands;
+                stop = on && (failed || l > lim);
+            } while (!__any_sync(0xffffffffu, stop));
+        }
+        if (l < n && (failed || l > lim)) {
+            if (l != fr + 1) {
+                // one by one, to the first special step and over it, or
+                // to the next place where blocks can go on
+                const int end = min(failed ? l + N : n, fr + 1);
+                int n1 = 0;
+                bool off;
+                do {
+                    fp64_move<OVER>(k, a.t, z[l]);
+                    off = !(off_band(a, a.t.x) < a.half);
+                    if (off || (ETA && !DENSE && l == flip)) break;
+                    if (DENSE && l == flip) {
+                        a.t.state ^= 1;
+                        flip = l + (int)__byte_perm(wt[l], 0, a.t.state ? 0x4432 : 0x4410);
+                        a.t.F = a.t.state ? a.bF1 : a.bF0;
+                    }
+                    n1 += a.t.state;
+                    if (!OVER) a.t.v = a.t.v + (k.invM * a.t.F) * k.hdt;
+                } while (++l < end);
+                a.sc1 += n1;
+                if (l < end) {
+                    if (DENSE) {
+                        a.nflip = (int64_t)s0 + flip;
+                        const FlipFromBuffer src{wt[l]};
+                        special_step<DBL, OVER, ETA>(k, st, i, g, a, s0 + l, off, src);
+                    } else {
+                        const FlipDraw src;
+                        special_step<DBL, OVER, ETA>(k, st, i, g, a, s0 + l, off, src);
+                    }
+                    flip = near(a.nflip - (int64_t)s0);
+                    ++l;
+                }
+            }
+            if (!(a.q & Q_RUN)) {
+                c.s_done = s0 + l - ((a.flags & LDP_FLAG_NONFINITE) ? 1 : 0);
+                l = n;
+            } else if (l == fr + 1) {
+                save();
+            }
+            lim = last_start();
+        }
+        __syncwarp();
+    }
+    if (l == fr + 1 && (a.q & Q_RUN)) save();   // at the buffer's end
+    if (DENSE && (a.q & Q_RUN)) a.nflip = (int64_t)s0 + flip;
+}
+
+// Steps s_begin .. s_end-1, one trajectory per thread, each drawing its own
+// noise, kOwnSteps steps at a time (two Philox blocks and four Box-Muller
+// pairs at once) into its row of shared memory, and then taking these steps
+// as in group mode, each lane at its own.  Bound by the issue of ~125
+// instructions a step, 100 of them the noise, at four warps a scheduler (122
+// registers).  65536 trajectories, kernel ms: 29.3 with two pairs at once one
+// after the other and four steps between votes, 25.5 with the pairs together,
+// 23.9 with rows of noise (blocks of four steps, or a try of four before the
+// steps one by one: 24.1).
+constexpr int kOwnSteps = 32;
+template <bool DBL, bool OVER, bool ETA>
+__global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, const TrajState st, int64_t g0,
+                                                         uint64_t s_begin, uint64_t s_end) {
+    __shared__ double rows[128 * (kOwnSteps + 1)];   // of an odd length: see fp64_group_kernel
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t g = (uint32_t)(g0 + i);
+    Lane a;
+    load_lane<DBL, OVER>(k, st, i, i < st.n, a);
+    const bool active = (a.q & Q_RUN) != 0u;
+    Course c = course(k, st, i, s_begin, s_end);
+    const double sig = OVER ? k.sig_r : k.sig_v;
+    double* z = rows + threadIdx.x * (kOwnSteps + 1);
+    uint64_t s0 = ((s_begin - 1) & ~3ull) + 1;   // the first step of a Philox block
+    int l = (int)(s_begin - s0);
+    while (s0 < s_end && __any_sync(0xffffffffu, (a.q & Q_RUN) != 0u)) {
+        const int n = s_end - s0 < (uint64_t)kOwnSteps ? (int)(s_end - s0) : kOwnSteps;
+#pragma unroll 1
+        for (int m = 0; m < n; m += 8) {
+            const uint64_t q = (s0 + (uint64_t)m - 1) >> 2;
+            const Words w = philox_at(q, g, TAG_STEP, k.key0, k.key1), w2 = philox_at(q + 1, g, TAG_STEP, k.key0, k.key1);
+            const uint32_t wa[4] = {w.w0, w.w2, w2.w0, w2.w2}, wb[4] = {w.w1, w.w3, w2.w1, w2.w3};
+            double r[8];
+            gauss_pairs_f64(wa, wb, r);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) z[m + j] = sig * r[j];
+        }
+        take_steps<DBL, OVER, ETA, false, kGrpSteps>(k, st, i, g, a, c, s0, l, n, z, nullptr);
+        l = 0;
+        s0 += kOwnSteps;
+    }
+    if (active) store_lane(k, st, i, a, c.s_done, s_begin, s_end);
+}
+
 template <bool DBL, bool OVER, bool ETA, bool DENSE>
 __global__ void __launch_bounds__(32 * (kGrpConsumers + kGrpProducers), 1) fp64_group_kernel(const KConst k, const TrajState st, int64_t g0,
                                                             uint64_t s_begin, uint64_t s_end, int nc, int T, int B) {
     // noise [2][M][R], then with DENSE waits [2][M][R]; rows of an odd length,
     // so that lanes at the same step are in different banks
-    constexpr int N = kGrpSteps;
     extern __shared__ double buf[];
     const int M = nc * T, R = B + 1, nthreads = blockDim.x;
     uint32_t* waits = (uint32_t*)(buf + 2 * R * M);
@@ -1032,118 +1134,20 @@ __global__ void __launch_bounds__(32 * (kGrpConsumers + kGrpProducers), 1) fp64_
     Lane a;
     load_lane<DBL, OVER>(k, st, i, lane < T && i < st.n, a);
     const bool active = (a.q & Q_RUN) != 0u;
-    const uint64_t fs = k.freq_save;
-    uint64_t s_done = s_end;   // this lane's first step not integrated
-    int64_t frame = (int64_t)((s_begin + fs - 1) / fs);   // this lane's next frame
-    double* px = st.fx ? st.fx + frame * st.n + i : nullptr;
-    const int ifs = fs < (1u << 30) ? (int)fs : 1 << 30;
+    Course c = course(k, st, i, s_begin, s_end);
     const int tl = lane < T ? tr : warp * T;   // idle lanes read a lane's noise
-    auto near = [](int64_t d) { return d < (1 << 30) ? (int)d : 1 << 30; };
     for (uint64_t b = 0; b < nblk; ++b) {
         const int u = (int)(b & 1);
         bar_sync(1 + u, nthreads);                   // buffer u full
         const double* z = buf + (u * M + tl) * R;
         const uint32_t* wt = waits + (u * M + tl) * R;
         const uint64_t s0 = sb + b * (uint64_t)B;
-        // Steps s0 + l, l < n; each lane at its own l: a lane goes on from a
-        // special step with a new block, and its warp waits for it at the
-        // buffer's end only.
         const int n = s_end - s0 < (uint64_t)B ? (int)(s_end - s0) : B;
-        int l = b == 0 ? (int)(s_begin - sb) : 0;
-        if (!(a.q & Q_RUN)) l = n;
-        // the places of the next frame and of the pending flip, and the last
-        // place a block can start at
-        int fr = k.fp_mode ? 1 << 30 : near(frame * (int64_t)fs - (int64_t)s0);
-        int flip = near(a.nflip - (int64_t)s0);
-        auto save = [&]() {
-            if (frame < k.nframe) {
-                if (k.write_x) save_frame<DBL>(k, st, i, a, frame);
-                else if (px) *px = a.t.x;
-            }
-            px += st.n;
-            ++frame;
-            fr = min(fr + ifs, 1 << 30);
-        };
-        auto last_start = [&]() { return min(min(n, fr + 1), ETA && !DENSE ? flip : n) - N; };
-        int lim = last_start();
-        while (__any_sync(0xffffffffu, l < n)) {
-            bool failed = false;
-            if (!__any_sync(0xffffffffu, l < n && l > lim)) {
-                // blocks, until a lane cannot go on with one
-                const bool flat = OVER && !DENSE && !__any_sync(0xffffffffu, (a.q & Q_FORCE) != 0u);
-                bool on, stop;
-#pragma unroll 1
-                do {
-                    on = l <= lim;
-                    const int lc = on ? l : 0;
-                    double rf[N];
-#pragma unroll
-                    for (int m = 0; m < N; ++m) rf[m] = z[lc + m];
-                    bool stands;
-                    if (DENSE) {
-                        uint32_t w[N];
-#pragma unroll
-                        for (int m = 0; m < N; ++m) w[m] = wt[lc + m];
-                        stands = dense_block<OVER, N>(k, a, on, flip, lc, rf, w);
-                    } else if (flat) {
-                        stands = quiet_moves<OVER, true, N>(k, a, on, rf);
-                    } else {
-                        stands = quiet_moves<OVER, false, N>(k, a, on, rf);
-                    }
-                    l += stands ? N : 0;
-                    failed = on && !stands;
-                    stop = on && (failed || l > lim);
-                } while (!__any_sync(0xffffffffu, stop));
-            }
-            if (l < n && (failed || l > lim)) {
-                if (l != fr + 1) {
-                    // one by one, to the first special step and over it, or
-                    // to the next place where blocks can go on
-                    const int end = min(failed ? l + N : n, fr + 1);
-                    int n1 = 0;
-                    bool off;
-                    do {
-                        fp64_move<OVER>(k, a.t, z[l]);
-                        off = !(off_band(a, a.t.x) < a.half);
-                        if (off || (ETA && !DENSE && l == flip)) break;
-                        if (DENSE && l == flip) {
-                            a.t.state ^= 1;
-                            flip = l + (int)__byte_perm(wt[l], 0, a.t.state ? 0x4432 : 0x4410);
-                            a.t.F = a.t.state ? a.bF1 : a.bF0;
-                        }
-                        n1 += a.t.state;
-                        if (!OVER) a.t.v = a.t.v + (k.invM * a.t.F) * k.hdt;
-                    } while (++l < end);
-                    a.sc1 += n1;
-                    if (l < end) {
-                        if (DENSE) {
-                            a.nflip = (int64_t)s0 + flip;
-                            const FlipFromBuffer src{wt[l]};
-                            special_step<DBL, OVER, ETA>(k, st, i, g, a, s0 + l, off, src);
-                        } else {
-                            const FlipDraw src;
-                            special_step<DBL, OVER, ETA>(k, st, i, g, a, s0 + l, off, src);
-                        }
-                        flip = near(a.nflip - (int64_t)s0);
-                        ++l;
-                    }
-                }
-                if (!(a.q & Q_RUN)) {
-                    s_done = s0 + l - ((a.flags & LDP_FLAG_NONFINITE) ? 1 : 0);
-                    l = n;
-                } else if (l == fr + 1) {
-                    save();
-                }
-                lim = last_start();
-            }
-            __syncwarp();
-        }
-        if (l == fr + 1 && (a.q & Q_RUN)) save();   // at the buffer's end
-        if (DENSE && (a.q & Q_RUN)) a.nflip = (int64_t)s0 + flip;
+        take_steps<DBL, OVER, ETA, DENSE, kGrpSteps>(k, st, i, g, a, c, s0, b == 0 ? (int)(s_begin - sb) : 0, n, z, wt);
         __syncwarp();
         bar_arrive(3 + u, nthreads);                 // buffer u released
     }
-    if (active) store_lane(k, st, i, a, s_done, s_begin, s_end);
+    if (active) store_lane(k, st, i, a, c.s_done, s_begin, s_end);
 }
 
 template <bool DBL, bool OVER>
