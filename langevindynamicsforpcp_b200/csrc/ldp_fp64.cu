@@ -818,8 +818,11 @@ __device__ __forceinline__ bool quiet_moves(const KConst& k, Lane& a, bool want,
 // trajectories, B steps a buffer, one Philox block and two Box-Muller pairs
 // for four steps of a trajectory.  A consumer's chain of a quiet step is then
 // two additions (three operations where there is a force).  Two buffers
-// alternate; named barriers 1-2 ("full") and 3-4 ("empty") over all the CTA's
-// warps hand them over, every arrival matched by one wait, with no spin loop.
+// alternate; four named barriers ("full" and "empty" of either) over a
+// consumer warp and its producer warps hand them over, every arrival matched
+// by one wait, with no spin loop.  Each consumer warp has its own: with the
+// CTA's four on common barriers each waits for the slowest at every buffer
+// (900 double-barrier trajectories 6.65 / 5.19 ms).
 //
 // T is chosen so that every scheduler of the GPU has one consumer warp
 // (launch_fp64_group): a warp waits for each of its lanes' special steps, so
@@ -1084,23 +1087,28 @@ __global__ void __launch_bounds__(32 * (kGrpConsumers + kGrpProducers), 1) fp64_
     // noise [2][M][R], then with DENSE waits [2][M][R]; rows of an odd length,
     // so that lanes at the same step are in different banks
     extern __shared__ double buf[];
-    const int M = nc * T, R = B + 1, nthreads = blockDim.x;
+    const int M = nc * T, R = B + 1, P = (blockDim.x >> 5) - nc;
     uint32_t* waits = (uint32_t*)(buf + 2 * R * M);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t i0 = (int64_t)blockIdx.x * M;
+    // its consumer warp (producer warp p draws for the warp p mod nc), that
+    // warp's trajectories, and the threads that share its barriers
+    const int cw = warp < nc ? warp : (warp - nc) % nc, t0 = cw * T;
+    const int64_t i0 = (int64_t)blockIdx.x * M + t0;
+    const int nthreads = 32 * (1 + (P - cw + nc - 1) / nc);
+    const int full = 4 * cw, empty = 4 * cw + 2;
     const uint64_t a0 = (s_begin - 1) >> 2;           // the first buffer starts on a Philox block
     const uint64_t sb = 4 * a0 + 1;
     const uint64_t nblk = s_end > s_begin ? (s_end - sb + B - 1) / B : 0;
     if (warp >= nc) {
         // ---- producers ----
-        const int p = (warp - nc) * 32 + lane, np = nthreads - 32 * nc;
+        const int p = (warp - nc) / nc * 32 + lane, np = nthreads - 32;
         const double sig = OVER ? k.sig_r : k.sig_v;
         for (uint64_t b = 0; b < nblk; ++b) {
             const int u = (int)(b & 1);
-            if (b >= 2) bar_sync(3 + u, nthreads);   // buffer u released by the consumers
-            double* z = buf + u * R * M;
-            for (int e = p; e < (B >> 2) * M; e += np) {
-                const int quad = e / M, tr = e - quad * M;
+            if (b >= 2) bar_sync(empty + u, nthreads);   // buffer u released by the consumer
+            double* z = buf + (u * M + t0) * R;
+            for (int e = p; e < (B >> 2) * T; e += np) {
+                const int quad = e / T, tr = e - quad * T;
                 const uint64_t q = a0 + b * (uint64_t)(B >> 2) + (uint64_t)quad;
                 if (i0 + tr >= st.n || 4 * q + 1 >= s_end) continue;
                 const Words w = philox_at(q, (uint32_t)(g0 + i0 + tr), TAG_STEP, k.key0, k.key1);
@@ -1111,9 +1119,9 @@ __global__ void __launch_bounds__(32 * (kGrpConsumers + kGrpProducers), 1) fp64_
                 for (int m = 0; m < 4; ++m) o[m] = sig * n[m];
             }
             if (DENSE) {
-                uint32_t* wt = waits + u * R * M;
-                for (int e = p; e < B * M; e += np) {
-                    const int step = e / M, tr = e - step * M;
+                uint32_t* wt = waits + (u * M + t0) * R;
+                for (int e = p; e < B * T; e += np) {
+                    const int step = e / T, tr = e - step * T;
                     const uint64_t s = sb + b * (uint64_t)B + (uint64_t)step;
                     if (i0 + tr >= st.n || s >= s_end) continue;
                     const Words wf = philox_at(s, (uint32_t)(g0 + i0 + tr), TAG_FLIP, k.key0, k.key1);
@@ -1121,31 +1129,30 @@ __global__ void __launch_bounds__(32 * (kGrpConsumers + kGrpProducers), 1) fp64_
                 }
             }
             __syncwarp();
-            bar_arrive(1 + u, nthreads);             // buffer u full
+            bar_arrive(full + u, nthreads);          // buffer u full
         }
-        // the consumers' release of the last two buffers
-        for (uint64_t b = (nblk > 2 ? nblk - 2 : 0); b < nblk; ++b) bar_sync(3 + (int)(b & 1), nthreads);
+        // the consumer's release of the last two buffers
+        for (uint64_t b = (nblk > 2 ? nblk - 2 : 0); b < nblk; ++b) bar_sync(empty + (int)(b & 1), nthreads);
         return;
     }
     // ---- consumers ----
-    const int tr = warp * T + lane;
-    const int64_t i = i0 + tr;
+    const int64_t i = i0 + lane;
     const uint32_t g = (uint32_t)(g0 + i);
     Lane a;
     load_lane<DBL, OVER>(k, st, i, lane < T && i < st.n, a);
     const bool active = (a.q & Q_RUN) != 0u;
     Course c = course(k, st, i, s_begin, s_end);
-    const int tl = lane < T ? tr : warp * T;   // idle lanes read a lane's noise
+    const int tl = t0 + (lane < T ? lane : 0);   // idle lanes read a lane's noise
     for (uint64_t b = 0; b < nblk; ++b) {
         const int u = (int)(b & 1);
-        bar_sync(1 + u, nthreads);                   // buffer u full
+        bar_sync(full + u, nthreads);                // buffer u full
         const double* z = buf + (u * M + tl) * R;
         const uint32_t* wt = waits + (u * M + tl) * R;
         const uint64_t s0 = sb + b * (uint64_t)B;
         const int n = s_end - s0 < (uint64_t)B ? (int)(s_end - s0) : B;
         take_steps<DBL, OVER, ETA, DENSE, kGrpSteps>(k, st, i, g, a, c, s0, b == 0 ? (int)(s_begin - sb) : 0, n, z, wt);
         __syncwarp();
-        bar_arrive(3 + u, nthreads);                 // buffer u released
+        bar_arrive(empty + u, nthreads);             // buffer u released
     }
     if (active) store_lane(k, st, i, a, c.s_done, s_begin, s_end);
 }
