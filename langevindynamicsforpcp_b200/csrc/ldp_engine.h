@@ -81,5 +81,8 @@ int launch_fp64_steps(const KConst& k, const TrajState& st, int64_t g0, uint64_t
 // for bit).
 int launch_fp64_group(const KConst& k, const TrajState& st, int64_t g0, uint64_t s_begin, uint64_t s_end, int sms,
                       int min_lanes, void* stream);
+// WRITEX's force, barrier height and energies of the frames saved in steps
+// s_begin .. s_end-1, all of which are done.
+int launch_fp64_series(const KConst& k, const TrajState& st, uint64_t s_begin, uint64_t s_end, int sms, void* stream);
 
 }  // namespace ldp

@@ -756,14 +756,6 @@ __device__ __forceinline__ void special_step(const KConst& k, const TrajState& s
     if (!OVER) a.t.v = a.t.v + (k.invM * a.t.F) * k.hdt;
 }
 
-// A saved frame (after its step, a multiple of FREQSAVE); the energy and the
-// barrier height are those of the position, whatever kind of step led there.
-template <bool DBL>
-__device__ __forceinline__ void save_frame(const KConst& k, const TrajState& st, int64_t i, Lane& a, int64_t frame) {
-    if (k.write_x) energy_force<DBL>(k, a.t);
-    record(k, st, a.t, i, frame);
-}
-
 // N steps from the band, rf[m] their noise; true and the lane (one that wants
 // to) moved on when they stand.  FLAT: no lane of the warp has a force (fma(0, c, x) is x).
 template <bool OVER, bool FLAT, int N>
@@ -952,9 +944,12 @@ __device__ __forceinline__ void take_steps(const KConst& k, const TrajState& st,
     int fr = k.fp_mode ? 1 << 30 : near(c.frame * (int64_t)k.freq_save - (int64_t)s0);
     int flip = near(a.nflip - (int64_t)s0);
     auto save = [&]() {
-        if (c.frame < k.nframe) {
-            if (k.write_x) save_frame<DBL>(k, st, i, a, c.frame);
-            else if (c.px) *c.px = a.t.x;
+        if (c.frame < k.nframe && c.px) {
+            *c.px = a.t.x;
+            if (k.write_x && st.fv) {   // the rest of WRITEX: fp64_series_kernel
+                c.px[st.fv - st.fx] = a.t.v;
+                c.px[st.fst - st.fx] = (double)a.t.state;
+            }
         }
         c.px += st.n;
         ++c.frame;
@@ -1155,6 +1150,43 @@ __global__ void __launch_bounds__(32 * (kGrpConsumers + kGrpProducers), 1) fp64_
         bar_arrive(empty + u, nthreads);             // buffer u released
     }
     if (active) store_lane(k, st, i, a, c.s_done, s_begin, s_end);
+}
+
+// WRITEX's other series of frames f0 .. f1 - 1 from their position, velocity
+// and barrier state: force, energy and barrier height are those of the
+// position, whatever kind of step led there.  The steps save three of the
+// seven series only: a frame cost its stepping warp 200-300 cycles more with all of
+// them (the sample
+// input, a frame in 80 steps, 6.83 / 6.66 ms; a frame a step 0.544 / 0.523), and
+// this pass over the frames is memory-bound.
+template <bool DBL>
+__global__ void __launch_bounds__(256) fp64_series_kernel(const KConst k, const TrajState st, int64_t f0, int64_t f1) {
+    const int64_t n = st.n, end = f1 * n, stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t o = f0 * n + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < end; o += stride) {
+        const int64_t f = o / n;
+        // (not past the end of a trajectory that ended early)
+        if (f * (int64_t)k.freq_save > st.counts[(int64_t)LDP_C_STEPS * n + (o - f * n)]) continue;
+        T64 t{};
+        t.x = st.fx[o];
+        t.v = st.fv[o];
+        t.state = (int)st.fst[o];
+        indices<DBL>(k, t);
+        energy_force<DBL>(k, t);
+        st.ff[o] = t.F;
+        st.fb[o] = t.barrier;
+        st.fpe[o] = t.E;
+        st.fke[o] = k.mhalf * (t.v * t.v);
+    }
+}
+
+int launch_fp64_series(const KConst& k, const TrajState& st, uint64_t s_begin, uint64_t s_end, int sms, void* stream) {
+    const int64_t fs = (int64_t)k.freq_save;
+    const int64_t f0 = ((int64_t)s_begin + fs - 1) / fs, f1 = std::min<int64_t>(k.nframe, ((int64_t)s_end - 1) / fs + 1);
+    if (!k.write_x || !st.fx || !st.fv || f1 <= f0 || st.n <= 0) return 0;
+    const int64_t blocks = std::min<int64_t>(((f1 - f0) * st.n + 255) / 256, (int64_t)8 * sms);
+    if (k.dbl) fp64_series_kernel<true><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(k, st, f0, f1);
+    else fp64_series_kernel<false><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(k, st, f0, f1);
+    return (int)cudaGetLastError();
 }
 
 template <bool DBL, bool OVER>

@@ -594,6 +594,14 @@ static ldp_status submit_on(ldp_ctx* ctx, ldp_job* job, cudaStream_t s) {
             }
             ++job->launches;
         }
+        if (fixed && job->k.write_x) {
+            e = launch_fp64_series(job->k, job->st, first, last + 1, ctx->sm_count, s);
+            if (e) {
+                ldp_set_error(ctx, "series launch failed: %s", cudaGetErrorString((cudaError_t)e));
+                return LDP_ERR_DEVICE;
+            }
+            ++job->launches;
+        }
         CUDA_OR_FAIL(ctx, cudaEventRecord(job->ev[1], s));
     }
     if (job->o.mode == LDP_MODE_FIXED_STEPS && !job->lags.empty()) {
