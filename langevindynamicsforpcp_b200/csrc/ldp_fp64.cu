@@ -556,10 +556,10 @@ __device__ __forceinline__ void band_forces(const KConst& k, const T64& t, doubl
 // Steps of a lane
 //
 // A lane steps one trajectory; all lanes of a launch are at the same step.
-// Steps are taken in blocks without a test between them (quiet_block): they
+// Steps are taken in blocks without a test between them (quiet_moves): they
 // stand when the position stayed in the quiet band and, with rare flips, no
 // flip was pending in the block.  The lanes whose block does not stand take
-// its steps one by one (one_step): quiet; quick (the flank of the barrier
+// its steps one by one (take_steps): quiet; quick (the flank of the barrier
 // entered or left, or the edge between the cells of a pair crossed); or full
 // (fp64_after_move).  Same operations on the same values in every case, so
 // the results are those of full steps throughout, bit for bit.
@@ -835,8 +835,9 @@ __device__ __forceinline__ bool quiet_moves(const KConst& k, Lane& a, bool want,
 //
 // What it measured (ns a step; one CTA a trajectory, or of 32 trajectories,
 // with a producer warp or four, flips drawn for every step / this): the
-// sample input, 32 trajectories, p = 1/2: 62.3 / 40.8; rare flips, 592: 91 /
-// 45, 2000: 312 / 68, 5003 underdamped: 235 / 60, 16000: 503 / 202.
+// sample input, 32 trajectories, p = 1/2: 62.3 / 40.3; 900 of two barriers:
+// 190 / 84; rare flips, 592: 91 / 45, 2000: 312 / 68, 5003 underdamped: 235 /
+// 56, 16000: 503 / 202.
 // ---------------------------------------------------------------------------
 constexpr int kGrpConsumers = 4;   // consumer warps of a CTA at most: one to a scheduler
 constexpr int kGrpProducers = 8;   // producer warps (4: 16000 trajectories 263 ns a step, 12: 197)
@@ -869,16 +870,22 @@ struct FlipFromBuffer {
 };
 
 // quiet_moves with flips taken from the producer's waits w[m]; l the first
-// step's place in the buffer, flip that of the pending flip.
-template <bool OVER, int N>
+// step's place in the buffer, flip that of the pending flip.  The state is
+// kept as the byte selector of its half of a wait (kWait0 or kWait1), the
+// steps in state 1 as the selectors' sum; FLAT as there.  One warp alone on
+// its scheduler takes ~50 cycles a step: the sample input 6.66 / 6.55 ms with
+// these.
+constexpr uint32_t kWait0 = 0x4410, kWait1 = 0x4432;
+template <bool OVER, bool FLAT, int N>
 __device__ __forceinline__ bool dense_block(const KConst& k, Lane& a, bool want, int& flip, int l, const double* rf,
                                             const uint32_t* w) {
     double x = a.t.x, r = a.t.rprev, v = a.t.v, F = a.t.F;
-    int nf = flip - l, state = a.t.state, n1 = 0, far = 0;
+    int nf = flip - l, far = 0;
+    uint32_t sel = a.t.state ? kWait1 : kWait0, sum = 0;
 #pragma unroll
     for (int m = 0; m < N; ++m) {
         if (OVER) {
-            x = fma(F, k.c_drift, x);
+            if (!FLAT) x = fma(F, k.c_drift, x);
             x = x + rf[m];
             x = x + r;
             r = rf[m];
@@ -890,13 +897,15 @@ __device__ __forceinline__ bool dense_block(const KConst& k, Lane& a, bool want,
         }
         far = max(far, off_band(a, x));
         if (nf == m) {
-            state ^= 1;
-            nf = m + (int)__byte_perm(w[m], 0, state ? 0x4432 : 0x4410);
+            sel ^= kWait0 ^ kWait1;
+            nf = m + (int)__byte_perm(w[m], 0, sel);
         }
-        F = state ? a.bF1 : a.bF0;
-        n1 += state;
+        if (!OVER || !FLAT) F = (sel & 2u) ? a.bF1 : a.bF0;
+        sum += sel;
         if (!OVER) v = v + (k.invM * F) * k.hdt;
     }
+    const int state = (int)(sel >> 1) & 1, n1 = (int)((sum - N * kWait0) / (kWait1 - kWait0));
+    if (OVER && FLAT) F = state ? a.bF1 : a.bF0;
     if (!(want && far < a.half)) return false;
     a.t.x = x;
     a.t.rprev = r;
@@ -961,7 +970,7 @@ __device__ __forceinline__ void take_steps(const KConst& k, const TrajState& st,
         bool failed = false;
         if (!__any_sync(0xffffffffu, l < n && l > lim)) {
             // blocks, until a lane cannot go on with one
-            const bool flat = OVER && !DENSE && !__any_sync(0xffffffffu, (a.q & Q_FORCE) != 0u);
+            const bool flat = OVER && !__any_sync(0xffffffffu, (a.q & Q_FORCE) != 0u);
             bool on, stop;
 #pragma unroll 1
             do {
@@ -975,7 +984,8 @@ __device__ __forceinline__ void take_steps(const KConst& k, const TrajState& st,
                     uint32_t w[N];
 #pragma unroll
                     for (int m = 0; m < N; ++m) w[m] = wt[lc + m];
-                    stands = dense_block<OVER, N>(k, a, on, flip, lc, rf, w);
+                    stands = flat ? dense_block<OVER, true, N>(k, a, on, flip, lc, rf, w)
+                                  : dense_block<OVER, false, N>(k, a, on, flip, lc, rf, w);
                 } else if (flat) {
                     stands = quiet_moves<OVER, true, N>(k, a, on, rf);
                 } else {
@@ -1155,10 +1165,9 @@ __global__ void __launch_bounds__(32 * (kGrpConsumers + kGrpProducers), 1) fp64_
 // WRITEX's other series of frames f0 .. f1 - 1 from their position, velocity
 // and barrier state: force, energy and barrier height are those of the
 // position, whatever kind of step led there.  The steps save three of the
-// seven series only: a frame cost its stepping warp 200-300 cycles more with all of
-// them (the sample
-// input, a frame in 80 steps, 6.83 / 6.66 ms; a frame a step 0.544 / 0.523), and
-// this pass over the frames is memory-bound.
+// seven series only, which keeps the rest out of the stepping warps' chains
+// (the sample input, a frame in 80 steps, 6.83 / 6.66 ms; a frame a step 0.544
+// / 0.523); this pass over the frames is memory-bound.
 template <bool DBL>
 __global__ void __launch_bounds__(256) fp64_series_kernel(const KConst k, const TrajState st, int64_t f0, int64_t f1) {
     const int64_t n = st.n, end = f1 * n, stride = (int64_t)gridDim.x * blockDim.x;
