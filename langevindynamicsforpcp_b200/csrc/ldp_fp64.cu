@@ -818,8 +818,14 @@ __device__ __forceinline__ bool quiet_moves(const KConst& k, Lane& a, bool want,
 //
 // T is chosen so that every scheduler of the GPU has one consumer warp
 // (launch_fp64_group): a warp waits for each of its lanes' special steps, so
-// fewer lanes a warp step faster, and warps beyond one a scheduler slow each
-// other and the producers down.
+// fewer lanes a warp step faster.  TWO: two consumer warps a scheduler, of half
+// as many lanes, in two CTAs an SM.  Overdamped steps (two or three FP64
+// operations in a row) leave a scheduler to the other warp; underdamped ones
+// (five, and more instructions) do not, and with frequent flips and eight
+// lanes a warp the fewer producers count.  One / two, ms for 24000 steps: 900
+// trajectories of two barriers 2.67 / 2.03, rare flips 1.54 / 1.35, 2000 3.42 /
+// 2.93 and 1.79 / 1.63; 8000 6.33 / 6.52 and 3.03 / 2.64; underdamped 900 1.25 /
+// 1.34, 5003 1.48 / 1.87.
 //
 // Within a buffer each lane is at its own step: after a special step it goes
 // on with a new block of kGrpSteps steps, so a special step costs its warp
@@ -841,6 +847,7 @@ __device__ __forceinline__ bool quiet_moves(const KConst& k, Lane& a, bool want,
 // ---------------------------------------------------------------------------
 constexpr int kGrpConsumers = 4;   // consumer warps of a CTA at most: one to a scheduler
 constexpr int kGrpProducers = 8;   // producer warps (4: 16000 trajectories 263 ns a step, 12: 197)
+constexpr int kGrpTwoProducers = 4;   // ... of a CTA with TWO
 constexpr int kGrpSteps = 8;       // steps of a consumer's block (16: 5 % slower at 2 lanes a warp, 10 % faster at 1)
 constexpr int kGrpItems = 8;       // items (four steps of a trajectory) of a producer lane in a buffer (4: 219 ns)
 constexpr int kGrpBuffer = 256;    // steps of a buffer at most
@@ -1086,8 +1093,8 @@ __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, cons
     if (active) store_lane(k, st, i, a, c.s_done, s_begin, s_end);
 }
 
-template <bool DBL, bool OVER, bool ETA, bool DENSE>
-__global__ void __launch_bounds__(32 * (kGrpConsumers + kGrpProducers), 1) fp64_group_kernel(const KConst k, const TrajState st, int64_t g0,
+template <bool DBL, bool OVER, bool ETA, bool DENSE, bool TWO>
+__global__ void __launch_bounds__(32 * (kGrpConsumers + (TWO ? kGrpTwoProducers : kGrpProducers)), TWO ? 2 : 1) fp64_group_kernel(const KConst k, const TrajState st, int64_t g0,
                                                             uint64_t s_begin, uint64_t s_end, int nc, int T, int B) {
     // noise [2][M][R], then with DENSE waits [2][M][R]; rows of an odd length,
     // so that lanes at the same step are in different banks
@@ -1222,12 +1229,16 @@ static int launch_steps_t(const KConst& k, const TrajState& st, int64_t g0, uint
 
 template <bool DBL, bool OVER, bool ETA>
 static int launch_group_t(const KConst& k, const TrajState& st, int64_t g0, uint64_t s0, uint64_t s1, int nc, int T,
-                          int P, int B, bool dense, cudaStream_t stream) {
+                          int P, int B, bool dense, bool two, cudaStream_t stream) {
     const int M = nc * T;
     const int64_t grid = (st.n + M - 1) / M;
     const size_t smem = (size_t)2 * (B + 1) * M * (dense ? 12 : 8);
-    auto* kern = fp64_group_kernel<DBL, OVER, ETA, false>;
-    if (ETA && dense) kern = fp64_group_kernel<DBL, OVER, ETA, ETA>;
+    auto* kern = fp64_group_kernel<DBL, OVER, ETA, false, false>;
+    if (ETA && dense) kern = fp64_group_kernel<DBL, OVER, ETA, ETA, false>;
+    if (OVER && two) {
+        kern = fp64_group_kernel<DBL, OVER, ETA, false, OVER>;
+        if (ETA && dense) kern = fp64_group_kernel<DBL, OVER, ETA, ETA, OVER>;
+    }
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     kern<<<(unsigned)grid, 32 * (nc + P), smem, stream>>>(k, st, g0, s0, s1, nc, T, B);
@@ -1238,33 +1249,35 @@ int launch_fp64_group(const KConst& k, const TrajState& st, int64_t g0, uint64_t
                       int min_lanes, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     if (st.n <= 0) return 0;
-    // One consumer warp to each of the GPU's schedulers, with as many lanes
-    // as that takes.
-    int T = (int)std::min<int64_t>(32, (st.n + 4 * sms - 1) / (4 * sms));
-    T = std::max(T, min_lanes);
-    const int nc = (int)std::min<int64_t>(kGrpConsumers, (st.n + (int64_t)sms * T - 1) / ((int64_t)sms * T));
-    const int M = nc * T;
     double p = 0.0, pmin = 1.0;
     for (int b = 0; b < 2; ++b) {
         const double f = k.eta ? -std::expm1(k.ln1m[b]) : 0.0;
         p = std::max(p, f);
         pmin = std::min(pmin, f);
     }
+    // One consumer warp to each of the GPU's schedulers, or two, with as many
+    // lanes as that takes.
+    int T = (int)std::min<int64_t>(32, (st.n + 4 * sms - 1) / (4 * sms));
+    const bool two = k.over && T > min_lanes && (min_lanes == 1 || p < 1.0 / 1024);
+    if (two) T = (int)std::min<int64_t>(32, (st.n + 8 * sms - 1) / (8 * sms));
+    T = std::max(T, min_lanes);
+    const int nc = (int)std::min<int64_t>(kGrpConsumers, (st.n + (int64_t)sms * T - 1) / ((int64_t)sms * T));
+    const int M = nc * T;
     const bool dense = k.eta && pmin >= 1.0 / 1024 && p * T > 1.0 / 40;
-    const int P = kGrpProducers;
+    const int P = two ? kGrpTwoProducers : kGrpProducers;
     int B = 8 * ((32 * P * kGrpItems * 4 / M + 7) / 8);
-    const int room = (200 << 10) / (2 * M * (dense ? 12 : 8)) - 1;   // shared memory
+    const int room = ((two ? 100 : 200) << 10) / (2 * M * (dense ? 12 : 8)) - 1;   // shared memory
     B = std::min(std::min(std::max(B, 16), kGrpBuffer), room / 8 * 8);
     const int sel = (k.dbl ? 4 : 0) | (k.over ? 2 : 0) | (k.eta ? 1 : 0);
     switch (sel) {
-        case 0: return launch_group_t<false, false, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
-        case 1: return launch_group_t<false, false, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
-        case 2: return launch_group_t<false, true, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
-        case 3: return launch_group_t<false, true, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
-        case 4: return launch_group_t<true, false, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
-        case 5: return launch_group_t<true, false, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
-        case 6: return launch_group_t<true, true, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
-        default: return launch_group_t<true, true, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, s);
+        case 0: return launch_group_t<false, false, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, two, s);
+        case 1: return launch_group_t<false, false, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, two, s);
+        case 2: return launch_group_t<false, true, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, two, s);
+        case 3: return launch_group_t<false, true, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, two, s);
+        case 4: return launch_group_t<true, false, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, two, s);
+        case 5: return launch_group_t<true, false, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, two, s);
+        case 6: return launch_group_t<true, true, false>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, two, s);
+        default: return launch_group_t<true, true, true>(k, st, g0, s_begin, s_end, nc, T, P, B, dense, two, s);
     }
 }
 

@@ -1,6 +1,7 @@
 """Latency and group mode of FP64 plain jobs against one trajectory per
 thread, bit for bit, where the split over warps changes (one trajectory, one
-more than SMs, one more than schedulers, one more than eight lanes to each),
+more than SMs, one more than schedulers, one more than eight lanes to each or
+to two warps of each, one more than two lanes),
 with rare and frequent flips (drawn by the stepping warps, or ahead for every
 step), frames at every step, inside blocks and at their ends, and launches
 that start anywhere in a block of four steps."""
@@ -27,7 +28,8 @@ def run(p, n, latency, group, spl):
 
 @pytest.mark.parametrize("n,double,over,tau,freq,spl,write_x", [
     (1, 0, 1, 1e-5, 1, 0, 1), (149, 1, 1, 1e-1, 7, 333, 0), (593, 0, 0, 1e-3, 8, 1001, 1), (593, 1, 0, 1e-5, 3, 0, 0),
-    (4737, 0, 1, 1e-2, 5, 0, 0), (1300, 0, 1, 0.0, 11, 2050, 0)])
+    (4737, 0, 1, 1e-2, 5, 0, 0), (1300, 0, 1, 0.0, 11, 2050, 0), (593, 1, 1, 1e-5, 3, 1500, 1),
+    (1185, 0, 1, 1e-1, 4, 0, 0), (9473, 0, 1, 1e-1, 2, 0, 0)])
 def test_modes_equal_one_trajectory_per_thread(n, double, over, tau, freq, spl, write_x):
     name = "CuIDB_double__2.0_7.2_m1.0_1.00e-05.inp" if double else "quick_test__2.0_7.2_m1.0_1.00e-05.inp"
     p = ldp.params_from_inp(os.path.join(GOLDEN, name), ldp.MODEL_DOUBLE if double else ldp.MODEL_SINGLE)
