@@ -672,8 +672,8 @@ __device__ __forceinline__ int full_step(const KConst& k, const TrajState& st, i
     return 0;
 }
 
-// A quick step after its move (not at the barrier's pending flip); false when
-// the step must be a full one.
+// A quick step after its move and the barrier's flip; false when the step must
+// be a full one.
 template <bool DBL, bool ETA>
 __device__ __forceinline__ bool quick_step(const KConst& k, const TrajState& st, int64_t i, uint32_t g, Lane& a,
                                            uint64_t s) {
@@ -740,16 +740,23 @@ __device__ __forceinline__ bool quick_step(const KConst& k, const TrajState& st,
 template <bool DBL, bool OVER, bool ETA, class Src>
 __device__ __forceinline__ void special_step(const KConst& k, const TrajState& st, int64_t i, uint32_t g, Lane& a,
                                              uint64_t s, bool off, const Src& src) {
-    const bool flip = ETA && (int64_t)s == a.nflip;
-    if (!off) {
-        // the current barrier's flip and nothing else
+    const int64_t nflip = a.nflip;
+    const bool flip = ETA && (int64_t)s == nflip;
+    if (flip) {
         a.t.state ^= 1;
         Words wf;
         bool have = false;
         a.nflip = src.schedule(k, g, s, a.t.state, &wf, &have);
+    }
+    if (!off) {
+        // the current barrier's flip and nothing else
         a.t.F = a.t.state ? a.bF1 : a.bF0;
         a.sc1 += a.t.state;
-    } else if (flip || !quick_step<DBL, ETA>(k, st, i, g, a, s)) {
+    } else if (!quick_step<DBL, ETA>(k, st, i, g, a, s)) {
+        if (flip) {   // as before the flip: a full step takes it too
+            a.t.state ^= 1;
+            a.nflip = nflip;
+        }
         full_step<DBL, OVER, ETA>(k, st, i, g, a, s, src);
         return;   // the velocity's second half-kick included
     }
@@ -833,7 +840,7 @@ __device__ __forceinline__ bool quiet_moves(const KConst& k, Lane& a, bool want,
 // block's remaining steps one by one as well (5000).
 //
 // DENSE: barriers flip so often that a lane could not draw its flips as they
-// come.  Producers then also draw the wait of a flip at every step for both
+// come.  Producers (of one trajectory per thread: the thread) then also draw the wait of a flip at every step for both
 // states (its TAG_FLIP words, one logarithm), in 16 bits: -ln(2^-64) /
 // -ln(1 - p) < 2^16 for p >= 1/1024.  A flip drawn by the consumer costs its
 // warp ~1000 cycles, the waits of all steps ~25 cycles a step and a longer
@@ -841,8 +848,8 @@ __device__ __forceinline__ bool quiet_moves(const KConst& k, Lane& a, bool want,
 //
 // What it measured (ns a step; one CTA a trajectory, or of 32 trajectories,
 // with a producer warp or four, flips drawn for every step / this): the
-// sample input, 32 trajectories, p = 1/2: 62.3 / 40.3; 900 of two barriers:
-// 190 / 84; rare flips, 592: 91 / 45, 2000: 312 / 68, 5003 underdamped: 235 /
+// sample input, 32 trajectories, p = 1/2: 62.3 / 39.2; 900 of two barriers:
+// 190 / 64; rare flips, 592: 91 / 45, 2000: 312 / 68, 5003 underdamped: 235 /
 // 56, 16000: 503 / 202.
 // ---------------------------------------------------------------------------
 constexpr int kGrpConsumers = 4;   // consumer warps of a CTA at most: one to a scheduler
@@ -858,14 +865,20 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
-// Waits of a flip at step s into state 0 (low half) and 1: flip_wait for
-// either state, the logarithm evaluated once.
-__device__ __forceinline__ uint32_t dense_waits(const KConst& k, uint32_t hi, uint32_t lo) {
-    const double u = ((double)(((uint64_t)hi << 32) | lo) + 1.0) * 0x1p-64;
-    const double lu = log_f64(u);
-    const uint32_t w0 = 1u + (uint32_t)floor(lu / k.ln1m[0]);
-    const uint32_t w1 = k.ln1m[1] == k.ln1m[0] ? w0 : 1u + (uint32_t)floor(lu / k.ln1m[1]);
-    return w0 | (w1 << 16);
+// Waits of a flip into state 0 (low half) and 1 by the words of N steps:
+// flip_wait for either state, the logarithms evaluated once and together.
+template <int N>
+__device__ __forceinline__ void dense_waits(const KConst& k, const Words (&wf)[N], uint32_t (&out)[N]) {
+    double u[N], lu[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) u[j] = ((double)(((uint64_t)wf[j].w0 << 32) | wf[j].w1) + 1.0) * 0x1p-64;
+    log_f64(u, lu);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const uint32_t w0 = 1u + (uint32_t)floor(lu[j] / k.ln1m[0]);
+        const uint32_t w1 = k.ln1m[1] == k.ln1m[0] ? w0 : 1u + (uint32_t)floor(lu[j] / k.ln1m[1]);
+        out[j] = w0 | (w1 << 16);
+    }
 }
 
 // The consumer's flip schedule source with DENSE: the producer's waits.
@@ -1059,11 +1072,13 @@ __device__ __forceinline__ void take_steps(const KConst& k, const TrajState& st,
 // after the other and four steps between votes, 25.5 with the pairs together,
 // 23.9 with rows of noise (blocks of four steps, or a try of four before the
 // steps one by one: 24.1).
-constexpr int kOwnSteps = 32;
-template <bool DBL, bool OVER, bool ETA>
+constexpr int kOwnSteps = 32, kOwnDense = 16;
+template <bool DBL, bool OVER, bool ETA, bool DENSE>
 __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, const TrajState st, int64_t g0,
                                                          uint64_t s_begin, uint64_t s_end) {
-    __shared__ double rows[128 * (kOwnSteps + 1)];   // of an odd length: see fp64_group_kernel
+    constexpr int S = DENSE ? kOwnDense : kOwnSteps;
+    __shared__ double rows[128 * (S + 1)];   // of an odd length: see fp64_group_kernel
+    __shared__ uint32_t wrows[DENSE ? 128 * (S + 1) : 1];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t g = (uint32_t)(g0 + i);
     Lane a;
@@ -1071,11 +1086,12 @@ __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, cons
     const bool active = (a.q & Q_RUN) != 0u;
     Course c = course(k, st, i, s_begin, s_end);
     const double sig = OVER ? k.sig_r : k.sig_v;
-    double* z = rows + threadIdx.x * (kOwnSteps + 1);
+    double* z = rows + threadIdx.x * (S + 1);
+    uint32_t* wt = wrows + (DENSE ? threadIdx.x * (S + 1) : 0);
     uint64_t s0 = ((s_begin - 1) & ~3ull) + 1;   // the first step of a Philox block
     int l = (int)(s_begin - s0);
     while (s0 < s_end && __any_sync(0xffffffffu, (a.q & Q_RUN) != 0u)) {
-        const int n = s_end - s0 < (uint64_t)kOwnSteps ? (int)(s_end - s0) : kOwnSteps;
+        const int n = s_end - s0 < (uint64_t)S ? (int)(s_end - s0) : S;
 #pragma unroll 1
         for (int m = 0; m < n; m += 8) {
             const uint64_t q = (s0 + (uint64_t)m - 1) >> 2;
@@ -1086,9 +1102,21 @@ __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, cons
 #pragma unroll
             for (int j = 0; j < 8; ++j) z[m + j] = sig * r[j];
         }
-        take_steps<DBL, OVER, ETA, false, kGrpSteps>(k, st, i, g, a, c, s0, l, n, z, nullptr);
+        if (DENSE) {
+#pragma unroll 1
+            for (int m = 0; m < n; m += 2) {
+                const uint64_t q = s0 + (uint64_t)m;
+                const Words wf[2] = {philox_at(q, g, TAG_FLIP, k.key0, k.key1),
+                                     philox_at(q + 1, g, TAG_FLIP, k.key0, k.key1)};
+                uint32_t w[2];
+                dense_waits(k, wf, w);
+                wt[m] = w[0];
+                wt[m + 1] = w[1];
+            }
+        }
+        take_steps<DBL, OVER, ETA, DENSE, kGrpSteps>(k, st, i, g, a, c, s0, l, n, z, wt);
         l = 0;
-        s0 += kOwnSteps;
+        s0 += S;
     }
     if (active) store_lane(k, st, i, a, c.s_done, s_begin, s_end);
 }
@@ -1136,8 +1164,10 @@ __global__ void __launch_bounds__(32 * (kGrpConsumers + (TWO ? kGrpTwoProducers 
                     const int step = e / T, tr = e - step * T;
                     const uint64_t s = sb + b * (uint64_t)B + (uint64_t)step;
                     if (i0 + tr >= st.n || s >= s_end) continue;
-                    const Words wf = philox_at(s, (uint32_t)(g0 + i0 + tr), TAG_FLIP, k.key0, k.key1);
-                    wt[tr * R + step] = dense_waits(k, wf.w0, wf.w1);
+                    const Words wf[1] = {philox_at(s, (uint32_t)(g0 + i0 + tr), TAG_FLIP, k.key0, k.key1)};
+                    uint32_t w[1];
+                    dense_waits(k, wf, w);
+                    wt[tr * R + step] = w[0];
                 }
             }
             __syncwarp();
@@ -1205,6 +1235,17 @@ int launch_fp64_series(const KConst& k, const TrajState& st, uint64_t s_begin, u
     return (int)cudaGetLastError();
 }
 
+// The larger and the smaller flip probability of a step.
+static void flip_rates(const KConst& k, double* p, double* pmin) {
+    *p = 0.0;
+    *pmin = 1.0;
+    for (int b = 0; b < 2; ++b) {
+        const double f = k.eta ? -std::expm1(k.ln1m[b]) : 0.0;
+        *p = std::max(*p, f);
+        *pmin = std::min(*pmin, f);
+    }
+}
+
 template <bool DBL, bool OVER>
 static int launch_init_t(const KConst& k, const TrajState& st, int64_t g0, int block, cudaStream_t stream) {
     const int64_t grid = (st.n + block - 1) / block;
@@ -1223,7 +1264,17 @@ template <bool DBL, bool OVER, bool ETA>
 static int launch_steps_t(const KConst& k, const TrajState& st, int64_t g0, uint64_t s0, uint64_t s1, int block,
                           cudaStream_t stream) {
     const int64_t grid = (st.n + block - 1) / block;
-    fp64_steps_kernel<DBL, OVER, ETA><<<(unsigned)grid, block, 0, stream>>>(k, st, g0, s0, s1);
+    double p, pmin;
+    flip_rates(k, &p, &pmin);
+    // DENSE: drawing the waits of every step costs about as much as the noise,
+    // a flip drawn as it comes a special step of its lane.  65536 trajectories
+    // x 12000 steps, ms as they come / DENSE: p = 0.5 18.3 / 14.8, 0.1 16.3 /
+    // 14.4, 0.01 9.3 / 13.7; two barriers 20.7 / 20.7, 19.4 / 19.5, 12.7 / 17.3;
+    // underdamped 16.5 / 10.9, 14.5 / 10.8, 7.4 / 10.7.
+    if (ETA && pmin > 0.05)
+        fp64_steps_kernel<DBL, OVER, ETA, ETA><<<(unsigned)grid, block, 0, stream>>>(k, st, g0, s0, s1);
+    else
+        fp64_steps_kernel<DBL, OVER, ETA, false><<<(unsigned)grid, block, 0, stream>>>(k, st, g0, s0, s1);
     return (int)cudaGetLastError();
 }
 
@@ -1249,12 +1300,8 @@ int launch_fp64_group(const KConst& k, const TrajState& st, int64_t g0, uint64_t
                       int min_lanes, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     if (st.n <= 0) return 0;
-    double p = 0.0, pmin = 1.0;
-    for (int b = 0; b < 2; ++b) {
-        const double f = k.eta ? -std::expm1(k.ln1m[b]) : 0.0;
-        p = std::max(p, f);
-        pmin = std::min(pmin, f);
-    }
+    double p, pmin;
+    flip_rates(k, &p, &pmin);
     // One consumer warp to each of the GPU's schedulers, or two, with as many
     // lanes as that takes.
     int T = (int)std::min<int64_t>(32, (st.n + 4 * sms - 1) / (4 * sms));
