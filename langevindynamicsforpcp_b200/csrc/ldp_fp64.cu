@@ -840,9 +840,9 @@ __device__ __forceinline__ bool quiet_moves(const KConst& k, Lane& a, bool want,
 // block's remaining steps one by one as well (5000).
 //
 // DENSE: barriers flip so often that a lane could not draw its flips as they
-// come.  Producers (of one trajectory per thread: the thread) then also draw the wait of a flip at every step for both
-// states (its TAG_FLIP words, one logarithm), in 16 bits: -ln(2^-64) /
-// -ln(1 - p) < 2^16 for p >= 1/1024.  A flip drawn by the consumer costs its
+// come.  Producers (with one trajectory per thread, the thread) then also draw
+// the wait of a flip at every step for both states (its TAG_FLIP words, one
+// logarithm), in 16 bits: -ln(2^-64) / -ln(1 - p) < 2^16 for p >= 1/1024.  A flip drawn by the consumer costs its
 // warp ~1000 cycles, the waits of all steps ~25 cycles a step and a longer
 // chain in the block: dense from p T = 1/40 on.
 //
@@ -1071,7 +1071,7 @@ __device__ __forceinline__ void take_steps(const KConst& k, const TrajState& st,
 // registers).  65536 trajectories, kernel ms: 29.3 with two pairs at once one
 // after the other and four steps between votes, 25.5 with the pairs together,
 // 23.9 with rows of noise (blocks of four steps, or a try of four before the
-// steps one by one: 24.1).
+// steps one by one: 24.1).  DENSE: see group mode above.
 constexpr int kOwnSteps = 32, kOwnDense = 16;
 template <bool DBL, bool OVER, bool ETA, bool DENSE>
 __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, const TrajState st, int64_t g0,
