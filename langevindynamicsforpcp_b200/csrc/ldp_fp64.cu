@@ -938,7 +938,7 @@ __device__ __forceinline__ bool dense_block(const KConst& k, Lane& a, bool want,
 }
 
 // Where a lane's run of steps stands besides its Lane: the next frame and its
-// place, and the first step not integrated.
+// place (null: no frames are kept), and the first step not integrated.
 struct Course {
     int64_t frame;
     double* px;
@@ -968,12 +968,13 @@ __device__ __forceinline__ void take_steps(const KConst& k, const TrajState& st,
     // special step with a new block, and its warp waits for it at the
     // buffer's end only.
     if (!(a.q & Q_RUN)) l = n;
-    // the places of the next frame and of the pending flip, and the last
-    // place a block can start at
-    int fr = k.fp_mode ? 1 << 30 : near(c.frame * (int64_t)k.freq_save - (int64_t)s0);
+    // the places of the next frame (beyond every buffer where none is kept:
+    // no frame is ever due, and save is not called) and of the pending flip,
+    // and the last place a block can start at
+    int fr = k.fp_mode || !c.px ? 1 << 30 : near(c.frame * (int64_t)k.freq_save - (int64_t)s0);
     int flip = near(a.nflip - (int64_t)s0);
     auto save = [&]() {
-        if (c.frame < k.nframe && c.px) {
+        if (c.frame < k.nframe) {   // the frame arrays hold nframe rows
             *c.px = a.t.x;
             if (k.write_x && st.fv) {   // the rest of WRITEX: fp64_series_kernel
                 c.px[st.fv - st.fx] = a.t.v;

@@ -110,3 +110,34 @@ def test_noalloc_rejects_too_many_trajectories_and_too_large_rings():
     st = L.lib().ldp_integrate_fp64_noalloc(C.byref(p), C.byref(o), 1, 1, 1, None, None, err, 256)
     assert st == 7
     assert b"a power of two from 16 to 256" in err.value
+
+
+@pytest.mark.parametrize("double,over,spl", [(0, 1, 0), (0, 0, 7001), (1, 1, 4099), (1, 0, 10_000)])
+def test_noalloc_without_frames(double, over, spl):
+    # d_frames_x = NULL: thousands of frame steps go by and none is stored;
+    # everything else equals the call with frames, within one launch and over
+    # several (that begin and end anywhere between two frames).  No memory is
+    # written beside the outputs: words around each stay as they were.
+    import torch
+    if double:
+        p = ldp.params_from_inp(os.path.join(GOLDEN, "CuIDB_double__2.0_7.2_m1.0_1.00e-05.inp"), ldp.MODEL_DOUBLE)
+        p.number_of_steps, p.freq_save, p.random_seed, p.waiting_time, p.write_x = 30_000, 20, 4321, 0, 0
+    else:
+        p = params(steps=30_000)
+    p.overdamped = over
+    lanes, ranks, job_id = 70, 2, 5
+    ref = noalloc(p, lanes, ranks, job_id)
+    n, guard = lanes * ranks * p.number_of_runs, 64
+    o = opts(lanes, ranks, job_id)
+    o.steps_per_launch = spl
+    bufs = [torch.full((guard + rows * n + guard,), -7, dtype=t, device="cuda")
+            for rows, t in ((L.NCOUNT, torch.int64), (L.NSUM, torch.float64), (1, torch.float64))]
+    err = C.create_string_buffer(256)
+    st = L.lib().ldp_integrate_fp64_noalloc(C.byref(p), C.byref(o), *(b[guard:].data_ptr() for b in bufs), None,
+                                            torch.cuda.current_stream().cuda_stream, err, 256)
+    assert st == 0, err.value.decode()
+    torch.cuda.synchronize()
+    for b, k in zip(bufs, ("counts", "sums", "x_final")):
+        h = b.cpu().numpy()
+        np.testing.assert_array_equal(h[guard:-guard].reshape(ref[k].shape), ref[k], err_msg=k)
+        assert (h[:guard] == -7).all() and (h[-guard:] == -7).all()
