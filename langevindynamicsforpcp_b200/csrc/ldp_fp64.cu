@@ -858,6 +858,7 @@ constexpr int kGrpTwoProducers = 4;   // ... of a CTA with TWO
 constexpr int kGrpSteps = 8;       // steps of a consumer's block (16: 5 % slower at 2 lanes a warp, 10 % faster at 1)
 constexpr int kGrpItems = 8;       // items (four steps of a trajectory) of a producer lane in a buffer (4: 219 ns)
 constexpr int kGrpBuffer = 256;    // steps of a buffer at most
+constexpr int kGrpShared = 200 << 10, kGrpTwoShared = 100 << 10;   // bytes of a CTA's buffers at most (TWO: two CTAs an SM)
 __device__ __forceinline__ void bar_sync(int id, int n) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
@@ -1291,7 +1292,11 @@ static int launch_group_t(const KConst& k, const TrajState& st, int64_t g0, uint
         kern = fp64_group_kernel<DBL, OVER, ETA, false, OVER>;
         if (ETA && dense) kern = fp64_group_kernel<DBL, OVER, ETA, ETA, OVER>;
     }
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // The limit is the kernel's, for all threads and contexts of the process,
+    // so it is set to the most that a launch of it takes: with a launch's own
+    // size here, another thread's smaller launch could lower it before this one.
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               OVER && two ? kGrpTwoShared : kGrpShared);
     if (e != cudaSuccess) return (int)e;
     kern<<<(unsigned)grid, 32 * (nc + P), smem, stream>>>(k, st, g0, s0, s1, nc, T, B);
     return (int)cudaGetLastError();
@@ -1314,7 +1319,7 @@ int launch_fp64_group(const KConst& k, const TrajState& st, int64_t g0, uint64_t
     const bool dense = k.eta && pmin >= 1.0 / 1024 && p * T > 1.0 / 40;
     const int P = two ? kGrpTwoProducers : kGrpProducers;
     int B = 8 * ((32 * P * kGrpItems * 4 / M + 7) / 8);
-    const int room = ((two ? 100 : 200) << 10) / (2 * M * (dense ? 12 : 8)) - 1;   // shared memory
+    const int room = (two ? kGrpTwoShared : kGrpShared) / (2 * M * (dense ? 12 : 8)) - 1;   // shared memory
     B = std::min(std::min(std::max(B, 16), kGrpBuffer), room / 8 * 8);
     const int sel = (k.dbl ? 4 : 0) | (k.over ? 2 : 0) | (k.eta ? 1 : 0);
     switch (sel) {
