@@ -311,21 +311,27 @@ int launch_msd(const double* frames, int64_t nframe, int64_t ntraj, const int64_
         if (G > 32) G = 32;
     }
     cudaError_t e;
+    // A kernel's shared-memory limit is the process's, whatever thread or
+    // context sets it: always the most a launch takes, never this launch's
+    // size, which could lower it before another thread's launch.
+    auto limit = [](auto* kern) {
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMsdSmemBytes);
+    };
     if (G >= 1 && nframe < (1 << 30) && nlag < (1 << 30)) {
         const size_t smem = (size_t)G * (size_t)per_traj;
         const int64_t nblk = (ntraj + G - 1) / G;
         if (lean) {
             auto* kern = msd_smem_f32_kernel<128, 2, 16, true>;
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            e = limit(kern);
             if (e != cudaSuccess) return (int)e;
             kern<<<(unsigned)nblk, 128, smem, s>>>(frames, (int)nframe, ntraj, G, lags, (int)nlag, msd0);
         } else if (f32) {
             auto* kern = msd_smem_f32_kernel<kMsdBlock, 6, 4, false>;
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            e = limit(kern);
             if (e != cudaSuccess) return (int)e;
             kern<<<(unsigned)nblk, kMsdBlock, smem, s>>>(frames, (int)nframe, ntraj, G, lags, (int)nlag, msd0);
         } else {
-            e = cudaFuncSetAttribute(msd_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            e = limit(msd_smem_kernel);
             if (e != cudaSuccess) return (int)e;
             msd_smem_kernel<<<(unsigned)nblk, kMsdBlock, smem, s>>>(frames, (int)nframe, ntraj, G, lags, (int)nlag,
                                                                    msd0);

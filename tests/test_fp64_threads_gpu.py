@@ -53,3 +53,50 @@ def test_two_threads_launch_one_kernel_with_other_shared_memory():
         for r in got[n]:
             for k in keys:
                 np.testing.assert_array_equal(r[k], alone[n][k], err_msg=f"{n} {k}")
+
+
+@pytest.mark.parametrize("precision", [ldp.PREC_FP64_PLAIN, ldp.PREC_FP32_BATCHED])
+def test_two_threads_launch_displacements_of_other_lengths(precision):
+    # The mean-square displacements' kernels hold trajectories of the job's
+    # frame count in shared memory: 1201 frames (94 KB a block in FP64, 5 KB
+    # a block for a batch's FP32 jobs) and 7001 (56 and 28 KB).
+    p = ldp.params_from_inp(os.path.join(GOLDEN, "quick_test__2.0_7.2_m1.0_1.00e-05.inp"))
+    p.tau, p.freq_save, p.write_x, p.write_restart, p.random_seed = 1.0, 1, 0, 0, 5
+
+    def run(c, steps, njobs):
+        p2 = type(p).from_buffer_copy(p)
+        p2.number_of_steps = steps
+        jobs = [ldp.Job(c, p2, lanes=3, job_id=2, precision=precision) for _ in range(njobs)]
+        try:
+            ldp.submit_batch(c, jobs)
+            return [j.wait().msd() for j in jobs]
+        finally:
+            for j in jobs:
+                j.close()
+
+    steps = (1200, 7000)
+    alone = {}
+    for m in steps:
+        with ldp.Context(0) as c:
+            alone[m] = run(c, m, 1)[0]
+    got, failed, start = {m: [] for m in steps}, [], threading.Barrier(len(steps))
+
+    def work(m):
+        try:
+            with ldp.Context(0) as c:
+                start.wait(60)
+                for _ in range(15):
+                    got[m] += run(c, m, 48)
+        except Exception as e:   # a refused launch, reported by the main thread
+            failed.append((m, e))
+
+    threads = [threading.Thread(target=work, args=(m,)) for m in steps]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+    for m in steps:
+        for lags, msd in got[m]:
+            np.testing.assert_array_equal(lags, alone[m][0])
+            np.testing.assert_array_equal(msd, alone[m][1])
