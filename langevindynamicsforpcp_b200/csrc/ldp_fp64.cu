@@ -1187,6 +1187,7 @@ __global__ void __launch_bounds__(32 * (kGrpConsumers + (TWO ? kGrpTwoProducers 
     const bool active = (a.q & Q_RUN) != 0u;
     Course c = course(k, st, i, s_begin, s_end);
     const int tl = t0 + (lane < T ? lane : 0);   // idle lanes read a lane's noise
+    __syncwarp();   // load_lane parts the lanes; the barriers want the warp together
     for (uint64_t b = 0; b < nblk; ++b) {
         const int u = (int)(b & 1);
         bar_sync(full + u, nthreads);                // buffer u full
