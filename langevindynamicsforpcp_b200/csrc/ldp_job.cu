@@ -8,7 +8,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -421,26 +420,6 @@ ldp_status ldp_job_create_unchecked(ldp_ctx* ctx, const ldp_params* p, const ldp
     return job_create(ctx, p, o, out, false);
 }
 
-// Whether `need` bytes of device memory are free.  The query is a driver call
-// that takes 0.02 to 10 ms (other processes' calls in its way: 16 jobs were
-// created in 1.3 to 79 ms), so a job that needs little of what a query in the
-// last two seconds found free, the jobs created since subtracted, is not
-// queried for.
-static bool fits(ldp_ctx* ctx, size_t need, size_t* free_b) {
-    const auto now = std::chrono::steady_clock::now();
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    if (need < ctx->free_left / 8 && now - ctx->free_when < std::chrono::seconds(2)) {
-        ctx->free_left -= need;
-        return true;
-    }
-    size_t total_b = 0;
-    *free_b = 0;
-    cudaMemGetInfo(free_b, &total_b);
-    ctx->free_when = now;
-    ctx->free_left = need <= *free_b ? *free_b - need : 0;
-    return need <= *free_b;
-}
-
 static ldp_status job_create(ldp_ctx* ctx, const ldp_params* p, const ldp_job_opts* o, ldp_job** out, bool check_mem) {
     if (!ctx || !p || !out) return LDP_ERR_INVALID;
     *out = nullptr;
@@ -497,8 +476,12 @@ static ldp_status job_create(ldp_ctx* ctx, const ldp_params* p, const ldp_job_op
 
     const size_t need = job_arena(job, false);
     cudaSetDevice(ctx->device);
-    size_t free_b = 0;
-    if (check_mem && !fits(ctx, need + ((size_t)256 << 20), &free_b)) {
+    // Asked anew for every job (0.02 ms, at times up to 10 ms where other
+    // processes' driver calls are in the way): other contexts, libraries and
+    // processes take device memory too, so an earlier answer tells nothing.
+    size_t free_b = 0, total_b = 0;
+    if (check_mem) cudaMemGetInfo(&free_b, &total_b);
+    if (check_mem && need + ((size_t)256 << 20) > free_b) {
         ldp_set_error(ctx, "job needs %.2f GB of device memory, %.2f GB free", need / 1e9, free_b / 1e9);
         delete job;
         return LDP_ERR_NOMEM;
