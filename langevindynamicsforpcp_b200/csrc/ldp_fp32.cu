@@ -50,6 +50,7 @@
 
 #include "ldp_device.cuh"
 #include "ldp_fp32.h"
+#include "ldp_share.h"
 
 namespace ldp {
 
@@ -1212,9 +1213,8 @@ __device__ __noinline__ void save_slot(const QueueDev* qp, const SlotsDev* Sp, R
 }
 
 // How a launch that finds fewer items than it has lanes shares them out
-// (avail: items unclaimed at the last publication): as few warps to each
-// scheduler of the GPU as hold them, all schedulers alike.  Returns the lanes
-// a warp fills at its first claim, 0 for a warp that leaves the items to
+// (avail: items unclaimed at the last publication), by share_out.  Returns the
+// lanes a warp fills at its first claim, 0 for a warp that leaves the items to
 // others, 32 where every lane is wanted.  (24000 steps, frames every 20, warps
 // filled one after the other / this way: 16000 trajectories 5.6 / 3.0 ms,
 // 32000 5.8 / 3.4, 60000 5.7 / 4.3 overdamped; 1024 2.5 / 1.9.  One warp to a
@@ -1226,17 +1226,15 @@ __device__ __noinline__ void save_slot(const QueueDev* qp, const SlotsDev* Sp, R
 // threads of the block call.
 __device__ __forceinline__ int first_claim(unsigned long long avail, const SlotsDev& S) {
     __shared__ unsigned rank;
-    const unsigned sms = (unsigned)S.sms, wpb = blockDim.x >> 5, schedulers = sms * 4;
-    if (avail == 0 || avail > (unsigned long long)gridDim.x * blockDim.x) return 32;
+    const unsigned sms = (unsigned)S.sms, wpb = blockDim.x >> 5, blocks = gridDim.x / sms;
+    const Share share = share_out(avail, sms, blocks * wpb);
+    if (share.lanes == 32 && share.warps == sms * blocks * wpb) return 32;
     unsigned smid;
     asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
     if (threadIdx.x == 0) rank = atomicAdd(&S.sm_rank[smid & (unsigned)(kSmRanks - 1)], 1u);
     __syncthreads();
-    const unsigned n = (unsigned)avail, k = (n + schedulers * 32 - 1) / (schedulers * 32);
-    const unsigned cap = min(32u, (n + schedulers * k - 1) / (schedulers * k));
-    const unsigned used = (n + cap - 1) / cap;   // warps that take cap items (the last one fewer)
-    const unsigned layer = rank % (gridDim.x / sms) * wpb + (threadIdx.x >> 5);
-    return layer * sms + smid % sms < used ? (int)cap : 0;
+    const unsigned layer = rank % blocks * wpb + (threadIdx.x >> 5);
+    return layer * sms + smid % sms < share.warps ? (int)share.lanes : 0;
 }
 
 // Warp-aggregated refill of the warp's idle lanes (all lanes call): the

@@ -1,0 +1,38 @@
+"""How persistent FP32 launches claim trajectories, where their number is
+bounded: a graph over a queue of few warps."""
+import os
+
+import numpy as np
+import pytest
+
+import langevindynamicsforpcp_b200 as ldp
+from langevindynamicsforpcp_b200 import _tune
+
+GOLDEN = os.path.join(os.path.dirname(__file__), "golden", "inp")
+pytestmark = pytest.mark.gpu
+KEYS = ("counts", "sums", "x_final", "state_final")
+
+
+def params(steps, freq):
+    p = ldp.params_from_inp(os.path.join(GOLDEN, "quick_test__2.0_7.2_m1.0_1.00e-05.inp"))
+    p.overdamped, p.tau, p.write_x, p.write_restart, p.random_seed = 1, 1e-2, 0, 0, 21
+    p.number_of_steps, p.freq_save = steps, freq
+    return p
+
+
+@pytest.mark.parametrize("block,n", [(32, 4736), (32, 1185), (64, 9472), (160, 23_680)])
+def test_graph_of_few_warps_ends_within_its_launches(block, n):
+    # Fewer warps (or fewer than the next multiple of four) to an SM than it
+    # has schedulers, as many trajectories as lanes and fewer: the graph's
+    # number of launches is a bound for slots that never idle beside
+    # unclaimed items.  (148 SMs; on others the sizes are other ones.)
+    p = params(4000, 3)
+    with ldp.Context(0) as c, ldp.Job(c, p, lanes=n, precision=ldp.PREC_FP32_BATCHED, job_id=3) as j:
+        alone = j.run().results(frames=False)
+    with ldp.Context(0) as c:
+        _tune.set_fp32_shape(c, block=block, blocks_per_sm=1, pair_budget=2048)
+        with ldp.Job(c, p, lanes=n, precision=ldp.PREC_FP32_BATCHED, job_id=3) as j:
+            ldp.submit_batch(c, [j], graph=True)
+            got = j.wait().results(frames=False)
+    for k in KEYS:
+        np.testing.assert_array_equal(got[k], alone[k], err_msg=k)
