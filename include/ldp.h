@@ -303,7 +303,12 @@ ldp_status  ldp_write_default_inp(const char *path, int model);
 
 /* Jobs.  Replaces LangevinEquationSIMDMultiple::Initialize/Integrate and the
  * trial loop of LangevinEquationRunnerMPI::Run
- * (src/langevinDynamicsSingleBarrier.h:1276, 1386, 3429-3589). */
+ * (src/langevinDynamicsSingleBarrier.h:1276, 1386, 3429-3589).
+ * ldp_job_create allocates no device memory; it refuses a job with
+ * LDP_ERR_NOMEM that the device cannot hold at that moment: neither the memory
+ * that earlier jobs of the process freed nor the device's free memory, 256 MB
+ * left over, is enough.  The memory itself is taken at submission, which
+ * returns LDP_ERR_NOMEM when other jobs or programs have taken it since. */
 void        ldp_job_opts_default(ldp_job_opts *o);
 ldp_status  ldp_job_create(ldp_ctx *ctx, const ldp_params *p,
                            const ldp_job_opts *o, ldp_job **out);

@@ -160,6 +160,7 @@ static int queue_init(ldp_ctx* ctx, Fp32Queue& Q, int type, int ring_slots) {
     Q.free_slots.clear();
     for (int i = kFp32MaxJobs - 1; i >= 0; --i) Q.free_slots.push_back(i);
     Q.ready = true;
+    ctx->fp32_ready |= 1u << type;
     return 0;
 }
 

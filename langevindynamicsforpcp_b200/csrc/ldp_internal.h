@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <mutex>
 #include <string>
@@ -37,6 +38,7 @@ struct ldp_ctx {
     int fp32_blocks_per_sm = 0;    // resident blocks per SM (0: default 4)
     uint64_t fp32_pair_budget = 0; // step pairs per slot per launch (0: default)
     int fp32_ring_slots = 0;       // cell-table ring slots per slot (0: default 64)
+    std::atomic<unsigned> fp32_ready{0};   // model types (bits) whose FP32 queue has its memory
     int64_t fp64_latency_max = kFp64LatencyMaxTraj;   // latency mode up to this many trajectories
     int64_t fp64_group_max = kFp64GroupMaxTraj;       // then group mode up to this many
     cudaStream_t side = nullptr;   // post-processing beside running batches (high priority)

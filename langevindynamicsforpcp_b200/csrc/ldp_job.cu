@@ -420,6 +420,29 @@ ldp_status ldp_job_create_unchecked(ldp_ctx* ctx, const ldp_params* p, const ldp
     return job_create(ctx, p, o, out, false);
 }
 
+// Whether `need` bytes of device memory are free now: a driver call of 0.02
+// ms, ten and more at times, where other processes' calls are in its way.
+// Asked anew each time: other contexts, libraries and processes take memory
+// too, so an earlier answer tells nothing.
+static bool device_holds(size_t need, size_t* free_b) {
+    size_t total_b = 0;
+    return cudaMemGetInfo(free_b, &total_b) == cudaSuccess && need <= *free_b;
+}
+
+// Whether the pool that the job's memory comes from holds `need` unused bytes
+// now, freed by earlier jobs: memory of this process that no other can take,
+// told without a call into the kernel driver.  (An FP32 job's queue has memory
+// of its own: it has to be there already.)
+static bool pool_holds(const ldp_job* job, size_t need) {
+    if (job->o.precision == LDP_PREC_FP32_BATCHED && !(job->ctx->fp32_ready >> fp32_type_of(job) & 1u)) return false;
+    cudaMemPool_t pool;
+    uint64_t reserved = 0, used = 0;
+    return cudaDeviceGetMemPool(&pool, job->ctx->device) == cudaSuccess &&
+           cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+           cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+           reserved >= used && reserved - used >= need;
+}
+
 static ldp_status job_create(ldp_ctx* ctx, const ldp_params* p, const ldp_job_opts* o, ldp_job** out, bool check_mem) {
     if (!ctx || !p || !out) return LDP_ERR_INVALID;
     *out = nullptr;
@@ -476,12 +499,8 @@ static ldp_status job_create(ldp_ctx* ctx, const ldp_params* p, const ldp_job_op
 
     const size_t need = job_arena(job, false);
     cudaSetDevice(ctx->device);
-    // Asked anew for every job (0.02 ms, at times up to 10 ms where other
-    // processes' driver calls are in the way): other contexts, libraries and
-    // processes take device memory too, so an earlier answer tells nothing.
-    size_t free_b = 0, total_b = 0;
-    if (check_mem) cudaMemGetInfo(&free_b, &total_b);
-    if (check_mem && need + ((size_t)256 << 20) > free_b) {
+    size_t free_b = 0;
+    if (check_mem && !pool_holds(job, need) && !device_holds(need + ((size_t)256 << 20), &free_b)) {
         ldp_set_error(ctx, "job needs %.2f GB of device memory, %.2f GB free", need / 1e9, free_b / 1e9);
         delete job;
         return LDP_ERR_NOMEM;
