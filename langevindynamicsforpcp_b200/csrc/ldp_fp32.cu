@@ -1240,7 +1240,7 @@ __device__ __forceinline__ int first_claim(unsigned long long avail, const Slots
 // Warp-aggregated refill of the warp's idle lanes (all lanes call): the
 // first `most` lanes with `need` claim trajectories from the queue.  Returns
 // whether the warp is done claiming: the queue had fewer than the lanes
-// wanted, or lanes were left out.
+// wanted.
 template <int K>
 __device__ __noinline__ bool refill(const QueueDev* qp, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
                                     bool need, int most) {
@@ -1251,7 +1251,7 @@ __device__ __noinline__ bool refill(const QueueDev* qp, const SlotsDev* Sp, Rare
     const unsigned all = __ballot_sync(kFull, need);
     need = need && __popc(all & ((1u << lane) - 1u)) < most;
     const unsigned m = __ballot_sync(kFull, need);
-    if (!m) return all != 0;
+    if (!m) return false;
     const int leader = __ffs(m) - 1;
     unsigned long long base = 0, got = 0;
     if ((int)lane == leader) {
@@ -1286,7 +1286,7 @@ __device__ __noinline__ bool refill(const QueueDev* qp, const SlotsDev* Sp, Rare
             idle_lane(sm, t);
         }
     }
-    return got < (unsigned long long)__popc(m) || m != all;
+    return got < (unsigned long long)__popc(m);
 }
 
 // The hot loop: blocks of four steps of the warp's lanes, from their state
@@ -1396,13 +1396,15 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
     constexpr int C = kMixed ? K_ANY : K;
     load_slot<C>(&q, &S, &sm, t, slot);
 
-    bool dry = false;   // the queue had nothing left for this warp
+    // Idle lanes look at the queue from block `look` on: kDry once it had
+    // nothing left for this warp.
+    constexpr uint32_t kDry = ~0u;
     int most = !kMixed ? first_claim(*q.avail, S) : 32;
-    uint32_t it = 0;
+    uint32_t it = 0, look = 0;
     while (it < quad_budget) {
         // lanes become idle in the slow path only
         if (__any_sync(kFull, sm.job[t] < 0)) {
-            const bool need = sm.job[t] < 0 && !dry && slot < S.nslots;
+            const bool need = sm.job[t] < 0 && it >= look && slot < S.nslots;
             const bool asked = __any_sync(kFull, need);
             if (asked) {
                 if (!kMixed && most == 0) {
@@ -1413,11 +1415,19 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
                         __nanosleep(20000);
                     most = 32;
                 }
-                if (refill<C>(&q, &S, &sm, t, slot, need, most)) dry = true;
+                // Lanes left out of the warp's share take what is still there
+                // once the other warps have had theirs (lanes of theirs may
+                // hold another job's trajectories): 64 blocks are 25-45 us.
+                if (refill<C>(&q, &S, &sm, t, slot, need, most)) look = kDry;
+                else if (!kMixed && most < 32) look = it + 64;
                 most = 32;
             }
             if (__all_sync(kFull, sm.job[t] < 0)) {
-                if (dry || !asked) {
+                if (!kMixed && it < look && look != kDry) {   // the share has ended already
+                    look = it;
+                    continue;
+                }
+                if (look == kDry || !asked) {
                     *drained = true;
                     break;
                 }
@@ -1433,8 +1443,9 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
         // warps of all types on one SM (mixed launches).
         constexpr bool kOnlyRolled = kMixed || (K & 2) != 0;
         const bool often = !kOnlyRolled && sm.job[t] >= 0 && q.jobs[sm.job[t]].flips_often != 0;
-        if (kOnlyRolled || __any_sync(kFull, often)) it += run_blocks<K, true>(q.jobs, &sm, t, quad_budget - it);
-        else it += run_blocks<K, kOnlyRolled>(q.jobs, &sm, t, quad_budget - it);
+        const uint32_t blocks = (!kMixed && it < look ? min(quad_budget, look) : quad_budget) - it;
+        if (kOnlyRolled || __any_sync(kFull, often)) it += run_blocks<K, true>(q.jobs, &sm, t, blocks);
+        else it += run_blocks<K, kOnlyRolled>(q.jobs, &sm, t, blocks);
         const uint32_t halt = sm.pw[t] / P_HALT;
         if (__any_sync(kFull, halt != 0)) {
             if (halt) {

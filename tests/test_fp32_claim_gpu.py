@@ -1,11 +1,12 @@
 """How persistent FP32 launches claim trajectories, where their number is
-bounded: a graph over a queue of few warps."""
+bounded: a graph over a queue of few warps, and a job beside another."""
 import os
 
 import numpy as np
 import pytest
 
 import langevindynamicsforpcp_b200 as ldp
+from langevindynamicsforpcp_b200 import _lib as L
 from langevindynamicsforpcp_b200 import _tune
 
 GOLDEN = os.path.join(os.path.dirname(__file__), "golden", "inp")
@@ -36,3 +37,33 @@ def test_graph_of_few_warps_ends_within_its_launches(block, n):
             got = j.wait().results(frames=False)
     for k in KEYS:
         np.testing.assert_array_equal(got[k], alone[k], err_msg=k)
+
+
+def test_one_launch_claims_all_beside_another_jobs_trajectories():
+    # A first-passage job's 5000 trajectories hold lanes here and there when
+    # 105000 more come, nearly as many as the idle lanes: the warps that fill
+    # only a share at first take the rest in the same launch, so the job runs
+    # in as many launches as it does alone.
+    p = params(4000, 3)
+    slow = params(4000, 3)
+    slow.tau, slow.barrier_heights[0][0], slow.barrier_heights[0][1] = 0.0, 80.0, 80.0   # no passage within the cap
+
+    def job(c):
+        return ldp.Job(c, p, lanes=105_000, precision=ldp.PREC_FP32_BATCHED, job_id=3)
+    out = []
+    for beside in (False, True):
+        with ldp.Context(0) as c:
+            _tune.set_fp32_shape(c, blocks_per_sm=3, pair_budget=2500)
+            other = ldp.Job(c, slow, lanes=5000, precision=ldp.PREC_FP32_BATCHED, job_id=4,
+                            mode=ldp.MODE_FIRST_PASSAGE, step_cap=40_000)
+            if beside:
+                other.submit()   # a launch or two of its eight
+            with job(c) as j:
+                r = j.submit().wait().results(frames=False)
+                out.append((j.timing()["launches"], r))
+            if beside:
+                assert (other.wait().results(frames=False)["counts"][L.C_STEPS] == 40_000).all()
+            other.close()
+    assert out[1][0] == out[0][0]
+    for k in KEYS:
+        np.testing.assert_array_equal(out[1][1][k], out[0][1][k], err_msg=k)
