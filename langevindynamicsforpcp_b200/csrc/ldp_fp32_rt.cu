@@ -127,7 +127,6 @@ static int queue_init(ldp_ctx* ctx, Fp32Queue& Q, int type, int ring_slots) {
     Q.grid = ctx->sm_count * blocks(false);
     Q.wide_grid = std::max(Q.grid, ctx->sm_count * blocks(true));
     Q.pair_budget = ctx->fp32_pair_budget ? ctx->fp32_pair_budget : (1u << 15);
-    const int64_t nslots = (int64_t)Q.wide_grid * Q.block;
     // queue + job table
     size_t qb = al256(sizeof(int64_t) * kFp32MaxRanges) * 2 + al256(sizeof(int32_t) * kFp32MaxRanges) +
                 al256(sizeof(unsigned long long) * 3) + al256(sizeof(int32_t)) + al256(sizeof(JobF) * kFp32MaxJobs) +
@@ -148,7 +147,14 @@ static int queue_init(ldp_ctx* ctx, Fp32Queue& Q, int type, int ring_slots) {
     Q.q.nranges = (int32_t*)(a + o); o += al256(sizeof(int32_t));
     Q.q.jobs = (JobF*)(a + o); o += al256(sizeof(JobF) * kFp32MaxJobs);
     Q.rem = (unsigned long long*)(a + o);
-    e = (cudaError_t)slots_init(nslots, ring_slots, ctx->sm_count, &Q.s, &Q.smem);
+    // Slots for the wide grid (168 MB at 64 ring entries; 126 MB for the narrow
+    // one), or for the narrow grid alone where the device cannot hold them.
+    e = (cudaError_t)slots_init((int64_t)Q.wide_grid * Q.block, ring_slots, ctx->sm_count, &Q.s, &Q.smem);
+    if (e == cudaErrorMemoryAllocation && Q.wide_grid > Q.grid) {
+        cudaGetLastError();
+        Q.wide_grid = Q.grid;
+        e = (cudaError_t)slots_init((int64_t)Q.grid * Q.block, ring_slots, ctx->sm_count, &Q.s, &Q.smem);
+    }
     if (e != cudaSuccess) return (int)e;
     e = cudaMallocHost((void**)&Q.h_stage, 4096 * Fp32Queue::kStageSlots);
     if (e != cudaSuccess) return (int)e;

@@ -10,6 +10,7 @@ import pytest
 
 import langevindynamicsforpcp_b200 as ldp
 from langevindynamicsforpcp_b200 import _lib as L
+from langevindynamicsforpcp_b200 import _tune
 
 GOLDEN = os.path.join(os.path.dirname(__file__), "golden", "inp")
 pytestmark = pytest.mark.gpu
@@ -66,9 +67,36 @@ def freed_by_an_earlier_job(precision):
         np.testing.assert_array_equal(after[k], before[k], err_msg=k)
 
 
+def no_room_for_the_slots_of_wide_launches(precision):
+    # 16384 ring entries a slot: the slots of three blocks to an SM take 30 GB,
+    # those of four 40 GB, and 36 GB are left.
+    import numpy as np
+    p = params(1200)
+    out = []
+    for ring in (0, 1 << 14):
+        with ldp.Context(0) as c:
+            held = None
+            if ring:
+                _tune.set_fp32_shape(c, ring_slots=ring)
+                held = take(36 << 30)
+            with ldp.Job(c, p, lanes=300, precision=precision, job_id=4) as j:
+                out.append(j.run().results(frames=False))
+            del held
+    for k in ("counts", "sums", "x_final"):
+        np.testing.assert_array_equal(out[1][k], out[0][k], err_msg=k)
+
+
 @pytest.mark.parametrize("precision", [ldp.PREC_FP64_PLAIN, ldp.PREC_FP32_BATCHED])
 @pytest.mark.parametrize("what", [taken_since_the_last_job, freed_by_an_earlier_job])
 def test_creation_counts_memory_as_it_is(what, precision):
+    in_a_process(what, precision)
+
+
+def test_slots_that_fit_are_used():
+    in_a_process(no_room_for_the_slots_of_wide_launches, ldp.PREC_FP32_BATCHED)
+
+
+def in_a_process(what, precision):
     c = mp.get_context("spawn").Process(target=what, args=(precision,))
     c.start()
     c.join(120)
