@@ -1,5 +1,6 @@
 """How persistent FP32 launches claim trajectories, where their number is
-bounded: a graph over a queue of few warps, and a job beside another."""
+bounded (a graph over a queue of few warps, a job beside another), and where
+they just fill the grid."""
 import os
 
 import numpy as np
@@ -67,3 +68,27 @@ def test_one_launch_claims_all_beside_another_jobs_trajectories():
     assert out[1][0] == out[0][0]
     for k in KEYS:
         np.testing.assert_array_equal(out[1][1][k], out[0][1][k], err_msg=k)
+
+
+def test_full_grids_and_one_trajectory_more():
+    # As many trajectories as a launch of three blocks to an SM has lanes (one
+    # trajectory each, launched alone), as one of four has, and one more than
+    # each: the last one then waits in the queue, or makes the launch a wider
+    # one.  All are prefixes of a run on one block to an SM, where nearly all
+    # trajectories wait.
+    p = params(1050, 1)
+    with ldp.Context(0) as c:
+        with ldp.Job(c, p, lanes=1, precision=ldp.PREC_FP32_BATCHED, job_id=3) as j:
+            j.run()
+        three = _tune.get_fp32_shape(c)["grid"] * 256
+        assert three % (3 * 256) == 0
+        four = three // 3 * 4
+        with ldp.Context(0) as c1:
+            _tune.set_fp32_shape(c1, blocks_per_sm=1)
+            with ldp.Job(c1, p, lanes=four + 1, precision=ldp.PREC_FP32_BATCHED, job_id=3) as j:
+                whole = j.run().results(frames=False)
+        for n in (three - 1, three, three + 1, four, four + 1):
+            with ldp.Job(c, p, lanes=n, precision=ldp.PREC_FP32_BATCHED, job_id=3) as j:
+                got = j.run().results(frames=False)
+            for k in KEYS:
+                np.testing.assert_array_equal(got[k], whole[k][..., :n], err_msg=f"{n} {k}")
