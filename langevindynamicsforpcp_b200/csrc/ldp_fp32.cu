@@ -281,8 +281,8 @@ __device__ __noinline__ void f_record_extra(bool DBL, const JobF* Jp, int64_t o,
     if (J.fst) J.fst[o] = (double)state;
 }
 
-__device__ __forceinline__ void f_record(const bool DBL, const JobF& J, uint32_t traj, int64_t frame, int cell, float xp, float v,
-                                         float F, int state) {
+__device__ __forceinline__ void f_record(const bool DBL, const JobF& J, uint32_t traj, int64_t frame, int cell,
+                                         float xp, float v, float F, int state) {
     if (frame >= J.nframe) return;   // the frame arrays hold nframe rows
     const int64_t o = frame * J.ntraj + traj;
     if (J.fx) J.fx[o] = (double)cell * J.Ld + (double)xp;
@@ -517,8 +517,8 @@ __device__ __noinline__ void f_end_lane(bool OVER, const JobF* Jp, const SlotsDe
 // The general step s of one lane (position already advanced):
 // the FP64 step order of ldp_fp64.cu from the index update on, on the lane
 // state in shared memory.
-__device__ __forceinline__ void general_step(const bool DBL, const bool OVER, const JobF* jobs, const SlotsDev* Sp, RareSm* smp, int t, int64_t slot,
-                                          uint64_t s) {
+__device__ __forceinline__ void general_step(const bool DBL, const bool OVER, const JobF* jobs, const SlotsDev* Sp,
+                                             RareSm* smp, int t, int64_t slot, uint64_t s) {
     RareSm& sm = *smp;
     const SlotsDev& S = *Sp;
     const float kInf = __int_as_float(0x7f800000);
@@ -868,7 +868,8 @@ __device__ __forceinline__ void flip_here(const bool DBL, const JobF& J, RareSm&
 // Leaves a pair: the lane state as general steps would have left it (the
 // ring entry of the cell first left, the transition-path clocks, and, in the
 // pair's other cell, the swapped barriers).
-__device__ __forceinline__ void unpair(const bool DBL, const JobF& J, const SlotsDev& S, RareSm& sm, int t, int64_t slot, uint32_t pw) {
+__device__ __forceinline__ void unpair(const bool DBL, const JobF& J, const SlotsDev& S, RareSm& sm, int t,
+                                       int64_t slot, uint32_t pw) {
     if (!(pw & P_CROSSED)) return;
     const int cell = sm.cell[t], sw = sm.sw[t];
     const int key = fkey(DBL, cell, sw & W_LB);
@@ -1049,7 +1050,8 @@ __device__ __forceinline__ bool quick_step(const bool DBL, const bool flips, con
 }
 
 // One step's move.
-__device__ __forceinline__ void f_move(const bool OVER, float& xp, float& rv, float F, float c1, float c2, float c3, float nz) {
+__device__ __forceinline__ void f_move(const bool OVER, float& xp, float& rv, float F, float c1, float c2, float c3,
+                                       float nz) {
     if (OVER) {
         xp = fmaf(F, c1, xp);
         xp = xp + nz;

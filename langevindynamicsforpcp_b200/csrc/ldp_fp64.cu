@@ -1,10 +1,12 @@
-// ldp_fp64.cu -- plain FP64 trajectory kernels (one trajectory per thread).
+// ldp_fp64.cu -- plain FP64 trajectory kernels: one trajectory per thread, and
+// group mode (few trajectories), whose stepping lanes other warps draw the
+// noise for.
 //
 // Device restatement of LangevinEquationSIMDMultiple and its overdamped
 // subclass (src/langevinDynamicsSingleBarrier.h:823-2888) and of the
 // double-barrier engine (src/langevinDynamicsDoubleBarrier.h:933-3507): the
-// per-lane SIMD loop becomes one CUDA thread per trajectory, the lane's
-// __m512d registers become this thread's registers, and the lazily grown
+// per-lane SIMD loop becomes one CUDA thread stepping each trajectory, the
+// lane's __m512d registers become this thread's registers, and the lazily grown
 // per-cell barrier table (src/DataLocator.h:100-188) becomes a tagged ring
 // of visited cells in HBM whose never-visited entries are a pure function of
 // (trajectory, cell).
@@ -842,15 +844,17 @@ __device__ __forceinline__ bool quiet_moves(const KConst& k, Lane& a, bool want,
 // DENSE: barriers flip so often that a lane could not draw its flips as they
 // come.  Producers (with one trajectory per thread, the thread) then also draw
 // the wait of a flip at every step for both states (its TAG_FLIP words, one
-// logarithm), in 16 bits: -ln(2^-64) / -ln(1 - p) < 2^16 for p >= 1/1024.  A flip drawn by the consumer costs its
-// warp ~1000 cycles, the waits of all steps ~25 cycles a step and a longer
-// chain in the block: dense from p T = 1/40 on.
+// logarithm), in 16 bits: -ln(2^-64) / -ln(1 - p) < 2^16 for p >= 1/1024.  A
+// flip drawn by the consumer costs its warp ~1000 cycles, the waits of all
+// steps ~25 cycles a step and a longer chain in the block: dense from
+// p T = 1/40 on.
 //
 // What it measured (ns a step; one CTA a trajectory, or of 32 trajectories,
 // with a producer warp or four, flips drawn for every step / this): the
-// sample input, 32 trajectories, p = 1/2: 62.3 / 39.2; 900 of two barriers:
-// 190 / 64; rare flips, 592: 91 / 45, 2000: 312 / 68, 5003 underdamped: 235 /
-// 56, 16000: 503 / 202.
+// sample input, 32 trajectories, p = 1/2, a frame in 80 steps: 62.7 / 38.1;
+// 900 of two barriers, a frame in 50: 199 / 61; rare flips, a frame in 20,
+// 592: 135 / 53, 2000: 481 / 68, 16000: 575 / 150; 5003 underdamped, a frame
+// in 30: 235 / 56.
 // ---------------------------------------------------------------------------
 constexpr int kGrpConsumers = 4;   // consumer warps of a CTA at most: one to a scheduler
 constexpr int kGrpProducers = 8;   // producer warps (4: 16000 trajectories 263 ns a step, 12: 197)
@@ -858,7 +862,8 @@ constexpr int kGrpTwoProducers = 4;   // ... of a CTA with TWO
 constexpr int kGrpSteps = 8;       // steps of a consumer's block (16: 5 % slower at 2 lanes a warp, 10 % faster at 1)
 constexpr int kGrpItems = 8;       // items (four steps of a trajectory) of a producer lane in a buffer (4: 219 ns)
 constexpr int kGrpBuffer = 256;    // steps of a buffer at most
-constexpr int kGrpShared = 200 << 10, kGrpTwoShared = 100 << 10;   // bytes of a CTA's buffers at most (TWO: two CTAs an SM)
+constexpr int kGrpShared = 200 << 10;      // bytes of a CTA's buffers at most
+constexpr int kGrpTwoShared = 100 << 10;   // ... with TWO (two CTAs an SM)
 __device__ __forceinline__ void bar_sync(int id, int n) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
@@ -1097,7 +1102,8 @@ __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, cons
 #pragma unroll 1
         for (int m = 0; m < n; m += 8) {
             const uint64_t q = (s0 + (uint64_t)m - 1) >> 2;
-            const Words w = philox_at(q, g, TAG_STEP, k.key0, k.key1), w2 = philox_at(q + 1, g, TAG_STEP, k.key0, k.key1);
+            const Words w = philox_at(q, g, TAG_STEP, k.key0, k.key1);
+            const Words w2 = philox_at(q + 1, g, TAG_STEP, k.key0, k.key1);
             const uint32_t wa[4] = {w.w0, w.w2, w2.w0, w2.w2}, wb[4] = {w.w1, w.w3, w2.w1, w2.w3};
             double r[8];
             gauss_pairs_f64(wa, wb, r);
@@ -1124,8 +1130,9 @@ __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, cons
 }
 
 template <bool DBL, bool OVER, bool ETA, bool DENSE, bool TWO>
-__global__ void __launch_bounds__(32 * (kGrpConsumers + (TWO ? kGrpTwoProducers : kGrpProducers)), TWO ? 2 : 1) fp64_group_kernel(const KConst k, const TrajState st, int64_t g0,
-                                                            uint64_t s_begin, uint64_t s_end, int nc, int T, int B) {
+__global__ void __launch_bounds__(32 * (kGrpConsumers + (TWO ? kGrpTwoProducers : kGrpProducers)), TWO ? 2 : 1)
+    fp64_group_kernel(const KConst k, const TrajState st, int64_t g0, uint64_t s_begin, uint64_t s_end, int nc, int T,
+                      int B) {
     // noise [2][M][R], then with DENSE waits [2][M][R]; rows of an odd length,
     // so that lanes at the same step are in different banks
     extern __shared__ double buf[];
@@ -1230,7 +1237,8 @@ __global__ void __launch_bounds__(256) fp64_series_kernel(const KConst k, const 
 
 int launch_fp64_series(const KConst& k, const TrajState& st, uint64_t s_begin, uint64_t s_end, int sms, void* stream) {
     const int64_t fs = (int64_t)k.freq_save;
-    const int64_t f0 = ((int64_t)s_begin + fs - 1) / fs, f1 = std::min<int64_t>(k.nframe, ((int64_t)s_end - 1) / fs + 1);
+    const int64_t f0 = ((int64_t)s_begin + fs - 1) / fs;
+    const int64_t f1 = std::min<int64_t>(k.nframe, ((int64_t)s_end - 1) / fs + 1);
     if (!k.write_x || !st.fx || !st.fv || f1 <= f0 || st.n <= 0) return 0;
     const int64_t blocks = std::min<int64_t>(((f1 - f0) * st.n + 255) / 256, (int64_t)8 * sms);
     if (k.dbl) fp64_series_kernel<true><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(k, st, f0, f1);

@@ -19,9 +19,15 @@ constexpr int kCtxF64Streams = 2;   // streams FP64 plain jobs of a batch share
 // FP64 plain fixed-step jobs of at most this many trajectories run in
 // latency mode by default, jobs above that and up to kFp64GroupMaxTraj in
 // group mode (launch_fp64_group with at least 1 and 8 lanes a warp), larger
-// ones one trajectory per thread: a stepping warp to each scheduler is full
-// at 18944 trajectories, where one per thread is as fast (16000 trajectories
-// with rare flips: 202 ns a step in group mode; 32000 per thread: 373).
+// ones one trajectory per thread.  The limit suits underdamped steps and
+// frequent flips, whose one stepping warp a scheduler is full at 18944
+// trajectories; overdamped ones with rare flips have two and gain up to 37888
+// (not used).  Group mode / one per thread, ns a step, a frame every 20:
+//                                   16384      20000      32000      37888
+//   underdamped, rare flips       101 / 167  215 / 210  218 / 212  220 / 213
+//   overdamped, flips at p = 0.01 322 / 425  708 / 473  714 / 483  715 / 485
+//   overdamped, rare flips        149 / 255  172 / 289  240 / 300  266 / 303
+//   two barriers, rare flips      167 / 293  192 / 330  264 / 338  292 / 344
 constexpr int64_t kFp64LatencyMaxTraj = 2048;
 constexpr int64_t kFp64GroupMaxTraj = 16384;
 
