@@ -222,6 +222,10 @@ __device__ __forceinline__ float force_of(const bool DBL, const JobF& J, float x
     }
 }
 
+// force_of where no flank is: its zero's sign is the model's (a saved frame of
+// WRITEX shows it).
+__device__ __forceinline__ float flat_force(const bool DBL) { return DBL ? -0.0f : 0.0f; }
+
 // Open band (lo, hi) of consecutive breakpoints around xp; lo = hi = xp when
 // xp sits on a breakpoint, so that the next step takes the general path.
 // Single barrier: the breakpoints are -L/2, -w, 0, w (clamped to the cell).
@@ -951,7 +955,7 @@ __device__ __noinline__ void special_step(const JobF* jobs, const SlotsDev* Sp, 
             sm.xp[t] = xn;
             sm.lo[t] = e1;
             sm.hi[t] = e2;
-            sm.F[t] = 0.f;
+            sm.F[t] = flat_force(DBL);
             settle(DBL, &J, &sm, t, s, xn);
             return;
         }
@@ -1045,7 +1049,7 @@ __device__ __forceinline__ bool quick_step(const bool DBL, const bool flips, con
     xp = xn;
     lo = e1;
     hi = e2;
-    F = 0.0f;
+    F = flat_force(DBL);
     return true;
 }
 

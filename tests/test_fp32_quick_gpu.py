@@ -164,3 +164,19 @@ def test_launches_of_four_blocks_to_an_sm(graph):
     for a, b in zip(three, outcome(0)[0]):
         for k in a:
             np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+
+
+@pytest.mark.parametrize("kind", ["single_over", "single_under", "double_over", "double_under"])
+@pytest.mark.parametrize("tau", [1e-3, 1.0])
+def test_saved_forces_after_quick_steps_to_the_bit(kind, tau):
+    # The force of a frame after a crossing taken as a quick step is that of
+    # the general step, the sign of its zero included: the double barrier's
+    # is negative where there is no flank.
+    whole = run(params(kind, 9001, write_x=1, tau=tau, freq_save=5), 333)
+    short = run(params(kind, 9001, write_x=1, tau=tau, freq_save=5), 333, budget=2)
+    series = [k for k in whole if k.startswith("frames")]
+    assert len(series) == 7
+    for k in series:
+        np.testing.assert_array_equal(whole[k].view(np.int64), short[k].view(np.int64), err_msg=k)
+    f = whole["frames_f"]
+    assert (f == 0).any() and (np.signbit(f[f == 0]) == kind.startswith("double")).all()
