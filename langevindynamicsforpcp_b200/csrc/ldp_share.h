@@ -17,20 +17,19 @@ struct Share {
 };
 
 // avail unclaimed items over `sms` SMs of `wps` warps each: as few warps to
-// each scheduler (four to an SM) as hold the items, all schedulers alike.
-// Every warp and every lane where there are more items than lanes, and where
-// the launch has fewer warps than that takes (shapes of fewer warps to an SM
-// than schedulers): warps that each fill their share only would leave items
-// unclaimed beside idle lanes, and a batch's or graph's number of launches is
-// bounded for slots that never idle while items remain (fp32_launch_bound).
+// each scheduler (four to an SM) as hold the items, all schedulers alike; all
+// warps alike where the launch has fewer than that.  The shares hold every
+// item: warps that left some unclaimed beside idle lanes would break the bound
+// on a batch's or graph's launches (fp32_launch_bound), which counts on slots
+// that never idle while items remain.  Every warp and every lane where there
+// are more items than lanes.
 LDP_SHARE_FN Share share_out(unsigned long long avail, unsigned sms, unsigned wps) {
     const unsigned warps = sms * wps, schedulers = sms * 4;
-    const Share all{warps, 32};
-    if (avail == 0 || avail > (unsigned long long)warps * 32) return all;
+    if (avail == 0 || avail > (unsigned long long)warps * 32) return Share{warps, 32};
     const unsigned n = (unsigned)avail, k = (n + schedulers * 32 - 1) / (schedulers * 32);
-    const unsigned lanes = (n + schedulers * k - 1) / (schedulers * k);   // at most 32
-    const unsigned used = (n + lanes - 1) / lanes;                        // the last one fills fewer
-    return used > warps ? all : Share{used, lanes};
+    const unsigned share = schedulers * k < warps ? schedulers * k : warps;
+    const unsigned lanes = (n + share - 1) / share;        // at most 32
+    return Share{(n + lanes - 1) / lanes, lanes};          // the last one fills fewer
 }
 
 }  // namespace ldp
