@@ -818,7 +818,7 @@ __device__ __noinline__ void settle(bool DBL, const JobF* Jp, RareSm* smp, int t
     const long long wrap = block_wrap(s);
     nev = wrap < nev ? wrap : nev;
     if ((s & ((1ull << 34) - 1)) == 0) bind_block(J, sm, t, s);   // a new high word from the next step on
-    if (J.edge_flat && J.eta && (sw & W_CVALID) && !(sw & W_EVICT)) {
+    if (J.edge_flat && (sw & W_CVALID) && !(sw & W_EVICT)) {
         const bool right = !(xp < 0.0f);
         const int lb = sw & W_LB;
         const int well = cell - (right ? 0 : 1);

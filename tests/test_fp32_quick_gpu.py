@@ -180,3 +180,13 @@ def test_saved_forces_after_quick_steps_to_the_bit(kind, tau):
         np.testing.assert_array_equal(whole[k].view(np.int64), short[k].view(np.int64), err_msg=k)
     f = whole["frames_f"]
     assert (f == 0).any() and (np.signbit(f[f == 0]) == kind.startswith("double")).all()
+
+
+@pytest.mark.parametrize("kind", ["single_over", "single_under", "double_over", "double_under"])
+def test_pairs_of_barriers_that_never_flip(kind):
+    # TAU 0: crossings back and forth over a cell edge are quick steps too.
+    whole = run(params(kind, 9001, tau=0.0), 333)
+    for other in (run(params(kind, 9001, tau=0.0), 333, budget=2), run(params(kind, 9001, tau=0.0, write_x=1), 333)):
+        for k in whole:
+            np.testing.assert_array_equal(other[k], whole[k], err_msg=k)
+    assert (np.diff(np.sign(whole["frames_x"][1:] - whole["frames_x"][0]), axis=0) != 0).any()
