@@ -48,6 +48,8 @@
 // one fetch-and-add per warp and a ballot/popc prefix.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "ldp_device.cuh"
 #include "ldp_fp32.h"
 #include "ldp_share.h"
@@ -68,8 +70,9 @@ enum : int32_t { W_LB = 1, W_EVICT = 2, W_CVALID = 4, W_CSTATE = 8 };
 
 // Model type K: 0-3 (double * 2 + overdamped), or 4, the job's, for code
 // that serves all four; plus K_WIDE in the wide kernels (their own copies of
-// the out-of-line parts, compiled for fewer registers).
-constexpr int K_ANY = 4, K_WIDE = 8;
+// the out-of-line parts, compiled for fewer registers) and K_FULL in the
+// kernels for jobs of every mode (the others serve M_RARE and M_FLIPS).
+constexpr int K_ANY = 4, K_WIDE = 8, K_FULL = 16;
 template <int K>
 __device__ __forceinline__ bool is_double(const JobF& J) { return (K & K_ANY) ? J.dbl != 0 : (K & 2) != 0; }
 template <int K>
@@ -81,10 +84,11 @@ __device__ __forceinline__ bool is_over(const JobF& J) { return (K & K_ANY) ? J.
 // cross quickly; it is in the pair's other cell now; the other cell is the
 // right neighbour; the two barriers' states; the countdown ends at a frame
 // and nothing else; the pair's edge was crossed at least once; the other
-// cell's pending flip has come.
+// cell's pending flip has come.  Then the step of a block that needs the slow
+// path, one more than its place (three bits), and the job's mode (M_*).
 enum : uint32_t {
     P_FAST = 1, P_PAIR = 2, P_SWAP = 4, P_RIGHT = 8, P_S0 = 16, P_S1 = 32, P_FRAME = 64, P_CROSSED = 128,
-    P_OVERDUE = 256, P_HALT = 512
+    P_OVERDUE = 256, P_HALT = 512, P_HALTS = 7 * P_HALT, P_MODE = 1u << 16
 };
 
 // Per-thread rare state, structure of arrays (conflict-free by thread).
@@ -114,6 +118,7 @@ struct RareSm {
     long long nev[kMaxBlock];     // first step that is special for another reason than a frame
     long long xs[kMaxBlock];      // step of the last quick crossing
     uint32_t j[kMaxBlock], jh[kMaxBlock];   // next block of four steps, 4j+1 .. 4j+4: j's low and high word
+    const SlotsDev* slots;        // the launch's slots
 };
 static_assert(sizeof(RareSm) <= 55 * 1024, "four blocks to an SM");
 
@@ -273,8 +278,8 @@ __device__ __forceinline__ void f_energy(const bool DBL, const JobF& J, double x
 }
 
 // WRITEX frame fields (velocity, force, barrier, energies, state).
-__device__ __noinline__ void f_record_extra(bool DBL, const JobF* Jp, int64_t o, float xp, float v, float F, int state) {
-    const JobF& J = *Jp;
+__device__ __forceinline__ void record_extra(const bool DBL, const JobF& J, int64_t o, float xp, float v, float F,
+                                             int state) {
     double E, B;
     f_energy(DBL, J, (double)xp, state, &E, &B);
     if (J.fv) J.fv[o] = (double)v;
@@ -283,6 +288,9 @@ __device__ __noinline__ void f_record_extra(bool DBL, const JobF* Jp, int64_t o,
     if (J.fpe) J.fpe[o] = E;
     if (J.fke) J.fke[o] = J.mhalf * ((double)v * (double)v);
     if (J.fst) J.fst[o] = (double)state;
+}
+__device__ __noinline__ void f_record_extra(bool DBL, const JobF* Jp, int64_t o, float xp, float v, float F, int state) {
+    record_extra(DBL, *Jp, o, xp, v, F, state);
 }
 
 __device__ __forceinline__ void f_record(const bool DBL, const JobF& J, uint32_t traj, int64_t frame, int cell,
@@ -813,12 +821,12 @@ __device__ __noinline__ void settle(bool DBL, const JobF* Jp, RareSm* smp, int t
     const JobF& J = *Jp;
     RareSm& sm = *smp;
     const int state = sm.state[t], sw = sm.sw[t], cell = sm.cell[t];
-    uint32_t pw = (state ? P_S0 : 0u) | (J.edge_flat ? P_FAST : 0u);
+    uint32_t pw = (state ? P_S0 : 0u) | (J.edge_flat ? P_FAST : 0u) | P_MODE * (uint32_t)J.mode;
     long long nev = sm.nflip[t] < (long long)J.nsteps ? sm.nflip[t] : (long long)J.nsteps;
     const long long wrap = block_wrap(s);
     nev = wrap < nev ? wrap : nev;
     if ((s & ((1ull << 34) - 1)) == 0) bind_block(J, sm, t, s);   // a new high word from the next step on
-    if (J.edge_flat && (sw & W_CVALID) && !(sw & W_EVICT)) {
+    if ((sw & W_CVALID) && !(sw & W_EVICT)) {
         const bool right = !(xp < 0.0f);
         const int lb = sw & W_LB;
         const int well = cell - (right ? 0 : 1);
@@ -847,7 +855,7 @@ __device__ __noinline__ void settle(bool DBL, const JobF* Jp, RareSm* smp, int t
 // pair's first cell: its new state and pending flip, the state-1 run, the
 // force, the countdown; a pair stays one.
 __device__ __forceinline__ bool only_flip(const JobF& J, const RareSm& sm, int t, uint64_t s, uint32_t pw) {
-    return (pw & P_FAST) && !(pw & P_CROSSED) && (long long)s == sm.nflip[t] && (long long)s < sm.nxf[t] &&
+    return !(pw & P_CROSSED) && (long long)s == sm.nflip[t] && (long long)s < sm.nxf[t] &&
            s < J.nsteps && (s & ((1ull << 34) - 1)) != 0;
 }
 __device__ __forceinline__ void flip_here(const bool DBL, const JobF& J, RareSm& sm, int t, uint64_t s, float xp,
@@ -898,6 +906,18 @@ __device__ __forceinline__ void unpair(const bool DBL, const JobF& J, const Slot
     }
 }
 
+// Leaves a pair's crossings behind: unpair, and the word of the same pair seen
+// from the cell the lane is in.
+__device__ __forceinline__ void from_here(const bool DBL, const JobF& J, const SlotsDev& S, RareSm& sm, int t,
+                                          int64_t slot, uint32_t& pw) {
+    unpair(DBL, J, S, sm, t, slot, pw);
+    if (pw & P_SWAP) {   // the lane's cell is its pair's first now
+        pw ^= P_RIGHT;
+        if (((pw & P_S0) != 0u) != ((pw & P_S1) != 0u)) pw ^= P_S0 | P_S1;
+    }
+    pw &= ~(P_SWAP | P_CROSSED);
+}
+
 // A special step that is not a quick one: out of line, on the lane state in
 // shared memory, so that the hot loop's registers do not carry its working
 // set.  sm.left: 0 when the countdown ends at s.
@@ -914,12 +934,7 @@ __device__ __noinline__ void special_step(const JobF* jobs, const SlotsDev* Sp, 
     const JobF& J = jobs[job];
     const bool DBL = is_double<K>(J), OVER = is_over<K>(J);
     uint32_t pw = sm.pw[t];
-    unpair(DBL, J, S, sm, t, slot, pw);
-    if (pw & P_SWAP) {   // the lane's cell is its pair's first now
-        pw ^= P_RIGHT;
-        if (((pw & P_S0) != 0u) != ((pw & P_S1) != 0u)) pw ^= P_S0 | P_S1;
-    }
-    pw &= ~(P_SWAP | P_CROSSED);
+    from_here(DBL, J, S, sm, t, slot, pw);
     const float xp = sm.xp[t], lo = sm.lo[t], hi = sm.hi[t];
     if (sm.left[t] == 0 && xp > lo && xp < hi && only_flip(J, sm, t, s, pw)) {
         float F;
@@ -937,7 +952,7 @@ __device__ __noinline__ void special_step(const JobF* jobs, const SlotsDev* Sp, 
         const bool right = (pw & P_RIGHT) != 0u;
         const float xn = right ? xp - J.L : xp + J.L;
         const float e1 = right ? -J.halfL : J.edge_hi, e2 = right ? J.edge_lo : J.halfL;
-        if (xn > e1 && xn < e2) {
+        if (xn > e1 && xn < e2) {   // (no breakpoint between the edge and edge_lo or edge_hi)
             const int st = sm.state[t];
             const uint32_t g = sm.traj[t] + J.g0;
             long long nf;
@@ -955,7 +970,7 @@ __device__ __noinline__ void special_step(const JobF* jobs, const SlotsDev* Sp, 
             sm.xp[t] = xn;
             sm.lo[t] = e1;
             sm.hi[t] = e2;
-            sm.F[t] = flat_force(DBL);
+            sm.F[t] = J.edge_flat ? flat_force(DBL) : force_of(DBL, J, xn, now);
             settle(DBL, &J, &sm, t, s, xn);
             return;
         }
@@ -963,6 +978,22 @@ __device__ __noinline__ void special_step(const JobF* jobs, const SlotsDev* Sp, 
     general_step(DBL, OVER, jobs, Sp, smp, t, slot, s);
     if (sm.job[t] < 0) return;
     settle(DBL, &J, &sm, t, s, sm.xp[t]);
+}
+
+// The frame of step s, at which the countdown ends for it and nothing else
+// (P_FRAME).
+__device__ __forceinline__ void only_frame(const JobF& J, RareSm& sm, int t, uint64_t s, float xp, int& left,
+                                           uint32_t& pw) {
+    const int fidx = sm.fidx[t];
+    int cell = sm.cell[t];
+    if (pw & P_SWAP) cell += (pw & P_RIGHT) ? 1 : -1;
+    if (fidx < J.nframe && J.fx) J.fx[(int64_t)fidx * J.ntraj + sm.traj[t]] = (double)cell * J.Ld + (double)xp;
+    sm.fidx[t] = fidx + 1;
+    const long long nxf = sm.nxf[t] + (long long)J.freq_save, nev = sm.nev[t];
+    sm.nxf[t] = nxf;
+    const long long d = (nxf < nev ? nxf : nev) - (long long)s;
+    if (!(nxf < nev && d <= (long long)kLeftMax)) pw &= ~P_FRAME;
+    left = (int)(d < (long long)kLeftMax ? d : (long long)kLeftMax);
 }
 
 // The quick steps: the commonest special steps, in the hot loop, with the
@@ -998,16 +1029,7 @@ __device__ __forceinline__ bool quick_step(const bool DBL, const bool flips, con
             count_down(J, sm, t, s, nev, left, pw);
             return true;
         }
-        const int fidx = sm.fidx[t];
-        int cell = sm.cell[t];
-        if (swapped) cell += (pw & P_RIGHT) ? 1 : -1;
-        if (fidx < J.nframe && J.fx) J.fx[(int64_t)fidx * J.ntraj + sm.traj[t]] = (double)cell * J.Ld + (double)xp;
-        sm.fidx[t] = fidx + 1;
-        const long long nxf = sm.nxf[t] + (long long)J.freq_save, nev = sm.nev[t];
-        sm.nxf[t] = nxf;
-        const long long d = (nxf < nev ? nxf : nev) - (long long)s;
-        if (!(nxf < nev && d <= (long long)kLeftMax)) pw &= ~P_FRAME;
-        left = (int)(d < (long long)kLeftMax ? d : (long long)kLeftMax);
+        only_frame(J, sm, t, s, xp, left, pw);
         return true;
     }
     if (!(pw & P_FAST)) return false;
@@ -1050,6 +1072,125 @@ __device__ __forceinline__ bool quick_step(const bool DBL, const bool flips, con
     lo = e1;
     hi = e2;
     F = flat_force(DBL);
+    return true;
+}
+
+// The quick steps of jobs whose other special steps are frequent too (JobF::
+// full): those of quick_step, flips of the current barrier in every position
+// of a pair, crossings into a barrier whose pending flip has passed, frames with
+// the series of WRITEX, and all of these at the same step.  The step order is
+// the general step's: position and cell, flip, cell entry, force, frame.  Returns
+// false, and has done nothing, when the step needs special_step.
+template <bool DBL, bool OVER>
+__device__ __forceinline__ bool full_quick_step(const JobF& J, const SlotsDev& S, RareSm& sm, int t, uint64_t s,
+                                                bool countdown, float& xp, float rv, float& lo, float& hi, float& F,
+                                                int& left, uint32_t& pw) {
+    const bool in = xp > lo && xp < hi;
+    const bool frame = countdown && (pw & P_FRAME) != 0u;   // and nothing else
+    if (in && frame) {
+        only_frame(J, sm, t, s, xp, left, pw);
+        return true;
+    }
+    if (in && countdown && !frame && only_flip(J, sm, t, s, pw)) {
+        flip_here(DBL, J, sm, t, s, xp, F, left, pw);
+        return true;
+    }
+    const bool other = countdown && !frame;   // a flip, a barrier's pending flip, the last step ...
+    if (other && (s == J.nsteps || (s & ((1ull << 34) - 1)) == 0)) return false;
+    float xn = xp, l2 = lo, h2 = hi;
+    bool cross = false;
+    if (!in) {
+        const float hL = J.halfL;
+        if (fabsf(xp) < hL) {
+            if ((xp < 0.0f) != (lo < 0.0f)) return false;
+            if (DBL && (xp < J.xc) != (lo < J.xc)) return false;   // lo < xc: local barrier 0
+        } else {
+            if (!(pw & P_PAIR)) return false;
+            // the pair's other cell is the right neighbour
+            const bool right = ((pw & P_RIGHT) != 0u) != ((pw & P_SWAP) != 0u);
+            xn = right ? xp - J.L : xp + J.L;
+            if (!(right ? xp >= hL && xn > -hL && xn < J.edge_lo : xp < -hL && xn < hL && xn > J.edge_hi)) return false;
+            cross = true;
+        }
+        band_of(DBL, J, xn, &l2, &h2);
+        if (!(xn > l2 && xn < h2)) return false;
+    }
+    bool flip = false;
+    if (other) {
+        const long long a = sm.nflip[t], b = sm.cflip[t];
+        const bool swapped = (pw & P_SWAP) != 0u;
+        flip = (swapped ? b : a) == (long long)s;
+        if ((pw & P_PAIR) && (swapped ? a : b) == (long long)s) pw |= P_OVERDUE;
+    }
+    const bool overdue = cross && (pw & P_OVERDUE);
+    if (flip || overdue) {
+        const int64_t slot = (int64_t)blockIdx.x * blockDim.x + t;
+        from_here(DBL, J, S, sm, t, slot, pw);
+        const uint32_t g = sm.traj[t] + J.g0;
+        const Words w = philox_at(s, g, TAG_FLIP, J.key0, J.key1);
+        // the state-1 run of the lane's barrier
+        auto state_now = [&](int st) {
+            if (st) sm.since[t] = (long long)s;
+            else sm.sc1[t] += (long long)s - sm.since[t];
+        };
+        if (flip) {
+            pw ^= P_S0;
+            const int st = (pw & P_S0) ? 1 : 0;
+            sm.state[t] = st;
+            sm.nflip[t] = flip_schedule(s, w.w0, w.w1, J.ln1m[st]);
+            state_now(st);
+        }
+        if (overdue) {
+            long long nf;
+            const int st = caught_up(J, g, s, sm.cflip[t], (pw & P_S1) ? 0 : 1, w, &nf);
+            if (st != ((pw & P_S0) ? 1 : 0)) state_now(st);
+            sm.cflip[t] = nf;
+            sm.xs[t] = (long long)s;
+            pw = (pw & ~(P_S1 | P_OVERDUE)) | P_CROSSED | P_SWAP | (st ? P_S1 : 0u);
+            from_here(DBL, J, S, sm, t, slot, pw);   // into the cell entered
+        }
+    }
+    if (cross && !overdue) {
+        pw = (pw ^ P_SWAP) | P_CROSSED;
+        sm.xs[t] = (long long)s;
+        if (((pw & P_S0) != 0u) != ((pw & P_S1) != 0u)) {
+            if ((pw & P_SWAP) ? pw & P_S1 : pw & P_S0) sm.since[t] = (long long)s;
+            else sm.sc1[t] += (long long)s - sm.since[t];
+        }
+    }
+    const int st = ((pw & P_SWAP) ? pw & P_S1 : pw & P_S0) ? 1 : 0;
+    if (!in || flip) F = force_of(DBL, J, xn, st);
+    xp = xn;
+    lo = l2;
+    hi = h2;
+    if (frame && !overdue) {
+        only_frame(J, sm, t, s, xp, left, pw);
+        return true;
+    }
+    if (countdown && (long long)s == sm.nxf[t]) {
+        const int fidx = sm.fidx[t];
+        if (fidx < J.nframe) {
+            int cell = sm.cell[t];
+            if (pw & P_SWAP) cell += (pw & P_RIGHT) ? 1 : -1;
+            const int64_t o = (int64_t)fidx * J.ntraj + sm.traj[t];
+            if (J.fx) J.fx[o] = (double)cell * J.Ld + (double)xp;
+            if (J.write_x) record_extra(DBL, J, o, xp, OVER ? 0.0f : fmaf(F, J.hdt_invM, rv), F, st);
+        }
+        sm.fidx[t] = fidx + 1;
+        sm.nxf[t] += (long long)J.freq_save;
+    }
+    if (countdown || overdue) {
+        const long long a = sm.nflip[t], b = sm.cflip[t];
+        const bool swapped = (pw & P_SWAP) != 0u;
+        const long long own = swapped ? b : a, other = swapped ? a : b;
+        long long nev = block_wrap(s);
+        nev = (long long)J.nsteps < nev ? (long long)J.nsteps : nev;
+        nev = own < nev ? own : nev;
+        if (other <= (long long)s) pw |= P_OVERDUE;
+        if ((pw & (P_PAIR | P_OVERDUE)) == P_PAIR) nev = other < nev ? other : nev;
+        pw &= ~P_FRAME;
+        count_down(J, sm, t, s, nev, left, pw);
+    }
     return true;
 }
 
@@ -1299,8 +1440,9 @@ __device__ __noinline__ bool refill(const QueueDev* qp, const SlotsDev* Sp, Rare
 // in sm and back, until a lane needs the slow path or `most` blocks ran.
 // Returns the blocks run, the last one unfinished for lanes with a step h
 // that needs the slow path (P_HALT + h in their P_* word).  A function
-// without calls, so that nothing in it is held for one.
-template <int K, bool kRoll>
+// without calls, so that nothing in it is held for one.  M: which special
+// steps it takes itself (persistent_run chooses).
+template <int K, int M>
 __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t, uint32_t most) {
     constexpr bool DBL = (K & 2) != 0, OVER = (K & 1) != 0;
     RareSm& sm = *smp;
@@ -1314,6 +1456,8 @@ __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t
         if (OVER) c1 = J.c_drift;
         else { c1 = J.hdt_invM; c2 = J.hdt; c3 = J.expg; }
     }
+    // nearly every block has a special step: its steps one by one at once
+    const bool walk = M == M_FULL && job >= 0 && jobs[job].walk != 0;
     uint32_t it = 0;
     do {
         // ---- one Philox block, four steps ----
@@ -1328,18 +1472,21 @@ __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t
         // stand; else its lanes take them again one by one, the special ones
         // as quick steps where they can.
         const float x0 = xp, rv0 = rv;
-        float xs[4];
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            f_move(OVER, xp, rv, F, c1, c2, c3, nq[h]);
-            xs[h] = xp;
-            if (!OVER) rv = fmaf(F, c1, rv);
-        }
-        float xmin, xmax;
-        range4(xs[0], xs[1], xs[2], xs[3], &xmin, &xmax);
+        bool bad = true;
         left -= 4;
         ++it;
-        const bool bad = !(xmin > lo) | !(xmax < hi) | (left <= 0);
+        if (M != M_WALK && !(M == M_FULL && walk)) {
+            float xs[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                f_move(OVER, xp, rv, F, c1, c2, c3, nq[h]);
+                xs[h] = xp;
+                if (!OVER) rv = fmaf(F, c1, rv);
+            }
+            float xmin, xmax;
+            range4(xs[0], xs[1], xs[2], xs[3], &xmin, &xmax);
+            bad = !(xmin > lo) | !(xmax < hi) | (left <= 0);
+        }
         if (__any_sync(kFull, bad)) {
             bool halt = false;
             if (bad) {
@@ -1349,7 +1496,7 @@ __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t
                 const uint64_t s0 = (uint64_t)sm.jh[t] << 34 | (uint64_t)j << 2;
                 float n0 = nq[0], n1 = nq[1], n2 = nq[2];
                 const float n3 = nq[3];
-#pragma unroll kRoll ? 1 : 4
+#pragma unroll M <= M_WALK ? 4 : 1
                 for (int h = 0; h < 4; ++h) {
                     if (halt) continue;
                     f_move(OVER, xp, rv, F, c1, c2, c3, n0);
@@ -1358,8 +1505,12 @@ __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t
                     n2 = n3;
                     --left;
                     if (!(xp > lo) | !(xp < hi) | (left == 0)) {
-                        if (job < 0 || !quick_step(DBL, kRoll, jobs[job], sm, t, s0 + 1 + h, left == 0, xp, lo, hi, F,
-                                                    left, pw)) {
+                        const uint64_t s = s0 + 1 + h;
+                        if (job < 0 ||
+                            !(M == M_FULL ? full_quick_step<DBL, OVER>(jobs[job], *sm.slots, sm, t, s, left == 0, xp, rv, lo,
+                                                                       hi, F, left, pw)
+                                          : quick_step(DBL, M == M_FLIPS, jobs[job], sm, t, s, left == 0, xp, lo, hi, F,
+                                                       left, pw))) {
                             halt = true;
                             pw |= P_HALT * (1 + h);
                             sm.nz[0][t] = n0;
@@ -1399,34 +1550,36 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
     const int t = threadIdx.x;
     const int64_t slot = (int64_t)blockIdx.x * blockDim.x + t;
     // out-of-line parts of the model type, or of whichever type (kMixed)
-    constexpr int C = kMixed ? K_ANY : K;
+    constexpr int B = K & ~K_FULL, C = kMixed ? K_ANY : B;
+    sm.slots = &S;   // (all threads the same)
     load_slot<C>(&q, &S, &sm, t, slot);
 
     // Idle lanes look at the queue from block `look` on: kDry once it had
     // nothing left for this warp.
     constexpr uint32_t kDry = ~0u;
-    int most = !kMixed ? first_claim(*q.avail, S) : 32;
     uint32_t it = 0, look = 0;
+    if (!kMixed) {
+        const int most = first_claim(*q.avail, S);
+        if (most < 32) {
+            // leave the items to the warps that take them now; items still
+            // there after that (warps that were to take them have
+            // trajectories already) are claimed
+            if (most == 0 && *(volatile unsigned long long*)q.head < *(volatile unsigned long long*)q.tail)
+                __nanosleep(20000);
+            // Lanes left out of the warp's share take what is still there
+            // once the other warps have had theirs (lanes of theirs may hold
+            // another job's trajectories): 64 blocks are 25-45 us.
+            if (refill<C>(&q, &S, &sm, t, slot, sm.job[t] < 0 && slot < S.nslots, most ? most : 32)) look = kDry;
+            else if (most) look = 64;
+        }
+    }
     while (it < quad_budget) {
         // lanes become idle in the slow path only
         if (__any_sync(kFull, sm.job[t] < 0)) {
             const bool need = sm.job[t] < 0 && it >= look && slot < S.nslots;
             const bool asked = __any_sync(kFull, need);
             if (asked) {
-                if (!kMixed && most == 0) {
-                    // leave the items to the warps that take them now; items
-                    // still there after that (warps that were to take them
-                    // have trajectories already) are claimed
-                    if (*(volatile unsigned long long*)q.head < *(volatile unsigned long long*)q.tail)
-                        __nanosleep(20000);
-                    most = 32;
-                }
-                // Lanes left out of the warp's share take what is still there
-                // once the other warps have had theirs (lanes of theirs may
-                // hold another job's trajectories): 64 blocks are 25-45 us.
-                if (refill<C>(&q, &S, &sm, t, slot, need, most)) look = kDry;
-                else if (!kMixed && most < 32) look = it + 64;
-                most = 32;
+                if (refill<C>(&q, &S, &sm, t, slot, need, 32)) look = kDry;
             }
             if (__all_sync(kFull, sm.job[t] < 0)) {
                 if (!kMixed && it < look && look != kDry) {   // the share has ended already
@@ -1447,15 +1600,30 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
         // with the flips' code it no longer fits the instruction cache), the
         // rolled one for the double barrier (1e-5: 21.2 against 21.7) and for
         // warps of all types on one SM (mixed launches).
+        // Jobs with more frequent special steps of other kinds (JobF::full)
+        // take them in the loop too.
+        // Kernels of every mode take the highest that a lane's job asks for.
+        // (They are kernels of their own: with that many callees the loop here
+        // keeps its values on the stack, 13 % of the time of 100000 of two
+        // barriers at p = 0.01.)
         constexpr bool kOnlyRolled = kMixed || (K & 2) != 0;
-        const bool often = !kOnlyRolled && sm.job[t] >= 0 && q.jobs[sm.job[t]].flips_often != 0;
         const uint32_t blocks = (!kMixed && it < look ? min(quad_budget, look) : quad_budget) - it;
-        if (kOnlyRolled || __any_sync(kFull, often)) it += run_blocks<K, true>(q.jobs, &sm, t, blocks);
-        else it += run_blocks<K, kOnlyRolled>(q.jobs, &sm, t, blocks);
-        const uint32_t halt = sm.pw[t] / P_HALT;
+        if (K & K_FULL) {
+            const uint32_t mode = __reduce_max_sync(kFull, sm.pw[t] / P_MODE);
+            if (mode == M_FULL) it += run_blocks<B, (K & K_FULL) ? M_FULL : M_FLIPS>(q.jobs, &sm, t, blocks);
+            else if (!kMixed && mode == M_WALK)
+                it += run_blocks<B, (K & K_FULL) && !kMixed ? M_WALK : M_FLIPS>(q.jobs, &sm, t, blocks);
+            else if (kOnlyRolled || mode == M_FLIPS) it += run_blocks<B, M_FLIPS>(q.jobs, &sm, t, blocks);
+            else it += run_blocks<B, kOnlyRolled ? M_FLIPS : M_RARE>(q.jobs, &sm, t, blocks);
+        } else {
+            const bool often = !kOnlyRolled && sm.pw[t] / P_MODE >= M_FLIPS;
+            if (kOnlyRolled || __any_sync(kFull, often)) it += run_blocks<B, M_FLIPS>(q.jobs, &sm, t, blocks);
+            else it += run_blocks<B, kOnlyRolled ? M_FLIPS : M_RARE>(q.jobs, &sm, t, blocks);
+        }
+        const uint32_t halt = (sm.pw[t] & P_HALTS) / P_HALT;
         if (__any_sync(kFull, halt != 0)) {
             if (halt) {
-                sm.pw[t] &= P_HALT - 1;
+                sm.pw[t] &= ~P_HALTS;
                 slow_steps<C>(q.jobs, &S, &sm, t, slot, (uint64_t)sm.jh[t] << 32 | sm.j[t], (int)halt - 1);
             }
             __syncwarp();
@@ -1488,7 +1656,7 @@ __global__ void __launch_bounds__(256, (K & K_WIDE) ? kWideBlocks : kNarrowBlock
 // across launches in wtype (-1: none).  A warp ends its launch when the
 // budget is spent, no queue has work, or eight type changes in a row found
 // nothing to claim (claims raced away by other warps).
-template <int kUnused>
+template <int KF>
 __global__ void __launch_bounds__(256, kNarrowBlocks) fp32_mixed_kernel(const __grid_constant__ MixedDev m,
                                                                                uint32_t quad_budget) {
     extern __shared__ uint4 sm_raw[];
@@ -1530,10 +1698,10 @@ __global__ void __launch_bounds__(256, kNarrowBlocks) fp32_mixed_kernel(const __
         bool drained = false;
         uint32_t used;
         switch (type) {
-            case 0: used = persistent_run<0, true>(m.q[0], m.S, sm, left, &drained); break;
-            case 1: used = persistent_run<1, true>(m.q[1], m.S, sm, left, &drained); break;
-            case 2: used = persistent_run<2, true>(m.q[2], m.S, sm, left, &drained); break;
-            default: used = persistent_run<3, true>(m.q[3], m.S, sm, left, &drained); break;
+            case 0: used = persistent_run<KF + 0, true>(m.q[0], m.S, sm, left, &drained); break;
+            case 1: used = persistent_run<KF + 1, true>(m.q[1], m.S, sm, left, &drained); break;
+            case 2: used = persistent_run<KF + 2, true>(m.q[2], m.S, sm, left, &drained); break;
+            default: used = persistent_run<KF + 3, true>(m.q[3], m.S, sm, left, &drained); break;
         }
         left -= (used < left) ? used : left;
         if (drained) {
@@ -1565,54 +1733,64 @@ int launch_fp32_publish(const QueueDev& q, unsigned long long new_tail, int32_t 
 }
 
 using PersistentKernel = void (*)(QueueDev, SlotsDev, uint32_t);
-static PersistentKernel persistent_kernel(bool dbl, bool over, bool wide) {
+template <int F>
+static PersistentKernel persistent_kernel_of(bool dbl, bool over, bool wide) {
     switch ((wide ? 4 : 0) | (dbl ? 2 : 0) | (over ? 1 : 0)) {
-        case 0: return fp32_persistent_kernel<0>;
-        case 1: return fp32_persistent_kernel<1>;
-        case 2: return fp32_persistent_kernel<2>;
-        case 3: return fp32_persistent_kernel<3>;
-        case 4: return fp32_persistent_kernel<K_WIDE + 0>;
-        case 5: return fp32_persistent_kernel<K_WIDE + 1>;
-        case 6: return fp32_persistent_kernel<K_WIDE + 2>;
-        default: return fp32_persistent_kernel<K_WIDE + 3>;
+        case 0: return fp32_persistent_kernel<F + 0>;
+        case 1: return fp32_persistent_kernel<F + 1>;
+        case 2: return fp32_persistent_kernel<F + 2>;
+        case 3: return fp32_persistent_kernel<F + 3>;
+        case 4: return fp32_persistent_kernel<F + K_WIDE + 0>;
+        case 5: return fp32_persistent_kernel<F + K_WIDE + 1>;
+        case 6: return fp32_persistent_kernel<F + K_WIDE + 2>;
+        default: return fp32_persistent_kernel<F + K_WIDE + 3>;
     }
+}
+static PersistentKernel persistent_kernel(bool dbl, bool over, bool wide, bool full) {
+    return full ? persistent_kernel_of<K_FULL>(dbl, over, wide) : persistent_kernel_of<0>(dbl, over, wide);
+}
+
+// Resident blocks per SM of either kernel (with all modes or the two common
+// ones; the fewer, should they ever differ), 0 on error.
+template <class Kernel>
+static int resident_blocks(Kernel plain, Kernel full, int block) {
+    int least = 0;
+    for (Kernel kern : {plain, full}) {
+        // The kernel reads little global memory: give shared memory the whole
+        // carveout so that the occupancy the grid is sized for is resident.
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                             (int)cudaSharedmemCarveoutMaxShared);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RareSm));
+        int n = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, sizeof(RareSm));
+        if (e != cudaSuccess) return 0;
+        least = kern == plain ? n : std::min(least, n);
+    }
+    return least;
 }
 
 int fp32_blocks_per_sm(bool dbl, bool over, bool wide, int block) {
-    const PersistentKernel kern = persistent_kernel(dbl, over, wide);
-    // The kernel reads little global memory: give shared memory the whole
-    // carveout so that the occupancy the grid is sized for is resident.
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                         (int)cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RareSm));
-    int n = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, sizeof(RareSm));
-    return e == cudaSuccess ? n : 0;
+    return resident_blocks(persistent_kernel(dbl, over, wide, false), persistent_kernel(dbl, over, wide, true), block);
 }
 
 int fp32_mixed_blocks_per_sm(int block) {
-    int n = 0;
-    cudaError_t e = cudaFuncSetAttribute(fp32_mixed_kernel<0>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                         (int)cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fp32_mixed_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RareSm));
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fp32_mixed_kernel<0>, block, sizeof(RareSm));
-    return e == cudaSuccess ? n : 0;
+    return resident_blocks(fp32_mixed_kernel<0>, fp32_mixed_kernel<K_FULL>, block);
 }
 
-int launch_fp32_mixed(const MixedDev& m, uint32_t pair_budget, int grid, int block, void* stream) {
+int launch_fp32_mixed(const MixedDev& m, bool full, uint32_t pair_budget, int grid, int block, void* stream) {
     const uint32_t quad_budget = pair_budget > 1 ? pair_budget / 2 : 1;
     if (block != 256 || (int64_t)grid * block > m.S.nslots) return (int)cudaErrorInvalidValue;
-    fp32_mixed_kernel<0><<<grid, block, sizeof(RareSm), (cudaStream_t)stream>>>(m, quad_budget);
+    auto* kern = full ? fp32_mixed_kernel<K_FULL> : fp32_mixed_kernel<0>;
+    kern<<<grid, block, sizeof(RareSm), (cudaStream_t)stream>>>(m, quad_budget);
     return (int)cudaGetLastError();
 }
 
-int launch_fp32_persistent(bool dbl, bool over, bool wide, const QueueDev& q, const SlotsDev& s, uint32_t pair_budget,
-                           int grid, int block, void* stream) {
+int launch_fp32_persistent(bool dbl, bool over, bool wide, bool full, const QueueDev& q, const SlotsDev& s,
+                           uint32_t pair_budget, int grid, int block, void* stream) {
     const uint32_t quad_budget = pair_budget > 1 ? pair_budget / 2 : 1;   // blocks of four steps
     if (block > kMaxBlock) return (int)cudaErrorInvalidValue;
-    persistent_kernel(dbl, over, wide)<<<grid, block, sizeof(RareSm), (cudaStream_t)stream>>>(q, s, quad_budget);
+    persistent_kernel(dbl, over, wide, full)<<<grid, block, sizeof(RareSm), (cudaStream_t)stream>>>(q, s, quad_budget);
     return (int)cudaGetLastError();
 }
 

@@ -29,11 +29,17 @@ enum : int32_t {
     EV_FP = 32     // FIRST_PASSAGE mode: the first FPT2 event ends the trajectory
 };
 
+// Which special steps the hot loop takes itself (run_blocks): the commonest;
+// the same, its steps one by one at once; flips too; flips, frames and
+// crossings of every kind.
+enum : uint32_t { M_RARE = 0, M_WALK = 1, M_FLIPS = 2, M_FULL = 3 };
+
 // Per-job constants and output pointers (device resident, one per job).
 struct JobF {
     // model switches (jobs of one queue share dbl/over)
     int32_t dbl, over;
-    int32_t flips_often, pad0;   // flips are frequent among the special steps (run_blocks)
+    int32_t mode;          // M_*: the special steps that run_blocks takes itself
+    int32_t walk;          // M_FULL: nearly every block of four steps has a special one
     int32_t eta, eq, rs, rv, us, init_state, wt, fpt, tpt, cg, n_cg, write_x, at_bottom, fp_mode;
     int32_t lanes, nruns, slots_log2;
     int32_t evm;         // EV_* statistics switches of the event path
@@ -144,10 +150,11 @@ struct MixedDev {
 int launch_fp32_publish(const QueueDev& q, unsigned long long new_tail, int32_t new_nranges, void* stream);
 // Resident blocks per SM of the persistent kernel (0 on error).
 int fp32_blocks_per_sm(bool dbl, bool over, bool wide, int block);
-int launch_fp32_persistent(bool dbl, bool over, bool wide, const QueueDev& q, const SlotsDev& s, uint32_t pair_budget,
-                           int grid, int block, void* stream);
+// full: the kernel for jobs of every mode (M_*), else of M_RARE and M_FLIPS.
+int launch_fp32_persistent(bool dbl, bool over, bool wide, bool full, const QueueDev& q, const SlotsDev& s,
+                           uint32_t pair_budget, int grid, int block, void* stream);
 // Resident 256-thread blocks per SM of the mixed kernel, and its launch.
 int fp32_mixed_blocks_per_sm(int block);
-int launch_fp32_mixed(const MixedDev& m, uint32_t pair_budget, int grid, int block, void* stream);
+int launch_fp32_mixed(const MixedDev& m, bool full, uint32_t pair_budget, int grid, int block, void* stream);
 
 }  // namespace ldp

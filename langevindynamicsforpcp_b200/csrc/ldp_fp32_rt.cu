@@ -34,6 +34,7 @@ struct Fp32Queue {
     // unfinished job: until then slots past the narrow grid may hold some.
     int grid = 0, wide_grid = 0, block = 256;
     bool wide = false;
+    bool full = false;   // an unfinished job asks for another mode than M_RARE and M_FLIPS
     int cur_grid() const { return wide ? wide_grid : grid; }
     int64_t lanes() const { return (int64_t)cur_grid() * block; }
     uint64_t pair_budget = 1 << 15;
@@ -176,7 +177,6 @@ static void fill_jobf(const ldp_job* job, JobF* J) {
     const TrajState& S = job->st;
     const int64_t n = job->ntraj;
     J->dbl = k.dbl; J->over = k.over;
-    J->flips_often = k.eta && std::min(k.ln1m[0], k.ln1m[1]) < -1.5e-4;
     J->eta = k.eta; J->eq = k.eq; J->rs = k.rs; J->rv = k.rv; J->us = k.us; J->init_state = k.init_state;
     J->wt = k.wt; J->fpt = k.fpt; J->tpt = k.tpt; J->cg = k.cg; J->n_cg = k.n_cg; J->write_x = k.write_x;
     J->at_bottom = k.at_bottom; J->fp_mode = k.fp_mode; J->lanes = k.lanes; J->nruns = k.nruns;
@@ -226,6 +226,33 @@ static void fill_jobf(const ldp_job* job, JobF* J) {
         J->edge_hi = nb >= 3 ? J->bp[nb - 2] : -k.fhalfL;
         const bool flat = k.dbl ? (k.flo0 > -k.fhalfL && k.fhi1 < k.fhalfL) : (k.fw < k.fhalfL);
         J->edge_flat = (nb >= 3 && flat) ? 1 : 0;
+    }
+    {
+        // The special steps that the hot loop takes itself.  All of them
+        // (M_FULL) where they are frequent and nearly always quick ones, that
+        // is where a step is short against the bands; where it is not, lanes
+        // leave the loop at most blocks anyway and the other loops are shorter
+        // (32815 trajectories of two barriers, steps of 0.16 of a band, p =
+        // 0.5: M_FLIPS 8.9 ms, M_FULL 14.8; at 0.05: 164 / 139; 1093 of them,
+        // few lanes to a warp, 4.7 / 3.4).
+        // M_FLIPS / M_FULL, ms for 24400 steps of 100000 overdamped
+        // trajectories, dt 1e-4: one barrier, p = 0.5 93.7 / 50.9, 0.09 70.1 /
+        // 46.5, 0.01 28.7 / 28.1; two, 123 / 83, 93 / 69, 29 / 31.
+        // Underdamped ones cross few edges: 43.2 / 53.9 and 40.8 / 50.6, so
+        // only their WRITEX frames (20000 x 10400, a frame in 8: 5.3 / 3.1),
+        // flips at frame steps, and flanks that reach the cell edge (66 / 32)
+        // count.  A frame in four steps or fewer is a special step in every
+        // block: M_WALK (100000 underdamped x 5200, a frame in four: 2.01 /
+        // 1.83).
+        const double ln1m = k.eta ? std::min(k.ln1m[0], k.ln1m[1]) : 0.0;
+        const bool frames = !k.fp_mode, dense = frames && k.freq_save <= 4;
+        const double band = 2.0 * k.fhalfL / std::max(1, J->nbp - 1);   // on average
+        const double move = k.over ? 2.0 * (double)k.fsig_r : k.dt * k.sig_v0;
+        J->mode = ln1m < -1.5e-4 ? M_FLIPS : dense ? M_WALK : M_RARE;
+        if ((move < band / 10 || n <= 4096) && ((k.over && (ln1m < -0.05 || dense)) || (dense && J->mode == M_FLIPS) ||
+                                 (frames && k.write_x) || !J->edge_flat))
+            J->mode = M_FULL;
+        J->walk = ln1m < -0.1 || dense;
     }
     J->x0 = k.x0; J->v0 = k.v0; J->dt = k.dt; J->Ld = k.L; J->invL = k.invL; J->sig_v0 = k.sig_v0;
     J->sig_r_d = k.sig_r; J->a_lap = k.a_lap; J->c_lap[0] = k.c_lap[0]; J->c_lap[1] = k.c_lap[1];
@@ -283,7 +310,7 @@ bool fp32_queue_quiet(ldp_ctx* ctx, int type) {
 int fp32_launch_type(ldp_ctx* ctx, int type, uint32_t pair_budget, cudaStream_t st) {
     Fp32Queue& Q = ctx->fp32->q[type];
     if (!Q.ready) return 0;
-    return launch_fp32_persistent(type >= 2, (type & 1) != 0, Q.wide, Q.q, Q.s, pair_budget, Q.cur_grid(), Q.block, st);
+    return launch_fp32_persistent(type >= 2, (type & 1) != 0, Q.wide, Q.full, Q.q, Q.s, pair_budget, Q.cur_grid(), Q.block, st);
 }
 
 // One persistent launch over all four model types' queues (serving): the
@@ -317,7 +344,8 @@ int fp32_launch_mixed(ldp_ctx* ctx, uint32_t pair_budget, cudaStream_t st) {
     m.wtype = R.wtype;
     m.sm_type = R.wtype + R.mixed.nslots / 32;
     m.nwarps = R.mixed.nslots / 32;
-    return launch_fp32_mixed(m, pair_budget, R.mixed_grid, 256, st);
+    const bool full = R.q[0].full || R.q[1].full || R.q[2].full || R.q[3].full;
+    return launch_fp32_mixed(m, full, pair_budget, R.mixed_grid, 256, st);
 }
 
 // Slots of the mixed launches (0 before the first).
@@ -361,10 +389,17 @@ int fp32_register(ldp_job* job, cudaStream_t stream, bool publish) {
     int e = queue_init(ctx, Q, type, ctx->fp32_ring_slots ? ctx->fp32_ring_slots : 64);
     if (e) return e;
     if (Q.free_slots.empty()) return (int)cudaErrorMemoryAllocation;
+    JobF J;
+    fill_jobf(job, &J);
+    job->fp32_full = J.mode == M_WALK || J.mode == M_FULL;
     if (fp32_queue_quiet(ctx, type)) Q.wide = false;
     int64_t items = job->ntraj;
+    Q.full = job->fp32_full;
     for (const ldp_job* j : Q.table)
-        if (j && !j->done) items += j->ntraj;
+        if (j && !j->done) {
+            items += j->ntraj;
+            Q.full = Q.full || j->fp32_full;
+        }
     if (items > (int64_t)Q.grid * Q.block) Q.wide = Q.wide_grid > Q.grid;
     const int slot = Q.free_slots.back();
     Q.free_slots.pop_back();
@@ -372,8 +407,6 @@ int fp32_register(ldp_job* job, cudaStream_t stream, bool publish) {
     job->fp32_type = type;
     job->fp32_slot = slot;
     job->fp32_published = 0;
-    JobF J;
-    fill_jobf(job, &J);
     J.remaining = &Q.rem[slot];
     int64_t* h = stage(Q);
     static_assert(sizeof(JobF) <= 4096 - 64, "JobF must fit the staging buffer");
@@ -421,7 +454,7 @@ int fp32_pump(ldp_job* job, int nlaunch) {
     const bool dbl = job->k.dbl, over = job->k.over;
     for (int i = 0; i < nlaunch; ++i) {
         const uint32_t pb = (uint32_t)std::min<uint64_t>(Q.pair_budget, 0xffffffffull);
-        int e = launch_fp32_persistent(dbl, over, Q.wide, Q.q, Q.s, pb, Q.cur_grid(), Q.block, ctx->stream);
+        int e = launch_fp32_persistent(dbl, over, Q.wide, Q.full, Q.q, Q.s, pb, Q.cur_grid(), Q.block, ctx->stream);
         if (e) return e;
         ++job->launches;
     }

@@ -84,6 +84,7 @@ struct ldp_job {
     int32_t* d_i32b = nullptr;   // FP32 batched: 32-bit statistics state
     int fp32_type = -1;          // FP32 batched: queue (dbl*2 + over) the job is in
     int fp32_slot = -1;          // FP32 batched: index in that queue's job table
+    bool fp32_full = false;      // FP32 batched: needs the kernels for every mode (JobF::mode)
     int64_t fp32_published = 0;  // FP32 batched: trajectories published to the queue
     bool finalized = false;      // results post-processed after completion
     int fp32_phase = 0;          // 0 idle, 1 integrating, 2 finalizing, 3 in a batch graph

@@ -13,7 +13,7 @@ import numpy as np
 import pytest
 
 import langevindynamicsforpcp_b200 as ldp
-from langevindynamicsforpcp_b200 import _tune
+from langevindynamicsforpcp_b200 import _tune, serve
 
 GOLDEN = os.path.join(os.path.dirname(__file__), "golden", "inp")
 pytestmark = pytest.mark.gpu
@@ -190,3 +190,51 @@ def test_pairs_of_barriers_that_never_flip(kind):
         for k in whole:
             np.testing.assert_array_equal(other[k], whole[k], err_msg=k)
     assert (np.diff(np.sign(whole["frames_x"][1:] - whole["frames_x"][0]), axis=0) != 0).any()
+
+
+FULL = [  # kind, parameters: what makes lanes take every quick step in the loop, or walk
+    ("single_over", dict(tau=1e-5)), ("double_over", dict(tau=1e-5)),              # flips at p = 0.5
+    ("single_over", dict(tau=4e-4)), ("double_over", dict(tau=4e-4)),              # and 0.2
+    ("single_under", dict(tau=1e-5, write_x=1)), ("double_under", dict(tau=2e-3, write_x=1)),
+    ("single_over", dict(tau=1.0, write_x=1)), ("double_over", dict(tau=0.0, write_x=1)),
+    ("single_over", dict(tau=1e-2, freq_save=1)), ("double_over", dict(tau=1.0, freq_save=3)),   # frames
+    ("single_under", dict(tau=1.0, freq_save=1)), ("double_under", dict(tau=1.0, freq_save=4)),
+    ("single_under", dict(tau=1e-3, freq_save=2)),                                 # flips at frame steps
+    ("single_over", dict(tau=1e-3, flank=1.0)), ("single_under", dict(tau=1e-5, flank=1.2)),   # no flat band
+    ("single_over", dict(tau=1e-5, eq=0, eq_constant=8.0)), ("double_over", dict(tau=1e-5, timestep=1e-3)),
+]
+
+
+@pytest.mark.parametrize("kind,kw", FULL)
+def test_quick_steps_of_every_kind_equal_general_ones(kind, kw):
+    # Launches of one block of steps end every pair of cells; the job alone,
+    # in one launch with a job of rare special steps (the same kernel, lanes
+    # of both jobs in a warp), and in the serving kernel give the same bits.
+    kw = dict(kw)
+    steps = 1201 * kw.get("freq_save", 7)
+    p = params(kind, steps, **{k: v for k, v in kw.items() if k != "flank"})
+    if "flank" in kw:
+        p.barrier_half_width[0] = kw["flank"] * p.periodic_length / 2
+    whole = run(p, 333)
+    assert len([k for k in whole if k.startswith("frames")]) == (7 if p.write_x else 1)
+    short = run(p, 333, budget=2)
+    rare = params(kind, 1201 * 7, tau=1.0)
+    with ldp.Context(0) as c:
+        jobs = [ldp.Job(c, q, lanes=n, precision=ldp.PREC_FP32_BATCHED, job_id=i)
+                for q, n, i in ((rare, 100, 8), (p, 333, 3), (rare, 50, 9))]
+        ldp.submit_batch(c, jobs)
+        mixed = jobs[1].wait().results()
+        for j in jobs:
+            j.close()
+    served = {}
+    with ldp.Context(0) as c, serve.Server(c) as srv:
+        work = [(rare, 64, {}), (rare, 65, {}), (rare, 66, {}), (p, 333, {})]   # job ids 0 to 3
+        serve.run_stream(srv, work, np.zeros(len(work)), timeout_s=60,
+                         on_done=lambda i, j: served.__setitem__(i, j.results(frames=False)))
+    for other in (short, mixed, served[3]):
+        assert len(other) >= 7
+        for k in other:
+            a, b = other[k], whole[k]
+            if a.dtype == np.float64:
+                a, b = a.view(np.int64), b.view(np.int64)
+            np.testing.assert_array_equal(a, b, err_msg=k)
