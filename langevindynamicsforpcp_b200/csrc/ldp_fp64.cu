@@ -1084,6 +1084,11 @@ template <bool DBL, bool OVER, bool ETA, bool DENSE>
 __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, const TrajState st, int64_t g0,
                                                          uint64_t s_begin, uint64_t s_end) {
     constexpr int S = DENSE ? kOwnDense : kOwnSteps;
+    // Blocks of four where flips are frequent and steps overdamped, the edge
+    // between two cells being crossed often (65536 x 24400, p = 0.5, blocks of
+    // eight / four: one barrier 28.4 / 26.6 ms, two 42.4 / 39.6; underdamped
+    // first passage 10.0 / 10.1).
+    constexpr int kSteps = DENSE && OVER ? 4 : kGrpSteps;
     __shared__ double rows[128 * (S + 1)];   // of an odd length: see fp64_group_kernel
     __shared__ uint32_t wrows[DENSE ? 128 * (S + 1) : 1];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1122,7 +1127,7 @@ __global__ void __launch_bounds__(128, 4) fp64_steps_kernel(const KConst k, cons
                 wt[m + 1] = w[1];
             }
         }
-        take_steps<DBL, OVER, ETA, DENSE, kGrpSteps>(k, st, i, g, a, c, s0, l, n, z, wt);
+        take_steps<DBL, OVER, ETA, DENSE, kSteps>(k, st, i, g, a, c, s0, l, n, z, wt);
         l = 0;
         s0 += S;
     }
