@@ -23,7 +23,8 @@
 // countdown ended.  If not (about one block in five), the lanes concerned take
 // the block again step by step.  Their special steps are quick steps, inline
 // (a frame, a flank entered or left, the edge between the two cells of a pair
-// crossed, a flip where flips are frequent), or take the slow path out of line
+// crossed, a flip where flips are frequent, and in the kernels of jobs with many
+// special steps (M_FULL) nearly all kinds), or take the slow path out of line
 // (special_step): at last the general step, which follows the FP64 step
 // exactly (wrap, indices, flip, cell-table entry with lazy catch-up, force,
 // renewal statistics, frame, end).
@@ -289,7 +290,8 @@ __device__ __forceinline__ void record_extra(const bool DBL, const JobF& J, int6
     if (J.fke) J.fke[o] = J.mhalf * ((double)v * (double)v);
     if (J.fst) J.fst[o] = (double)state;
 }
-__device__ __noinline__ void f_record_extra(bool DBL, const JobF* Jp, int64_t o, float xp, float v, float F, int state) {
+__device__ __noinline__ void f_record_extra(bool DBL, const JobF* Jp, int64_t o, float xp, float v, float F,
+                                            int state) {
     record_extra(DBL, *Jp, o, xp, v, F, state);
 }
 
@@ -1507,8 +1509,8 @@ __device__ __noinline__ uint32_t run_blocks(const JobF* jobs, RareSm* smp, int t
                     if (!(xp > lo) | !(xp < hi) | (left == 0)) {
                         const uint64_t s = s0 + 1 + h;
                         if (job < 0 ||
-                            !(M == M_FULL ? full_quick_step<DBL, OVER>(jobs[job], *sm.slots, sm, t, s, left == 0, xp, rv, lo,
-                                                                       hi, F, left, pw)
+                            !(M == M_FULL ? full_quick_step<DBL, OVER>(jobs[job], *sm.slots, sm, t, s, left == 0, xp,
+                                                                       rv, lo, hi, F, left, pw)
                                           : quick_step(DBL, M == M_FLIPS, jobs[job], sm, t, s, left == 0, xp, lo, hi, F,
                                                        left, pw))) {
                             halt = true;
@@ -1600,12 +1602,10 @@ __device__ __forceinline__ uint32_t persistent_run(const QueueDev& q, const Slot
         // with the flips' code it no longer fits the instruction cache), the
         // rolled one for the double barrier (1e-5: 21.2 against 21.7) and for
         // warps of all types on one SM (mixed launches).
-        // Jobs with more frequent special steps of other kinds (JobF::full)
-        // take them in the loop too.
-        // Kernels of every mode take the highest that a lane's job asks for.
-        // (They are kernels of their own: with that many callees the loop here
-        // keeps its values on the stack, 13 % of the time of 100000 of two
-        // barriers at p = 0.01.)
+        // Kernels of every mode take the highest that a lane's job asks for
+        // (JobF::mode).  They are kernels of their own: with that many callees
+        // the loop here keeps its values on the stack, 13 % of the time of
+        // 100000 trajectories of two barriers at p = 0.01.
         constexpr bool kOnlyRolled = kMixed || (K & 2) != 0;
         const uint32_t blocks = (!kMixed && it < look ? min(quad_budget, look) : quad_budget) - it;
         if (K & K_FULL) {

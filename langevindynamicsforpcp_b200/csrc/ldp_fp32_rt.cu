@@ -310,7 +310,8 @@ bool fp32_queue_quiet(ldp_ctx* ctx, int type) {
 int fp32_launch_type(ldp_ctx* ctx, int type, uint32_t pair_budget, cudaStream_t st) {
     Fp32Queue& Q = ctx->fp32->q[type];
     if (!Q.ready) return 0;
-    return launch_fp32_persistent(type >= 2, (type & 1) != 0, Q.wide, Q.full, Q.q, Q.s, pair_budget, Q.cur_grid(), Q.block, st);
+    return launch_fp32_persistent(type >= 2, (type & 1) != 0, Q.wide, Q.full, Q.q, Q.s, pair_budget, Q.cur_grid(),
+                                  Q.block, st);
 }
 
 // One persistent launch over all four model types' queues (serving): the
