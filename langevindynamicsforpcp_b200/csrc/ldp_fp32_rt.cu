@@ -217,6 +217,9 @@ static void fill_jobf(const ldp_job* job, JobF* J) {
         c[nc++] = 0.0f;
         if (!k.dbl) { c[nc++] = -k.fw; c[nc++] = k.fw; }
         else { c[nc++] = k.flo0; c[nc++] = k.fxb[0]; c[nc++] = k.fxc; c[nc++] = k.fxb[1]; c[nc++] = k.fhi1; }
+        // (The flanks' meeting point is not a number where both barriers have
+        // no height in state 0: no breakpoint then, and no comparison with it.)
+        nc = (int)(std::remove_if(c, c + nc, [](float b) { return b != b; }) - c);
         std::sort(c, c + nc);
         int nb = 0;
         for (int i = 0; i < nc; ++i)
